@@ -208,38 +208,43 @@ static int radices(int n, int *rad, int *nrad)
  * computes it for aExpArg: 2 pi (n/2 - |t - n/2|) / n (SCFT.c:993-995). */
 static double kval(int t, int n) { return 2.0 * M_PI * (n / 2.0 - fabs(t - n / 2.0)) / n; }
 
-/* Dense 1-D operator of one axis, n x n, row-major K[i*n + j]. */
+/* Dense 1-D operator of one axis, n x n, row-major K[i*n + j]. Both kinds are
+ * sums over modes of E_m times cosines of m (i -+ j), so n^2 products with a
+ * table of the cosines give them (one sine or cosine per entry and mode took
+ * 0.5 s for a 96-point Dirichlet axis on a host with software quad precision,
+ * once per operator set). */
 static void dense_operator(int n, double alpha, int dirichlet, std::vector<long double> &K)
 {
     K.assign((size_t)n * n, 0.0L);
+    const long double pi = 3.141592653589793238462643383279502884L;
     if (dirichlet) {
-        /* odd extension of length N = 2(n+1): K = (2/L) sum_m E_m sin(pi m a/L) sin(pi m b/L) */
+        /* odd extension of length N = 2(n+1): K = (2/L) sum_m E_m sin(pi m a/L) sin(pi m b/L)
+         * = f(a - b) - f(a + b), f(d) = (1/L) sum_m E_m cos(pi m d / L) */
         const int L = n + 1, N = 2 * L;
-        std::vector<long double> E(n + 1);
+        std::vector<long double> E(n + 1), cs(N), f(N);
         for (int m = 1; m <= n; ++m) {
             const double kz = kval(m, N);
             E[m] = expl(-(long double)alpha * (long double)kz * (long double)kz);
         }
-        const long double pi = 3.141592653589793238462643383279502884L;
+        for (int d = 0; d < N; ++d) cs[d] = cosl(pi * d / L);
+        for (int d = 0; d < N; ++d) {
+            long double s = 0.0L;
+            for (int m = 1; m <= n; ++m) s += E[m] * cs[(m * d) % N];
+            f[d] = s / L;
+        }
         for (int a = 0; a < n; ++a)
-            for (int b = a; b < n; ++b) {
-                long double s = 0.0L;
-                for (int m = 1; m <= n; ++m)
-                    s += E[m] * sinl(pi * m * (a + 1) / L) * sinl(pi * m * (b + 1) / L);
-                s *= 2.0L / L;
-                K[(size_t)a * n + b] = s;
-                K[(size_t)b * n + a] = s;
-            }
+            for (int b = 0; b < n; ++b) K[(size_t)a * n + b] = f[a < b ? b - a : a - b] - f[a + b + 2];
     } else {
         /* circulant: K[i][j] = (1/n) sum_t E_t cos(2 pi t (i-j) / n) */
-        const long double pi = 3.141592653589793238462643383279502884L;
-        std::vector<long double> c(n);
+        std::vector<long double> c(n), E(n), cs(n);
+        for (int t = 0; t < n; ++t) {
+            const double k = kval(t, n);
+            E[t] = expl(-(long double)alpha * k * k);
+            cs[t] = cosl(2.0L * pi * t / n);
+        }
         for (int d = 0; d < n; ++d) {
             long double s = 0.0L;
-            for (int t = 0; t < n; ++t) {
-                const double k = kval(t, n);
-                s += expl(-(long double)alpha * k * k) * cosl(2.0L * pi * t * d / n);
-            }
+            for (int t = 0; t < n; ++t) s += E[t] * cs[(t * d) % n];
             c[d] = s / n;
         }
         for (int i = 0; i < n; ++i)
