@@ -110,10 +110,12 @@ typedef struct scft_options {
     int use_graph;   /* capture one iteration as a CUDA graph and replay it */
     int n_instances; /* instances in this context (batching form); 1 for a single solve */
     int kernel_path; /* 0: fused single-launch contour step where the shape has one, else per-axis
-                        passes; 1: per-axis passes only */
+                        passes, a launch each or all of a chain's in one; 1: per-axis passes, a
+                        launch each */
     int autotune;    /* 1 (default): time the launch forms on the context's own chains at
                         creation and keep the fastest (cached per shape and batch size): per-axis
-                        pass tiles, the fused 2D loop's one or two threads per line; 0: heuristics.
+                        pass tiles, passes as launches or as one loop, the fused 2D loop's one or
+                        two threads per line; 0: heuristics.
                         Every candidate gives bit-identical results. The timing is taken with the
                         context alone on the GPU: contexts whose iterations are kept in flight side
                         by side (pipelined parts of one batch, serving pools) run better on the
@@ -300,7 +302,8 @@ typedef struct scft_timing {
     long prop_launches;
     long kernel_launches;
     int fused_chain;   /* contour steps run in one persistent launch: 1 the fused 2D chain kernel,
-                          2 the 64^3 cluster kernel; 0 per-axis passes */
+                          2 the 64^3 cluster kernel; 0 per-axis passes (prop_launches tells whether
+                          each is a launch or a chain's passes run in one) */
     int threads_per_line; /* fused 2D kernel: 2 when a batch of at most one chain per SM gives each
                              line two threads (bit-identical results), else 1 */
 } scft_timing;

@@ -47,7 +47,7 @@ def _stale(out: Path, deps) -> bool:
 
 def build(verbose: bool = False, force: bool = False) -> Path:
     BUILD.mkdir(exist_ok=True)
-    headers = list(CSRC.glob("*.h")) + list((ROOT / "include").glob("*.h"))
+    headers = list(CSRC.glob("*.h")) + list(CSRC.glob("*.cuh")) + list((ROOT / "include").glob("*.h"))
     jobs = []
     objs = []
     for src in sorted(CSRC.glob("*.cu")):

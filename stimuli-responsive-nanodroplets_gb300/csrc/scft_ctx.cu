@@ -76,6 +76,8 @@ struct Axis {
     int dirichlet_dense; /* 1: dense operator (Dirichlet or a length with other prime factors) */
     int dirichlet;       /* 1: the MASK 1 z axis */
     int src;             /* grid axis 0, 1, 2 */
+    int tc;              /* 1: the pass runs on the tensor cores (geometry in t) */
+    TcGeom t;
 };
 
 /* Propagator chains of one instance in the reference's order of species:
@@ -113,6 +115,8 @@ struct scft_ctx {
     int fused2d = 0;
     int wide2d = 0; /* fused 2D loop with two threads per line (batches of at most one chain per SM) */
     int fused3d = 0;
+    int loop_tc = 0; /* the cluster contour loop on the tensor-core tiles (k_chain_tc) */
+    TcLoop loop;
     int *order = nullptr; /* chain indices, longest first */
     /* device noise replay (SCFT_NOISE_DRAND48) */
     unsigned long long *rng_in = nullptr;
@@ -598,10 +602,210 @@ static int build_fused2d(scft_ctx *c)
     c->wide2d = scft_step2d_wide(c->opt.precision, nx, d0.nz) && (long)c->B * c->nchains <= c->sms;
     return SCFT_OK;
 }
+/* Blocks of a tensor-core pass: half-axis and mirror symmetry on periodic axes of
+ * length 4k, mirror symmetry otherwise. */
+static void tc_shape(int n, int dirichlet, TcGeom &g)
+{
+    memset(&g, 0, sizeof(g));
+    g.n = n;
+    g.nb = (!dirichlet && n % 4 == 0) ? 4 : 2;
+    g.hb = g.nb == 4 ? n / 4 : (n + 1) / 2;
+    g.hp = (g.hb + 15) / 16 * 16;
+    g.w = 8;
+    g.nchunks = (g.hb + g.w - 1) / g.w;
+    g.parts = 1;
+    g.cpp = g.nchunks;
+}
+
+/* Block operators of the tensor-core passes (scft_pass_tc.cu): with u_b the sums
+ * and differences of a line's points (block 0 all sums, then the mirror
+ * difference; on a periodic axis of length 4k the half-axis difference's pair
+ * after them), y is built from M_b u_b by the same sums and differences. Points
+ * of block row and column i < hb; the middle point of an odd axis counts
+ * itself twice in its sum, which the operator's column halves. */
+static std::vector<long double> tc_blocks(const std::vector<long double> &K, int n, int nb, int hb)
+{
+    std::vector<long double> M((size_t)nb * hb * hb, 0.0L);
+    const int m = n / 2;
+    for (int i = 0; i < hb; ++i)
+        for (int j = 0; j < hb; ++j) {
+            const auto k = [&](int col) { return K[(size_t)i * n + col]; };
+            const size_t at = (size_t)i * hb + j, sz = (size_t)hb * hb;
+            if (nb == 2) {
+                const bool mid = 2 * j + 1 == n;
+                M[at] = mid ? k(j) / 2.0L : (k(j) + k(n - 1 - j)) / 2.0L;
+                M[sz + at] = mid ? 0.0L : (k(j) - k(n - 1 - j)) / 2.0L;
+            } else {
+                const long double a0 = k(j) + k(j + m), a1 = k(m - 1 - j) + k(n - 1 - j);
+                const long double b0 = k(j) - k(j + m), b1 = k(m - 1 - j) - k(n - 1 - j);
+                M[at] = (a0 + a1) / 4.0L;
+                M[sz + at] = (a0 - a1) / 4.0L;
+                M[2 * sz + at] = (b0 + b1) / 4.0L;
+                M[3 * sz + at] = (b0 - b1) / 4.0L;
+            }
+        }
+    return M;
+}
+
+static int tc_sk(int prec) { return prec == SCFT_PREC_FP32 ? 4 : 6; }
+
+/* fp16 bits of an integer |d| <= 512 */
+static uint16_t half_of_int(int d)
+{
+    if (d == 0) return 0;
+    const uint16_t sign = d < 0 ? 0x8000 : 0;
+    unsigned u = (unsigned)(d < 0 ? -d : d);
+    int e = 0;
+    while ((u >> e) > 1) ++e;
+    return (uint16_t)(sign | ((15 + e) << 10) | ((u << (10 - e)) & 0x3ff));
+}
+
+/* The operator digits of one axis in the layout of k_pass_tc: chunk, block,
+ * 16-point step, then rows (digit, output) as K-major 8 x 16-byte core
+ * matrices. Entries are integers M 2^kq below 2^(10 sk - 1) in balanced digits
+ * of 10 bits, kq = 10 sk - 1 for nb = 2 and 10 sk for nb = 4. */
+static std::vector<uint16_t> tc_table(const std::vector<long double> &K, const TcGeom &g, int sk)
+{
+    const std::vector<long double> M = tc_blocks(K, g.n, g.nb, g.hb);
+    const int kq = 10 * sk - (g.nb == 4 ? 0 : 1);
+    std::vector<uint16_t> T((size_t)g.nb * g.hp * g.nchunks * g.w * sk, 0);
+    for (int b = 0; b < g.nb; ++b)
+        for (int i = 0; i < g.hb; ++i)
+            for (int j = 0; j < g.hb; ++j) {
+                long long v = llroundl(ldexpl(M[((size_t)b * g.hb + i) * g.hb + j], kq));
+                const int c = i / g.w, o = i - c * g.w, wc = g.w;
+                const size_t chunk = (size_t)g.nb * g.hp * sk * ((size_t)c * g.w);
+                const size_t step = chunk + ((size_t)b * (g.hp / 16) + j / 16) * ((size_t)sk * wc * 16);
+                for (int d = sk - 1; d >= 0; --d) { /* lowest digit first */
+                    long long q = d > 0 ? ((v + 512) & 1023) - 512 : v;
+                    v = (v - q) >> 10;
+                    const int row = d * wc + o, k = j & 15;
+                    T[step + (size_t)(row / 8) * 128 + (k / 8) * 64 + (row % 8) * 8 + k % 8] = half_of_int((int)q);
+                }
+            }
+    return T;
+}
+
+/* Test hook: the operator a tensor-core pass applies, decoded from its digits
+ * (kept levels or not: the digits' value), and the operator itself, n x n
+ * row-major; periodic axes of length 4k use four blocks. */
+extern "C" int scft_tc_operator(int n, double alpha, int dirichlet, int prec, double *k_eff, double *k_ref)
+{
+    if (n < 2 || !k_eff || !k_ref) return SCFT_ERR_PARAM;
+    TcGeom g;
+    tc_shape(n, dirichlet, g);
+    std::vector<long double> K;
+    dense_operator(n, alpha, dirichlet, K);
+    const int sk = tc_sk(prec), m = n / 2;
+    const std::vector<uint16_t> T = tc_table(K, g, sk);
+    auto digit = [](uint16_t h) {
+        const int e = (h >> 10) & 31;
+        const long double v = e ? ldexpl(1024 + (h & 0x3ff), e - 25) : ldexpl(h & 0x3ff, -24);
+        return (h & 0x8000) ? -v : v;
+    };
+    const int kq = 10 * sk - (g.nb == 4 ? 0 : 1);
+    auto value = [&](int b, int i, int j) {
+        const int c = i / g.w, o = i - c * g.w, wc = g.w;
+        const size_t step = (size_t)g.nb * g.hp * sk * ((size_t)c * g.w) +
+                            ((size_t)b * (g.hp / 16) + j / 16) * ((size_t)sk * wc * 16);
+        long double v = 0.0L;
+        for (int d = 0; d < sk; ++d) {
+            const int row = d * wc + o, k = j & 15;
+            v = v * 1024.0L + digit(T[step + (size_t)(row / 8) * 128 + (k / 8) * 64 + (row % 8) * 8 + k % 8]);
+        }
+        return ldexpl(v, -kq);
+    };
+    auto side = [&](int p, int k) { return g.nb == 2 ? (p ? n - 1 - k : k) : p == 0 ? k : p == 1 ? m - 1 - k : p == 2 ? k + m : n - 1 - k; };
+    for (size_t u = 0; u < (size_t)n * n; ++u) {
+        k_eff[u] = 0.0;
+        k_ref[u] = (double)K[u];
+    }
+    for (int i = 0; i < g.hb; ++i)
+        for (int j = 0; j < g.hb; ++j)
+            for (int pi = 0; pi < g.nb; ++pi)
+                for (int pj = 0; pj < g.nb; ++pj) {
+                    long double s = 0.0L;
+                    for (int b = 0; b < g.nb; ++b) {
+                        /* sign of side p in block b: mirror parity b & 1, half-axis parity b >> 1 */
+                        const int sg = ((b & 1) & (pi & 1)) ^ ((b >> 1) & (pi >> 1)) ^ ((b & 1) & (pj & 1)) ^ ((b >> 1) & (pj >> 1));
+                        s += sg ? -value(b, i, j) : value(b, i, j);
+                    }
+                    k_eff[(size_t)side(pi, i) * n + side(pj, j)] += (double)((2 * i + 1 == n && pi) ? 0.0L : s);
+                }
+    return SCFT_OK;
+}
+
+/* Sets a tile and a number of parts; 0 if the parts do not divide the chunks into
+ * equal runs or the digits do not fit in shared memory. */
+static int tc_apply(int prec, TcGeom &g, int tile, int parts, int smem_limit)
+{
+    g.tile = tile;
+    g.parts = parts;
+    g.cpp = (g.nchunks + parts - 1) / parts;
+    if ((g.nchunks + g.cpp - 1) / g.cpp != parts) return 0;
+    g.op_part = (unsigned)((size_t)g.nb * g.hp * tc_sk(prec) * g.cpp * g.w * 2);
+    g.mag_nk8 = (unsigned)((0xFFFFFFFFull + g.hp / 8) / (g.hp / 8));
+    return scft_pass_tc_fits(prec, g, smem_limit);
+}
+
+struct TcChoice {
+    int tile, parts;
+    int key() const { return tile + 1000 * parts; }
+    double cost;
+};
+/* Clocks of a tile, roughly: loading and splitting per item of 2 NB points, 20 per
+ * MMA (16 is the rate), joining and writing the outputs. In the loop (512 threads)
+ * a warp multiplies one block at a time, in a pass of its own (256) all blocks. */
+static double tc_cta_cost(const TcGeom &g, int prec, int threads)
+{
+    const double items = std::ceil(g.tile * (g.hp / 2) / (double)threads), mmas = prec == SCFT_PREC_FP32 ? 9.0 : 21.0;
+    const double block = g.hp / 16 * mmas * 20.0 + 300.0, work = (g.tile + 15) / 16 * g.cpp, warps = threads / 32.0;
+    if (threads == 512) /* loop: a block at a time, then the outputs */
+        return 2000.0 + items * g.nb * 350.0 + std::ceil(work * g.nb / warps) * block +
+               std::ceil(g.tile * g.cpp * 8 / (double)threads) * g.nb * 300.0;
+    return 2000.0 + items * g.nb * 350.0 + std::ceil(work / warps) * g.nb * (block + 500.0);
+}
+
+/* Tiles and output parts of a pass, cheapest first: lines per CTA in steps of 16,
+ * chunks shared by 1..nchunks CTAs. An in-place pass (neither first nor last) has
+ * one part: another part's CTA could overwrite a line before this one has read it.
+ * The autotuner times the cheapest twelve. */
+static std::vector<TcChoice> tc_choices(const scft_ctx *c, const TcGeom &g0, int inplace, int smem_limit)
+{
+    std::vector<TcChoice> out;
+    const int prec = c->opt.precision;
+    const long chains = (long)c->B * c->nchains;
+    static const int tiles[] = {8, 16, 32, 48, 64, 80, 96, 112, 128};
+    for (int t : tiles) {
+        if (t > 8 && (long)t - 8 >= (g0.lines + 7) / 8 * 8) continue; /* more rows than lines */
+        for (int parts = 1; parts <= (inplace ? 1 : g0.nchunks); ++parts) {
+            TcGeom g = g0;
+            if (!tc_apply(prec, g, t, parts, smem_limit)) continue;
+            const double ctas = (double)((g.lines + t - 1) / t) * parts * chains;
+            /* two CTAs per SM where they fit: each takes ~1.5 times as long as alone */
+            const bool two = 2 * scft_pass_tc_smem(prec, g) + 2048 <= (size_t)smem_limit;
+            out.push_back({t, parts, std::ceil(ctas / (two ? 2.0 * c->sms : c->sms)) * (two ? 1.5 : 1.0) *
+                                         (4000.0 + tc_cta_cost(g, prec, 256))});
+        }
+    }
+    std::stable_sort(out.begin(), out.end(), [](const TcChoice &x, const TcChoice &y) { return x.cost < y.cost; });
+    return out;
+}
+
+
 /* Operator tables of one grid axis (pass slot ai) for one operator set. */
 static int axis_tables(scft_ctx *c, const Axis &A, double alpha, InstOps &o, int ai)
 {
     const int n = A.g.n;
+    if (A.tc) {
+        std::vector<long double> K;
+        dense_operator(n, alpha, A.dirichlet, K);
+        void *td = nullptr;
+        int rc = upload(c, &td, tc_table(K, A.t, tc_sk(c->opt.precision)));
+        if (rc) return rc;
+        o.tc[ai] = td;
+        return SCFT_OK;
+    }
     if (!A.dirichlet_dense) {
         std::vector<double> spec(n), tw(2 * n);
         for (int t = 0; t < n; ++t) {
@@ -708,6 +912,10 @@ static int build_axes(scft_ctx *c)
     }
     int optin_limit = 0;
     CK(cudaDeviceGetAttribute(&optin_limit, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device));
+    const int naxes = (dims[0] > 1) + (dims[1] > 1) + (dims[2] > 1);
+    const int fused = c->opt.kernel_path == 0 &&
+                      ((d.ny == 1 && scft_step2d_smem(c->opt.precision, d.nx, d.nz) > 0) ||
+                       (!c->surf[0].mask && scft_step3d_smem(c->opt.precision, d.nx, d.ny, d.nz) > 0));
     for (int ax = 0; ax < 3; ++ax) {
         const int n = dims[ax];
         if (n <= 1) continue;
@@ -751,6 +959,20 @@ static int build_axes(scft_ctx *c)
         }
         A.ntiles = (int)(lines / A.tile);
         const int ai = (int)c->axes.size();
+        /* Tensor-core form: every pass that a fused loop does not replace, for
+         * lines of 8 points and more whose digits and operator fit in shared
+         * memory (periodic up to 256 points, Dirichlet up to 160 in FP64). */
+        if (!fused && n >= 8 && c->m < (1L << 30)) {
+            tc_shape(n, A.dirichlet, A.t);
+            A.t.ls = A.g.ls;
+            A.t.inner = A.g.inner;
+            A.t.lines = lines;
+            const std::vector<TcChoice> ch = tc_choices(c, A.t, naxes == 3 && ai == 1, optin_limit);
+            if (!ch.empty()) {
+                A.tc = 1;
+                tc_apply(c->opt.precision, A.t, ch[0].tile, ch[0].parts, optin_limit);
+            }
+        }
         for (size_t u = 0; u < rep.size(); ++u) {
             const scft_derived &dr = c->der[rep[u]];
             const double alpha = ax == 0 ? dr.alphax : (ax == 1 ? dr.alphay : dr.alphaz);
@@ -761,7 +983,82 @@ static int build_axes(scft_ctx *c)
     }
     /* the limit is a cap, not a reservation: set the device maximum once */
     CK(scft_pass_configure(optin_limit));
+    CK(scft_pass_tc_configure(optin_limit));
     return SCFT_OK;
+}
+
+/* Cluster contour loop: for each cluster size the tiles and parts of every axis
+ * with the lowest cost of a step (clocks), such that every axis' operator part
+ * and the largest tile fit in shared memory together. */
+static double tc_loop_plan(const scft_ctx *c, int cluster, int smem_limit, TcLoop &best)
+{
+    const int nax = (int)c->axes.size(), prec = c->opt.precision;
+    std::vector<std::pair<double, TcGeom>> cand[3];
+    for (int ax = 0; ax < nax; ++ax) {
+        const TcGeom &g0 = c->axes[ax].t;
+        for (int t = 8; t <= 128; t += t < 16 ? 8 : 16) {
+            if (t > 16 && (long)t - 16 >= g0.lines) continue;
+            for (int parts = 1; parts <= std::min(cluster, g0.nchunks); ++parts) {
+                if (parts > 1 && ax > 0 && ax < nax - 1) continue; /* in place */
+                TcGeom g = g0;
+                if (!tc_apply(prec, g, t, parts, smem_limit)) continue;
+                const long slots = cluster / parts, tiles = (g.lines + t - 1) / t;
+                cand[ax].push_back({(double)((tiles + slots - 1) / slots) * tc_cta_cost(g, prec, 512) + 1500.0, g});
+            }
+        }
+        std::stable_sort(cand[ax].begin(), cand[ax].end(), [](const std::pair<double, TcGeom> &x, const std::pair<double, TcGeom> &y) { return x.first < y.first; });
+        if (cand[ax].size() > 24) cand[ax].resize(24);
+        if (cand[ax].empty()) return -1.0;
+    }
+    for (int ax = nax; ax < 3; ++ax) cand[ax].push_back({0.0, TcGeom()});
+    double cost = -1.0;
+    for (auto &x : cand[0])
+        for (auto &y : cand[1])
+            for (auto &z : cand[2]) {
+                const double t = x.first + y.first + z.first;
+                if (cost >= 0.0 && t >= cost) break;
+                TcLoop lp;
+                memset(&lp, 0, sizeof(lp));
+                lp.nax = nax;
+                lp.cluster = cluster;
+                lp.g[0] = x.second;
+                lp.g[1] = y.second;
+                lp.g[2] = z.second;
+                if (scft_chain_tc_layout(prec, lp) > (size_t)smem_limit) continue;
+                cost = t;
+                best = lp;
+            }
+    return cost;
+}
+
+struct LoopChoice {
+    double cost; /* clocks of an iteration's contour steps */
+    int resident; /* clusters that fit on the GPU */
+    TcLoop lp;
+};
+static std::vector<LoopChoice> tc_loops(const scft_ctx *c, int smem_limit)
+{
+    std::vector<LoopChoice> out;
+    for (const Axis &A : c->axes)
+        if (!A.tc) return out;
+    if (c->axes.empty() || c->opt.kernel_path != 0) return out;
+    double steps = 0.0;
+    for (const ChainDesc &cd : c->chains_h) steps += cd.len - 1;
+    for (int cluster = 1; cluster <= 16; cluster *= 2) {
+        LoopChoice ch;
+        const double per = tc_loop_plan(c, cluster, smem_limit, ch.lp);
+        if (per < 0.0) continue;
+        Step2DArgs a;
+        memset(&a, 0, sizeof(a));
+        ch.resident = 0;
+        if (scft_launch_chain_tc(c->opt.precision, ch.lp, a, 1, c->stream, &ch.resident) != cudaSuccess || ch.resident < 1) {
+            cudaGetLastError();
+            continue;
+        }
+        ch.cost = per * std::max((double)(c->maxlen - 1), steps / std::min((double)ch.resident, (double)c->chains_h.size()));
+        out.push_back(ch);
+    }
+    return out;
 }
 
 /* ------------------------------------------------------------ autotuner */
@@ -775,6 +1072,8 @@ static int build_axes(scft_ctx *c)
  * precision, axis geometry and number of chains. */
 static std::mutex g_tune_mu;
 static std::map<std::string, int> g_tune_cache;
+
+static int launch_steps(scft_ctx *c, const ChainDesc *chains, int nchains_total, int maxlen);
 
 static int autotune_axes(scft_ctx *c)
 {
@@ -791,6 +1090,14 @@ static int autotune_axes(scft_ctx *c)
         Axis &A = c->axes[ai];
         const long lines = c->m / A.g.n;
         const long divisor = A.src == 2 ? lines : A.g.inner;
+        auto adopt = [&](int choice) {
+            if (A.tc) {
+                tc_apply(c->opt.precision, A.t, choice % 1000, choice / 1000, optin);
+            } else {
+                A.tile = choice;
+                A.ntiles = (int)(lines / A.tile);
+            }
+        };
         char key[160];
         snprintf(key, sizeof(key), "%d|%d,%d,%d,%d,%d|%d|%d", c->opt.precision, A.g.n, A.g.ls, A.g.inner, A.g.outer,
                  A.g.dirichlet, total, ai == 0 ? 1 : (ai == npass - 1 ? 2 : 0));
@@ -798,21 +1105,27 @@ static int autotune_axes(scft_ctx *c)
             std::lock_guard<std::mutex> lk(g_tune_mu);
             auto it = g_tune_cache.find(key);
             if (it != g_tune_cache.end()) {
-                A.tile = it->second;
-                A.ntiles = (int)(lines / A.tile);
+                adopt(it->second);
                 continue;
             }
         }
         /* every divisor up to 64 (even ones for the FFT passes), not only powers of
          * two: with few chains (a single solve) a tile that gives about one CTA per
          * SM avoids a second, mostly empty wave */
+        /* a candidate: lines per CTA, and for a tensor-core pass the output parts
+         * (tile + 1000 * parts) */
         std::vector<int> cand;
-        for (int t = A.g.dirichlet ? 1 : 2; t <= 64; t += A.g.dirichlet ? 1 : 2)
-            if (divisor % t == 0 && lines / t >= 1 && scft_pass_smem_bytes(A.g, t, A.h, c->psize) <= (size_t)optin)
-                cand.push_back(t);
+        if (A.tc) {
+            const std::vector<TcChoice> ch = tc_choices(c, A.t, ai > 0 && ai < npass - 1, optin);
+            for (size_t k = 0; k < ch.size() && k < 12; ++k) cand.push_back(ch[k].key());
+        } else {
+            for (int t = A.g.dirichlet ? 1 : 2; t <= 64; t += A.g.dirichlet ? 1 : 2)
+                if (divisor % t == 0 && lines / t >= 1 && scft_pass_smem_bytes(A.g, t, A.h, c->psize) <= (size_t)optin)
+                    cand.push_back(t);
+        }
+        int best = A.tc ? TcChoice{A.t.tile, A.t.parts, 0.0}.key() : A.tile;
         if (cand.size() > 1) {
             float best_ms = 1e30f;
-            int best = A.tile;
             for (int t : cand) {
                 PassArgs pa;
                 memset(&pa, 0, sizeof(pa));
@@ -826,10 +1139,15 @@ static int autotune_axes(scft_ctx *c)
                 pa.axis = ai;
                 pa.h = A.h;
                 pa.even = A.even;
-                const int nt = (int)(lines / t);
-                cudaError_t e = scft_launch_pass(c->opt.precision, A.g, pa, nt, c->stream); /* warm-up */
+                const int nt = A.tc ? 0 : (int)(lines / t);
+                if (A.tc) adopt(t);
+                auto launch = [&]() {
+                    return A.tc ? scft_launch_pass_tc(c->opt.precision, A.t, pa, c->stream)
+                                : scft_launch_pass(c->opt.precision, A.g, pa, nt, c->stream);
+                };
+                cudaError_t e = launch(); /* warm-up */
                 if (e == cudaSuccess) e = cudaEventRecord(e0, c->stream);
-                for (int r = 0; r < 3 && e == cudaSuccess; ++r) e = scft_launch_pass(c->opt.precision, A.g, pa, nt, c->stream);
+                for (int r = 0; r < 3 && e == cudaSuccess; ++r) e = launch();
                 if (e == cudaSuccess) e = cudaEventRecord(e1, c->stream);
                 if (e == cudaSuccess) e = cudaEventSynchronize(e1);
                 float ms = 0.f;
@@ -844,15 +1162,101 @@ static int autotune_axes(scft_ctx *c)
                     best = t;
                 }
             }
-            A.tile = best;
-            A.ntiles = (int)(lines / A.tile);
         }
+        adopt(best);
         std::lock_guard<std::mutex> lk(g_tune_mu);
-        g_tune_cache[key] = A.tile;
+        g_tune_cache[key] = best;
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     return rc;
+}
+
+/* Contour steps by the cluster loop or by a launch per pass, the same arithmetic
+ * either way: the loop saves launches and set-up, the passes spread every step
+ * over all SMs. With the autotuner a few steps of each are timed on the context's
+ * chains (every chain runs them); the time of an iteration follows from the
+ * clusters that are resident together, or for the passes from the number of
+ * chains still running if they fill the GPU. Without it the estimates decide,
+ * the loop's doubled: with more clusters than the GPU holds it measured twice
+ * its estimate (192x96, 160 chains). */
+static int choose_loop_tc(scft_ctx *c)
+{
+    int optin = 0;
+    CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device));
+    std::vector<LoopChoice> ch = tc_loops(c, optin);
+    if (ch.empty()) return SCFT_OK;
+    const int npass = (int)c->axes.size(), nch = (int)c->chains_h.size(), last = c->maxlen - 1;
+    double total = 0.0, passes = 0.0, ctas = 0.0;
+    for (const ChainDesc &cd : c->chains_h) total += cd.len - 1;
+    for (int ai = 0; ai < npass; ++ai) {
+        const TcGeom &g = c->axes[ai].t;
+        const std::vector<TcChoice> p = tc_choices(c, g, ai > 0 && ai < npass - 1, optin);
+        passes += last * p[0].cost;
+        ctas += (double)((g.lines + g.tile - 1) / g.tile) * g.parts * nch / npass;
+    }
+    int best = -1;
+    if (c->opt.autotune && last > 0) {
+        char key[200];
+        snprintf(key, sizeof(key), "loop|%d|%d,%d,%d|%d|%d|%d,%.0f", c->opt.precision, c->nx, c->ny, c->nz,
+                 c->axes.back().dirichlet, nch, c->maxlen, total);
+        {
+            std::lock_guard<std::mutex> lk(g_tune_mu);
+            auto it = g_tune_cache.find(key);
+            if (it != g_tune_cache.end()) {
+                for (size_t k = 0; k < ch.size(); ++k)
+                    if (ch[k].lp.cluster == it->second) {
+                        c->loop_tc = 1;
+                        c->loop = ch[k].lp;
+                    }
+                return SCFT_OK;
+            }
+        }
+        const int steps = std::min(4, last);
+        cudaEvent_t e0 = nullptr, e1 = nullptr;
+        CK(cudaEventCreate(&e0));
+        CK(cudaEventCreate(&e1));
+        double best_t = 1e300;
+        int rc = SCFT_OK;
+        for (int k = -1; k < (int)ch.size() && rc == SCFT_OK; ++k) {
+            if (k >= 0 && ch[k].cost > 3.0 * passes) continue;
+            c->loop_tc = k >= 0;
+            if (k >= 0) c->loop = ch[k].lp;
+            float ms = 0.f;
+            rc = launch_steps(c, c->chains, nch, steps + 1); /* warm-up */
+            if (rc == SCFT_OK && cudaEventRecord(e0, c->stream) != cudaSuccess) rc = SCFT_ERR_CUDA;
+            for (int r = 0; r < 2 && rc == SCFT_OK; ++r) rc = launch_steps(c, c->chains, nch, steps + 1);
+            if (rc == SCFT_OK && (cudaEventRecord(e1, c->stream) != cudaSuccess || cudaEventSynchronize(e1) != cudaSuccess ||
+                                  cudaEventElapsedTime(&ms, e0, e1) != cudaSuccess)) {
+                set_err("autotune: %s", cudaGetErrorString(cudaGetLastError()));
+                rc = SCFT_ERR_CUDA;
+            }
+            if (rc) break;
+            const double waves = k < 0 ? 1.0 : std::ceil((double)nch / ch[k].resident), step = ms / 2 / steps / waves;
+            const double t = k < 0 ? step * (ctas > 2.0 * c->sms ? total / nch : last)
+                                   : step * std::max((double)last, total / std::min(nch, ch[k].resident));
+            if (t < best_t) {
+                best_t = t;
+                best = k;
+            }
+        }
+        cudaEventDestroy(e0);
+        cudaEventDestroy(e1);
+        if (rc) return rc;
+        std::lock_guard<std::mutex> lk(g_tune_mu);
+        g_tune_cache[key] = best < 0 ? 0 : ch[best].lp.cluster;
+    } else {
+        for (size_t k = 0; k < ch.size(); ++k) {
+            const double cost = ch[k].cost * (nch > ch[k].resident ? 2.0 : 1.3);
+            if (cost < passes) {
+                passes = cost;
+                best = (int)k;
+            }
+        }
+    }
+    c->loop_tc = best >= 0;
+    if (best >= 0) c->loop = ch[best].lp;
+    return SCFT_OK;
 }
 
 /* The fused 2D contour loop's launch form: one or two threads per line (every
@@ -1236,10 +1640,6 @@ extern "C" int scft_ctx_create(const scft_surface *surfaces, const scft_options 
         }
     }
 #undef ALLOC
-    if (opt.autotune && !c->fused2d && !c->fused3d && (rc = autotune_axes(c))) {
-        scft_ctx_destroy(c);
-        return rc;
-    }
     {
         /* longest chains first, so the persistent launch ends with short ones */
         std::vector<int> ord((size_t)B * c->nchains);
@@ -1251,6 +1651,14 @@ extern "C" int scft_ctx_create(const scft_surface *surfaces, const scft_options 
             return rc;
         }
     }
+    if (opt.autotune && !c->fused2d && !c->fused3d && (rc = autotune_axes(c))) {
+        scft_ctx_destroy(c);
+        return rc;
+    }
+    if (!c->fused2d && !c->fused3d && (rc = choose_loop_tc(c))) {
+        scft_ctx_destroy(c);
+        return rc;
+    }
     if (opt.autotune && c->fused2d && (rc = autotune_fused2d(c))) {
         scft_ctx_destroy(c);
         return rc;
@@ -1258,7 +1666,7 @@ extern "C" int scft_ctx_create(const scft_surface *surfaces, const scft_options 
     c->iter.assign(B, 0);
     c->rng.assign(3 * B, 0);
     c->fields_set.assign(B, 0);
-    c->prop_launches_per_iter = (c->fused2d || c->fused3d) ? 1L : (long)(c->maxlen - 1) * (long)c->axes.size();
+    c->prop_launches_per_iter = (c->fused2d || c->fused3d || c->loop_tc) ? 1L : (long)(c->maxlen - 1) * (long)c->axes.size();
     c->launches_per_iter = c->prop_launches_per_iter + 2 + 6 + (opt.noise_mode == SCFT_NOISE_DRAND48 ? 5 : 0);
     if (cudaStreamSynchronize(c->stream) != cudaSuccess) {
         set_err("context set-up failed: %s", cudaGetErrorString(cudaGetLastError()));
@@ -1526,6 +1934,17 @@ static int launch_steps(scft_ctx *c, const ChainDesc *chains, int nchains_total,
             CK(scft_launch_step2d(c->opt.precision, c->nx, c->nz, a, nchains_total, c->stream, 0, c->wide2d));
         return SCFT_OK;
     }
+    if (c->loop_tc) {
+        Step2DArgs a;
+        a.chains = chains;
+        a.order = (chains == c->chains) ? c->order : nullptr;
+        a.state = (chains == c->chains) ? c->state : nullptr;
+        a.s = 0;
+        a.s_end = maxlen - 1;
+        a.sstride = c->sm;
+        CK(scft_launch_chain_tc(c->opt.precision, c->loop, a, nchains_total, c->stream, nullptr));
+        return SCFT_OK;
+    }
     const int npass = (int)c->axes.size();
     for (int s = 0; s < maxlen - 1; ++s) {
         for (int pi = 0; pi < npass; ++pi) {
@@ -1543,7 +1962,10 @@ static int launch_steps(scft_ctx *c, const ChainDesc *chains, int nchains_total,
             pa.axis = pi;
             pa.h = A.h;
             pa.even = A.even;
-            CK(scft_launch_pass(c->opt.precision, A.g, pa, A.ntiles, c->stream));
+            if (A.tc)
+                CK(scft_launch_pass_tc(c->opt.precision, A.t, pa, c->stream));
+            else
+                CK(scft_launch_pass(c->opt.precision, A.g, pa, A.ntiles, c->stream));
         }
     }
     return SCFT_OK;
@@ -1658,7 +2080,9 @@ static int collect_chunk(scft_ctx *c, scft_iter_out *out)
     if (chunk > 0)
         for (int b = 0; b < c->B; ++b) c->iter[b] = c->hist_host[(size_t)(chunk - 1) * c->B + b].iter;
     if (status != SCFT_OK) {
-        if (c->fused2d && scft_step2d_take_fault())
+        int tc = c->fused2d;
+        for (const Axis &A : c->axes) tc |= A.tc;
+        if (tc && (scft_step2d_take_fault() | scft_pass_tc_take_fault()))
             set_err("non-finite Q, free energy or RMS (a tensor-core wait of the contour loop gave up)");
         else
             set_err("non-finite Q, free energy or RMS");

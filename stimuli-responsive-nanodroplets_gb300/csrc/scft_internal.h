@@ -33,6 +33,7 @@
 struct InstOps {
     const void *kz, *twx, *ex;
     const void *spec[3], *tw[3], *kA[3], *kB[3];
+    const void *tc[3]; /* operator digits of the tensor-core passes */
 };
 
 /* One propagator chain of one instance: q[0] from init, then len-1 contour
@@ -133,6 +134,40 @@ struct PassArgs {
 size_t scft_pass_smem_bytes(const AxisGeom &g, int tile, int h, int psize);
 cudaError_t scft_pass_configure(int smem_bytes);
 cudaError_t scft_launch_pass(int prec, const AxisGeom &g, const PassArgs &a, int ntiles, cudaStream_t st);
+
+/* Geometry of one axis pass on the tensor cores (scft_pass_tc.cu). The line's
+ * points fall into nb blocks of hb points (padded to hp, a multiple of 16); the
+ * operator's digits are stored per chunk of w block outputs, and `parts` CTAs
+ * share a tile of lines, each taking cpp chunks. */
+struct TcGeom {
+    int n, ls, inner;
+    long lines;
+    int nb, hb, hp;
+    int w, nchunks;
+    int tile, parts, cpp;
+    unsigned op_part;  /* bytes of operator digits a CTA holds */
+    unsigned mag_nk8;  /* ceil(2^32 / d), d = hp / 8 */
+};
+
+/* The cluster-resident contour loop over the same tiles (k_chain_tc). */
+struct TcLoop {
+    int nax, cluster; /* axes, CTAs per cluster */
+    TcGeom g[3];
+    int slots[3];      /* tiles taken side by side: cluster / parts */
+    unsigned op_at[3]; /* shared-memory offsets of the axes' operator digits and of the tile region */
+    unsigned tile_at;
+};
+
+size_t scft_pass_tc_smem(int prec, const TcGeom &g);
+int scft_pass_tc_fits(int prec, const TcGeom &g, int smem_limit);
+cudaError_t scft_pass_tc_configure(int smem_bytes);
+cudaError_t scft_launch_pass_tc(int prec, const TcGeom &g, const PassArgs &a, cudaStream_t st);
+struct Step2DArgs;
+size_t scft_chain_tc_layout(int prec, TcLoop &lp);
+cudaError_t scft_launch_chain_tc(int prec, const TcLoop &lp, const Step2DArgs &a, int nchains, cudaStream_t st,
+                                 int *clusters);
+/* 1 if a tensor-core wait of a pass gave up since the last call (clears it) */
+int scft_pass_tc_take_fault(void);
 
 /* Arguments shared by the non-propagator kernels (scft_post.cu). */
 struct PostArgs {

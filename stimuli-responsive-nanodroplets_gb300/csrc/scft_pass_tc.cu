@@ -1,0 +1,806 @@
+/*
+ * scft_pass_tc.cu — one axis pass of the contour step on the tensor cores, with
+ * the rounding of the value type: y = K x for every line of one grid axis, K the
+ * dense diffusion operator of that axis (funPDESolver_periodic and
+ * funPDESolver_DirichletBC, SCFT.c:2474-2631, apply the same factor by FFTs).
+ *
+ * GB300 issues FP64 at 1/58 of its FP32 rate and a double-float product costs
+ * 8-12 FP32 instructions, so a pass in either arithmetic is bound by its
+ * multiply-adds (192x96 film: 85 % of the FP64 rate in the dense z pass at
+ * large batches, 3 % of the copy bandwidth). Here the contraction runs on the
+ * fp16 tensor cores without rounding, by the splitting scheme of Ozaki, Ogita,
+ * Oishi and Rump ("Error-free transformations of matrix multiplication by using
+ * fast routines of matrix multiplication and its applications", Numer. Algor.
+ * 59, 2012):
+ *   - a line becomes integers X = x 2^e with one exponent per line (58 bits
+ *     for FP64 and FP32x2 values, 28 for FP32);
+ *   - the operator commutes with the reversal of the axis and, on a periodic
+ *     axis of length 4k, with the shift by half its length: integer sums and
+ *     differences split it into NB = 2 or 4 blocks of size n/NB, exactly;
+ *   - block operands and operators are cut into balanced digits of 10 bits,
+ *     which fp16 holds exactly; a product of two digit matrices with
+ *     |digit| <= 512 sums to an integer below 2^24 that the FP32 accumulators
+ *     hold exactly. Digit pairs (i, j) with i + j = l share the accumulator of
+ *     level l; the levels kept (6 of FP64's, 4 of FP32's) leave out terms of
+ *     2^-56 (2^-27) of the line's largest value;
+ *   - the levels are joined in 64-bit integers (FP32: three multiply-adds), and
+ *     each output is rounded once to the value type.
+ * Results do not depend on the tile, the number of output parts or what shares
+ * the launch: every line is computed by the same integer arithmetic.
+ *
+ * A CTA takes `tile` lines and a range of output chunks. Data digits and
+ * operator digits sit in shared memory as 8 x 16-byte cells, which ldmatrix
+ * reads without conflicts; a warp multiplies 16 lines x 8 outputs with
+ * mma.sync and joins the levels in its own registers. The same products by
+ * tcgen05.mma (accumulators in tensor memory, 64 or 128 lines) measured slower
+ * at every size tried: the MMAs of a chunk of 16 outputs took 1100-2000 clocks
+ * from issue to completion, the accumulators (24 words for 4 outputs) had to
+ * pass through shared memory to reach all warps (1200 clocks), and a tile fills
+ * 8-48 of the 64 rows. 192x96 film, FP64, 32 instances: 16.3 ms an iteration
+ * against 12.7; 64^3 blend: 18.4 against 14.3. The passes are bound by the
+ * integer pipe (splitting, joining: ~100 operations per value, 2 issue slots
+ * each) and by the rate of mma.sync (16 clocks each).
+ * Measured against the FP64 and double-float passes (FFT along periodic axes,
+ * dense products along the others), ms per iteration, contour steps and all:
+ * 192x96 film, one FP64 instance 4.36 -> 1.49, 32 FP64 instances 45.8 -> 12.7,
+ * 16 FP32x2 instances 11.4 -> 6.1; 64^3 four-diblock blend, FP64, 55.9 -> 15.2;
+ * 150x75 film, FP32, 4 instances 2.65 -> 1.8. Errors against 64-bit references
+ * are no larger than before in every form.
+ *
+ * A line with a NaN or an infinity comes out as NaN.
+ */
+#include <cuda_fp16.h>
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+#include <type_traits>
+
+#include "scft_dfloat.cuh"
+#include "scft_internal.h"
+#include "scft_mbar.cuh"
+
+/* Set when a tensor-core wait of a pass gave up (the tile is then written as NaN). */
+__device__ int g_scft_pass_fault;
+
+namespace {
+
+constexpr int W = 8;      /* block outputs of a chunk (the N of an MMA) */
+constexpr int ROWS = 128; /* lines of the largest tile */
+
+/* digits of the data, of the operator, and levels kept */
+template <typename P>
+struct Dig {
+    static constexpr int S = 6, SK = 6, L = 6;
+};
+template <>
+struct Dig<float> {
+    static constexpr int S = 3, SK = 4, L = 4;
+};
+
+template <typename P>
+struct FixT {
+    using T = long long;
+};
+template <>
+struct FixT<float> {
+    using T = int;
+};
+
+/* biased exponent of a value (0: zero or subnormal, taken as zero) */
+__device__ __forceinline__ int expo(double x) { return (__double2hiint(x) >> 20) & 0x7ff; }
+__device__ __forceinline__ int expo(dfloat x) { return (__float_as_int(x.hi) >> 23) & 0xff; }
+__device__ __forceinline__ int expo(float x) { return (__float_as_int(x) >> 23) & 0xff; }
+template <typename P>
+struct ExpoMax {
+    static constexpr int v = std::is_same<P, double>::value ? 2047 : 255; /* infinities and NaN */
+};
+
+/* x 2^s as an integer, s such that values below 2^(emax + 1 - bias) stay below
+ * 2^(58 - NB/4) (FP32: 2^(28 - NB/4), rounded to nearest; the others drop bits
+ * below that, of which a value within 2^-5 of the line's largest has none). A
+ * zero counts as 2^-bias, which every line but one of zeros shifts out, and a
+ * line of zeros comes out as zero. */
+template <int NB>
+__device__ __forceinline__ long long fix(double x, int emax)
+{
+    const int hi = __double2hiint(x);
+    const unsigned lo = (unsigned)__double2loint(x), h = ((unsigned)hi & 0xfffffu) | 0x100000u;
+    const long long m = (long long)(((unsigned long long)__funnelshift_l(lo, h, 10) << 32) | (lo << 10)); /* leading bit 62 */
+    const long long v = m >> min(emax - ((hi >> 20) & 0x7ff) + (NB == 4 ? 6 : 5), 63);
+    return hi < 0 ? -v : v;
+}
+template <int NB>
+__device__ __forceinline__ long long fix_part(float x, int emax)
+{
+    const int b = __float_as_int(x), e = (b >> 23) & 0xff;
+    const unsigned long long m = (unsigned long long)(((unsigned)b & 0x7fffffu) | 0x800000u) << (NB == 4 ? 33 : 34);
+    const int d = min(emax - e, 63); /* lo's exponent is never above hi's */
+    const long long v = e ? (long long)(m >> d) : 0;
+    return b < 0 ? -v : v;
+}
+template <int NB>
+__device__ __forceinline__ long long fix(dfloat x, int emax)
+{
+    return fix_part<NB>(x.hi, emax) + fix_part<NB>(x.lo, emax);
+}
+template <int NB>
+__device__ __forceinline__ int fix(float x, int emax)
+{
+    const int b = __float_as_int(x), e = (b >> 23) & 0xff;
+    const unsigned m = (((unsigned)b & 0x7fffffu) | 0x800000u) << (NB == 4 ? 3 : 4);
+    const int d = min(emax - e, 30);
+    const int v = e ? (int)((m + ((1u << d) >> 1)) >> d) : 0;
+    return b < 0 ? -v : v;
+}
+
+/* Digit i (0 = top) of two biased integers as a half2 of balanced digits: the
+ * fields' 16-bit windows side by side, masked, made 1024 + f in fp16, less 1536
+ * (the top field reaches 1024, so it has a mask of its own and is added). */
+template <int S, typename U>
+__device__ __forceinline__ uint32_t digit2(U ya, U yb, int i)
+{
+    const int bit = 10 * (S - 1 - i);
+    uint32_t t;
+    if (sizeof(U) == 8 && bit / 8 == 3) { /* the window straddles the words */
+        t = __byte_perm((uint32_t)(ya >> 24), (uint32_t)(yb >> 24), 0x5410);
+    } else {
+        const int word = sizeof(U) == 8 && bit >= 32 ? 1 : 0, byte = bit / 8 - 4 * word;
+        const uint32_t wa = word ? (uint32_t)((unsigned long long)ya >> 32) : (uint32_t)ya;
+        const uint32_t wb = word ? (uint32_t)((unsigned long long)yb >> 32) : (uint32_t)yb;
+        t = __byte_perm(wa, wb, byte == 0 ? 0x5410 : byte == 1 ? 0x6521 : 0x7632);
+    }
+    t >>= bit % 8;
+    t = i == 0 ? (t & 0x07ff07ffu) + 0x64006400u : (t & 0x03ff03ffu) | 0x64006400u;
+    const __half2 h = __hsub2(*reinterpret_cast<const __half2 *>(&t), __half2half2(__ushort_as_half(0x6600))); /* 1536 */
+    return *reinterpret_cast<const uint32_t *>(&h);
+}
+
+/* two consecutive values of a row, 16-byte aligned (FP32: 8) */
+__device__ __forceinline__ void ld2(const double *p, double (&v)[2])
+{
+    const double2 t = __ldcg(reinterpret_cast<const double2 *>(p));
+    v[0] = t.x;
+    v[1] = t.y;
+}
+__device__ __forceinline__ void ld2(const dfloat *p, dfloat (&v)[2])
+{
+    const float4 t = __ldcg(reinterpret_cast<const float4 *>(p));
+    v[0] = dfloat(t.x, t.y);
+    v[1] = dfloat(t.z, t.w);
+}
+__device__ __forceinline__ void ld2(const float *p, float (&v)[2])
+{
+    const float2 t = __ldcg(reinterpret_cast<const float2 *>(p));
+    v[0] = t.x;
+    v[1] = t.y;
+}
+__device__ __forceinline__ void st2(double *p, double a, double b) { *reinterpret_cast<double2 *>(p) = make_double2(a, b); }
+__device__ __forceinline__ void st2(dfloat *p, dfloat a, dfloat b)
+{
+    *reinterpret_cast<float4 *>(p) = make_float4(a.hi, a.lo, b.hi, b.lo);
+}
+__device__ __forceinline__ void st2(float *p, float a, float b) { *reinterpret_cast<float2 *>(p) = make_float2(a, b); }
+__device__ __forceinline__ double ld1(const double *p) { return __ldcg(p); }
+__device__ __forceinline__ float ld1(const float *p) { return __ldcg(p); }
+__device__ __forceinline__ dfloat ld1(const dfloat *p)
+{
+    const float2 t = __ldcg(reinterpret_cast<const float2 *>(p));
+    return dfloat(t.x, t.y);
+}
+
+/* four 8 x 8 matrices of 16-bit values from shared memory, rows of 16 bytes at each lane's address */
+__device__ __forceinline__ void ldsm4(uint32_t (&r)[4], uint32_t addr)
+{
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(addr)
+                 : "memory");
+}
+/* c += a b: 16 lines x 8 outputs x 16 points */
+__device__ __forceinline__ void mma16816(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1)
+{
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+
+__device__ __forceinline__ long long mad_wide(int a, int b, long long c)
+{
+    long long d;
+    asm("mad.wide.s32 %0, %1, %2, %3;" : "=l"(d) : "r"(a), "r"(b), "l"(c));
+    return d;
+}
+/* Levels of one block output joined: 64-bit integer in units of 2^60 of the
+ * digit products (level 5 rounds into level 4), FP32: a float in units of 2^50. */
+__device__ __forceinline__ long long join(const float (&d)[6][4], int v)
+{
+    long long y = __float2int_rn(fmaf(d[5][v], 0x1p-10f, d[4][v]));
+    y = mad_wide(__float2int_rn(d[3][v]), 1 << 10, y);
+    y = mad_wide(__float2int_rn(d[2][v]), 1 << 20, y);
+    y = mad_wide(__float2int_rn(d[1][v]), 1 << 30, y);
+    return y + ((long long)(__float2int_rn(d[0][v]) << 8) << 32);
+}
+__device__ __forceinline__ float join(const float (&d)[4][4], int v)
+{
+    return fmaf(fmaf(fmaf(d[3][v], 0x1p-10f, d[2][v]), 0x1p-10f, d[1][v]), 0x1p-10f, d[0][v]);
+}
+
+/* The joined value back in the value type, rounded once; the scales of fix() and
+ * of the operator table are folded into the exponents.
+ * FP64, the rare cases: a value below 2^-25 of its line's largest, exponents
+ * near the ends of the range, lines of zeros. */
+__device__ __noinline__ double from_fix_slow(long long acc, int emax)
+{
+    const unsigned long long u = acc < 0 ? (unsigned long long)-acc : (unsigned long long)acc;
+    if (emax < 64 || u == 0) return 0.0; /* below 2^-958 */
+    const int lz = __clzll((long long)u), eb = emax + 7 - lz; /* biased exponent */
+    const unsigned long long m = u << lz;
+    unsigned long long r = ((unsigned long long)(eb - 1) << 52) + (m >> 11) + ((m >> 10) & 1);
+    if (eb <= 0) r = 0;
+    if (eb >= 2047) r = 0x7ff0000000000000ull;
+    return __longlong_as_double((long long)(r | ((unsigned long long)acc & 0x8000000000000000ull)));
+}
+__device__ __forceinline__ void from_fix(long long acc, int emax, double &y)
+{
+    /* |acc| < 2^58; the integer pipe bounds this phase, so in 32-bit steps */
+    const unsigned long long u = (unsigned long long)(acc < 0 ? -acc : acc);
+    const unsigned hi = (unsigned)(u >> 32), lo = (unsigned)u;
+    if ((unsigned)(emax - 300) > 1400u || hi == 0) {
+        y = from_fix_slow(acc, emax);
+        return;
+    }
+    const int top = 31 - __clz((int)hi), k = 25 - top; /* leading bit to 57, then 53 bits */
+    unsigned h = __funnelshift_l(lo, hi, k), l = lo << k;
+    asm("add.cc.u32 %0, %0, 16;\n\taddc.u32 %1, %1, 0;" : "+r"(l), "+r"(h));
+    l = __funnelshift_r(l, h, 5);
+    h = (h >> 5) + (unsigned)(emax - 25 + top) * (1u << 20); /* the leading bit adds one to the exponent */
+    y = __hiloint2double((int)(h | ((unsigned)((unsigned long long)acc >> 32) & 0x80000000u)), (int)l);
+}
+__device__ __forceinline__ void from_fix(long long acc, int emax, dfloat &y)
+{
+    /* three signed pieces of 20 bits and what is above, exact in FP32 */
+    const int p0 = ((int)acc << 12) >> 12;
+    const long long a1 = (acc - p0) >> 20;
+    const int p1 = ((int)a1 << 12) >> 12;
+    const int p2 = (int)((a1 - p1) >> 20);
+    const dfloat s = dfo::fast_two_sum((float)p2 * 0x1p-16f, (float)p1 * 0x1p-36f);
+    const dfloat t = dfo::fast_two_sum(s.hi, dfo::f_add(s.lo, (float)p0 * 0x1p-56f));
+    const float sc = __int_as_float(emax << 23);
+    y = dfloat(t.hi * sc, t.lo * sc);
+}
+__device__ __forceinline__ void from_fix(float acc, int emax, float &y)
+{
+    y = (acc * 0x1p-16f) * __int_as_float(emax << 23);
+}
+
+__device__ __forceinline__ void set_nan(double &y) { y = __longlong_as_double(0x7ff8000000000000ll); }
+__device__ __forceinline__ void set_nan(dfloat &y) { y = dfloat(__int_as_float(0x7fc00000), __int_as_float(0x7fc00000)); }
+__device__ __forceinline__ void set_nan(float &y) { y = __int_as_float(0x7fc00000); }
+
+/* Shared memory (byte offsets): one barrier per axis, two sets of line exponents,
+ * operator digits (one region per axis), then the digits of a tile's lines. */
+constexpr uint32_t SM_BAR = 0, SM_FAIL = 32, SM_ELINE = 64, SM_OP = SM_ELINE + 2 * ROWS * 4;
+
+/* bytes of a tile's digits (an MMA reads 16 lines) */
+__host__ __device__ inline uint32_t tile_bytes(const TcGeom &g, int digits)
+{
+    return (uint32_t)((g.tile + 15) / 16 * 16) * g.hp * g.nb * digits * 2;
+}
+
+/* bytes of the exchange of block sums, for a part of the outputs */
+__host__ __device__ inline uint32_t exchange_bytes(const TcGeom &g, int value)
+{
+    return (uint32_t)((g.tile + 15) / 16 * 16) * (g.cpp * W * g.nb + 2) * value;
+}
+
+/* Where a CTA is. */
+struct TcPhase {
+    uint32_t tile; /* tiles done */
+    bool ok;       /* no wait has given up */
+};
+
+/* One tile of lines and one part of its outputs: y = K x (times b before the
+ * first axis, after the last). Ends with every thread of the CTA past the digits. */
+template <typename P, int NB, int NT, bool SPLIT>
+__device__ __forceinline__ void tc_tile(const TcGeom &g, const P *src, P *dst, const P *__restrict__ bz,
+                                        bool first, bool last, int tile_i, int part, unsigned char *smem,
+                                        uint32_t sm_op, uint32_t sm_a, uint32_t bar_op, TcPhase &ph)
+{
+    constexpr int S = Dig<P>::S, SK = Dig<P>::SK, L = Dig<P>::L;
+    using Fix = typename FixT<P>::T;
+    using UFix = typename std::make_unsigned<Fix>::type;
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0); /* uniform */
+    /* line exponents: one set in use, the other zeroed for the next tile */
+    int *eline = reinterpret_cast<int *>(smem + SM_ELINE) + (ph.tile & 1) * ROWS;
+    int *enext = reinterpret_cast<int *>(smem + SM_ELINE) + (~ph.tile & 1) * ROWS;
+    ++ph.tile;
+    const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(smem);
+    const int c0 = part * g.cpp, c1 = min(c0 + g.cpp, g.nchunks);
+    const int n = g.n, hb = g.hb, m = n / 2, ls = g.ls, nk8 = g.hp / 8;
+    const int L0 = tile_i * g.tile, nlines = (int)min((long)g.tile, g.lines - L0);
+    const bool vec = ls == 1 && n % 2 == 0; /* rows of whole pairs (n = 4 j for NB = 4) */
+    const int items = g.tile * nk8 * 4;
+    constexpr int CELL = S * NB * 128; /* one 8-line, 8-point core matrix of every digit and block */
+
+    /* first element of line r of the tile: rows (the axis is contiguous), columns of
+     * one plane (the slowest axis), or the general case */
+    auto line_base = [&](int r) {
+        const int line = L0 + r;
+        if (ls == 1) return line * n;
+        if (g.lines == g.inner) return line;
+        const int o = line / g.inner;
+        return o * n * ls + (line - o * g.inner);
+    };
+
+    /* position of point k of side p: 0 k, 1 its mirror; 2, 3 the same half an axis on (NB = 4) */
+    auto pos = [&](int p, int k) {
+        if (NB == 2) return p == 0 ? k : n - 1 - k;
+        return p == 0 ? k : p == 1 ? m - 1 - k : p == 2 ? k + m : n - 1 - k;
+    };
+
+    /* ---- load. An item is two neighbouring points (and their images) of one
+     * line; the warp's 32 items fill one 8-line core matrix of every digit. The
+     * values wait for the line's exponent in the words their digits will take. */
+#pragma unroll 1
+    for (int idx = tid; idx < items; idx += NT) {
+        const int u = idx >> 5, rg = nk8 == 1 ? u : (int)__umulhi((unsigned)u, g.mag_nk8), k8 = u - rg * nk8;
+        const int r = rg * 8 + ((idx >> 2) & 7), k = k8 * 8 + 2 * (idx & 3);
+        unsigned char *cell = smem + sm_a + u * CELL + (idx & 31) * 4;
+        P v[NB][2], bb[NB][2];
+        int em = 0;
+        const bool on = r < nlines && k < hb;
+        const int base = line_base(min(r, nlines - 1));
+        if (on && vec && k + 1 < hb) {
+#pragma unroll
+            for (int p = 0; p < NB; ++p) ld2(src + base + ((p & 1) ? pos(p, k + 1) : pos(p, k)), v[p]);
+            if (first) {
+#pragma unroll
+                for (int p = 0; p < NB; ++p) ld2(bz + base + ((p & 1) ? pos(p, k + 1) : pos(p, k)), bb[p]);
+            }
+#pragma unroll
+            for (int p = 1; p < NB; p += 2) {
+                P t = v[p][0];
+                v[p][0] = v[p][1];
+                v[p][1] = t;
+                t = bb[p][0];
+                bb[p][0] = bb[p][1];
+                bb[p][1] = t;
+            }
+        } else {
+#pragma unroll
+            for (int p = 0; p < NB; ++p)
+#pragma unroll
+                for (int q = 0; q < 2; ++q) {
+                    const bool in = on && k + q < hb;
+                    v[p][q] = bb[p][q] = P(0);
+                    if (in) v[p][q] = ld1(src + base + ls * pos(p, k + q));
+                    if (in && first) bb[p][q] = ld1(bz + base + ls * pos(p, k + q));
+                }
+        }
+#pragma unroll
+        for (int p = 0; p < NB; ++p)
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+                constexpr int PW = sizeof(P) / 4;
+                const P x = first ? v[p][q] * bb[p][q] : v[p][q];
+                em = max(em, expo(x));
+                uint32_t w[PW];
+                memcpy(w, &x, sizeof(P));
+#pragma unroll
+                for (int i = 0; i < PW; ++i) *reinterpret_cast<uint32_t *>(cell + ((p * 2 + q) * PW + i) * 128) = w[i];
+            }
+        atomicMax(&eline[r], em);
+    }
+    __syncthreads();
+
+    if (tid < ROWS) enext[tid] = 0;
+    /* ---- digits of the block operands, over the item's own words */
+#pragma unroll 1
+    for (int idx = tid; idx < items; idx += NT) {
+        const int u = idx >> 5, rg = nk8 == 1 ? u : (int)__umulhi((unsigned)u, g.mag_nk8);
+        const int em = eline[rg * 8 + ((idx >> 2) & 7)];
+        unsigned char *cell = smem + sm_a + u * CELL + (idx & 31) * 4;
+        Fix X[NB][2];
+#pragma unroll
+        for (int p = 0; p < NB; ++p)
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+                constexpr int PW = sizeof(P) / 4;
+                uint32_t w[PW];
+#pragma unroll
+                for (int i = 0; i < PW; ++i)
+                    w[i] = *reinterpret_cast<const uint32_t *>(cell + ((p * 2 + q) * PW + i) * 128);
+                P x;
+                memcpy(&x, w, sizeof(P));
+                X[p][q] = fix<NB>(x, em);
+            }
+        constexpr UFix BIAS = S == 6 ? (UFix)0x0802008020080200ull : (UFix)0x20080200u; /* 512 in every field */
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            if constexpr (NB == 4) { /* half-axis sums, then mirror sums */
+                const Fix a0 = X[0][q] + X[2][q], a1 = X[1][q] + X[3][q], b0 = X[0][q] - X[2][q], b1 = X[1][q] - X[3][q];
+                X[0][q] = a0 + a1;
+                X[1][q] = a0 - a1;
+                X[2][q] = b0 + b1;
+                X[3][q] = b0 - b1;
+            } else {
+                const Fix s = X[0][q] + X[1][q];
+                X[1][q] = X[0][q] - X[1][q];
+                X[0][q] = s;
+            }
+        }
+#pragma unroll
+        for (int b = 0; b < NB; ++b) {
+            const UFix ya = (UFix)X[b][0] + BIAS, yb = (UFix)X[b][1] + BIAS;
+#pragma unroll
+            for (int i = 0; i < S; ++i)
+                *reinterpret_cast<uint32_t *>(cell + (i * NB + b) * 128) = digit2<S, UFix>(ya, yb, i);
+        }
+    }
+    /* the operator digits, loaded once: one thread waits for all */
+    if (tid == 0 && !(ph.ok && mbar_wait(bar_op, 0))) *reinterpret_cast<volatile int *>(smem + SM_FAIL) = 1;
+    __syncthreads();
+    ph.ok = *reinterpret_cast<volatile int *>(smem + SM_FAIL) == 0;
+
+    /* ---- products, 16 lines x 8 outputs at a time, and the levels joined in registers */
+    using Acc = typename std::conditional<std::is_same<P, float>::value, float, long long>::type;
+    const int lt = (nlines + 15) / 16, nc = min(c1, (hb + W - 1) / W) - c0, ks = g.hp / 16;
+    /* ldmatrix rows: A (8 lines, 8 points) cells at (line half, point half) = (lane >> 3 & 1, lane >> 4),
+     * B (8 outputs, 8 points) cells at (digit, point half) = (lane >> 4, lane >> 3 & 1) */
+    const uint32_t a_lane = sbase + sm_a + (uint32_t)((((lane >> 3) & 1) * nk8 + (lane >> 4)) * CELL + (lane & 7) * 16);
+    const uint32_t b_lane = sbase + sm_op + (uint32_t)((lane >> 4) * 256 + ((lane >> 3) & 1) * 128 + (lane & 7) * 16);
+    /* accumulator v: line (lane >> 2) + 8 (v >> 1), output 2 (lane & 3) + (v & 1) */
+    auto products = [&](int l16, int cc, int b, Acc (&acc)[4]) {
+        const uint32_t a0 = a_lane + (uint32_t)(l16 * 2 * nk8 * CELL + b * 128);
+        const uint32_t b0 = b_lane + (uint32_t)((cc * NB + b) * ks * SK * 256);
+        float d[L][4];
+#pragma unroll
+        for (int l = 0; l < L; ++l)
+#pragma unroll
+            for (int v = 0; v < 4; ++v) d[l][v] = 0.0f;
+#pragma unroll 1
+        for (int k = 0; k < ks; ++k) {
+            uint32_t bf[SK / 2][4]; /* digits 2j, 2j + 1 */
+#pragma unroll
+            for (int j = 0; j < SK / 2; ++j) ldsm4(bf[j], b0 + (uint32_t)(k * SK * 256 + j * 512));
+#pragma unroll
+            for (int i = 0; i < S; ++i) {
+                uint32_t af[4];
+                ldsm4(af, a0 + (uint32_t)(2 * k * CELL + i * NB * 128));
+#pragma unroll
+                for (int j = 0; j < SK; ++j)
+                    if (i + j < L) mma16816(d[i + j], af, bf[j / 2][2 * (j & 1)], bf[j / 2][2 * (j & 1) + 1]);
+            }
+        }
+#pragma unroll
+        for (int v = 0; v < 4; ++v) acc[v] = join(d, v);
+    };
+    /* block sums back to the NB points of an output */
+    auto points = [&](const Acc (&s)[NB], int em, P (&y)[NB]) {
+        Acc t[NB];
+        if constexpr (NB == 4) {
+            const Acc s0 = s[0] + s[1], s1 = s[0] - s[1], s2 = s[2] + s[3], s3 = s[2] - s[3];
+            t[0] = s0 + s2;
+            t[1] = s1 + s3;
+            t[2] = s0 - s2;
+            t[3] = s1 - s3;
+        } else {
+            t[0] = s[0] + s[1];
+            t[1] = s[0] - s[1];
+        }
+#pragma unroll
+        for (int p = 0; p < NB; ++p) {
+            from_fix(t[p], em, y[p]);
+            if (em == ExpoMax<P>::v || !ph.ok) set_nan(y[p]);
+        }
+    };
+    if constexpr (SPLIT) {
+        /* a warp takes one block of them, and the sums meet in shared memory: four (two) times as
+         * many, shorter pieces of work, for tiles that would leave warps without any */
+        Acc *ex = reinterpret_cast<Acc *>(smem + sm_a + tile_bytes(g, S));
+        const int pitch = nc * W * NB + 2; /* values of a line: 16-byte rows, shifted by a bank group */
+#pragma unroll 1
+        for (int u = warp; u < lt * nc * NB; u += NT / 32) {
+            const int b = u % NB, v = u / NB, cc = v / lt, l16 = v - cc * lt;
+            Acc acc[4];
+            products(l16, cc, b, acc);
+#pragma unroll
+            for (int v4 = 0; v4 < 4; ++v4)
+                ex[(l16 * 16 + (lane >> 2) + 8 * (v4 >> 1)) * pitch + (cc * W + 2 * (lane & 3) + (v4 & 1)) * NB + b] = acc[v4];
+        }
+        __syncthreads();
+        /* a warp takes 8 lines x 4 outputs: whole sectors along either direction */
+        const int og = nc * (W / 4);
+#pragma unroll 1
+        for (int idx = tid; idx < (nlines + 7) / 8 * og * 32; idx += NT) {
+            const int u = idx >> 5, rg = u / og, o = (u - rg * og) * 4 + (idx & 3), r = rg * 8 + ((idx >> 2) & 7), k = c0 * W + o;
+            if (r >= nlines || k >= hb) continue;
+            const int base = line_base(r);
+            P f[NB], y[NB];
+            if (last) {
+#pragma unroll
+                for (int p = 0; p < NB; ++p) f[p] = ld1(bz + base + ls * pos(p, k));
+            }
+            Acc s[NB];
+#pragma unroll
+            for (int b = 0; b < NB; ++b) s[b] = ex[r * pitch + o * NB + b];
+            points(s, eline[r], y);
+#pragma unroll
+            for (int p = 0; p < NB; ++p) dst[base + ls * pos(p, k)] = last ? y[p] * f[p] : y[p];
+        }
+    } else {
+        /* a warp takes all blocks of them and writes the outputs from its registers */
+#pragma unroll 1
+        for (int u = warp; u < lt * nc; u += NT / 32) {
+            const int cc = u / lt, l16 = u - cc * lt, k0 = (c0 + cc) * W + 2 * (lane & 3);
+            Acc acc[NB][4];
+#pragma unroll
+            for (int b = 0; b < NB; ++b) products(l16, cc, b, acc[b]);
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int r = l16 * 16 + 8 * h + (lane >> 2);
+                if (r >= nlines) continue;
+                const int em = eline[r], base = line_base(r);
+                P y[2][NB];
+#pragma unroll
+                for (int q = 0; q < 2; ++q) {
+                    Acc s[NB];
+#pragma unroll
+                    for (int b = 0; b < NB; ++b) s[b] = acc[b][2 * h + q];
+                    points(s, em, y[q]);
+                }
+                if (vec && k0 + 1 < hb) {
+#pragma unroll
+                    for (int p = 0; p < NB; ++p) {
+                        const int at = base + ((p & 1) ? pos(p, k0 + 1) : pos(p, k0));
+                        P o[2] = {y[p & 1][p], y[1 - (p & 1)][p]};
+                        if (last) {
+                            P f[2];
+                            ld2(bz + at, f);
+                            o[0] = o[0] * f[0];
+                            o[1] = o[1] * f[1];
+                        }
+                        st2(dst + at, o[0], o[1]);
+                    }
+                } else {
+#pragma unroll
+                    for (int p = 0; p < NB; ++p)
+#pragma unroll
+                        for (int q = 0; q < 2; ++q) {
+                            if (k0 + q >= hb) continue;
+                            const int at = base + ls * pos(p, k0 + q);
+                            P o = y[q][p];
+                            if (last) o = o * ld1(bz + at);
+                            dst[at] = o;
+                        }
+                }
+            }
+        }
+    }
+    __syncthreads();
+}
+
+/* This part's operator digits. */
+template <typename P, int NB>
+__device__ __forceinline__ void tc_start_op(const TcGeom &g, const void *table, int part, uint32_t dst, uint32_t bar)
+{
+    /* consecutive chunks of the table; one thread */
+    constexpr int SK = Dig<P>::SK;
+    const int c0 = part * g.cpp, c1 = min(c0 + g.cpp, g.nchunks);
+    const uint32_t per = (uint32_t)(NB * g.hp * SK * 2); /* bytes per output */
+    const uint32_t bytes = per * (min(c1 * W, g.hp) - c0 * W);
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
+                 "l"(reinterpret_cast<const unsigned char *>(table) + per * (c0 * W)), "r"(bytes), "r"(bar)
+                 : "memory");
+}
+
+/* Barriers and line exponents; ends with a CTA barrier. */
+__device__ __forceinline__ void tc_begin(unsigned char *smem, int nax)
+{
+    for (int i = threadIdx.x; i < 2 * ROWS; i += blockDim.x) reinterpret_cast<int *>(smem + SM_ELINE)[i] = 0;
+    if (threadIdx.x == 32) {
+        *reinterpret_cast<volatile int *>(smem + SM_FAIL) = 0;
+        for (int i = 0; i < nax; ++i)
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"((uint32_t)__cvta_generic_to_shared(smem) + SM_BAR + 8 * i) : "memory");
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncthreads();
+}
+
+} // namespace
+
+/* One pass: a CTA per (tile, part) and chain. */
+template <typename P, int NB>
+__global__ void __launch_bounds__(256, 2) k_pass_tc(TcGeom g, PassArgs a)
+{
+    const ChainDesc cd = a.chains[blockIdx.y];
+    if (a.s >= cd.len - 1) return; /* uniform over the CTA */
+    if (a.state && a.state[cd.instance].done) return;
+
+    extern __shared__ __align__(128) unsigned char smem[];
+    const int part = blockIdx.x % g.parts, tile_i = blockIdx.x / g.parts;
+    tc_begin(smem, 1);
+    const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(smem), bar_op = sbase + SM_BAR;
+    if (threadIdx.x == 32) /* in flight until the products need them */
+        tc_start_op<P, NB>(g, cd.ops->tc[a.axis], part, sbase + SM_OP, bar_op);
+    const P *src = a.first ? reinterpret_cast<const P *>(cd.q) + (long)a.s * a.sstride
+                           : reinterpret_cast<const P *>(cd.tmp);
+    P *dst = a.last ? reinterpret_cast<P *>(cd.q) + (long)(a.s + 1) * a.sstride : reinterpret_cast<P *>(cd.tmp);
+    const P *bz = reinterpret_cast<const P *>(a.s < cd.seg_end ? cd.b0 : cd.b1);
+    TcPhase ph = {0, true};
+    tc_tile<P, NB, 256, false>(g, src, dst, bz, a.first, a.last, tile_i, part, smem, SM_OP, SM_OP + g.op_part, bar_op, ph);
+    if (!ph.ok && threadIdx.x == 0) atomicExch(&g_scft_pass_fault, 1);
+}
+
+/* The whole contour loop of a chain in one cluster. Each CTA keeps its part of
+ * every axis' operator digits in shared memory and takes the same tiles at every
+ * step; the slices pass between the CTAs through L2 (the intermediate slice of
+ * one axis, then q_{s+1}), ordered by a cluster barrier after each axis. A step
+ * thus costs two or three short phases per CTA, without the launches, the
+ * set-up and the cold instruction cache that a pass of its own has (~4 of 8 us
+ * on a 192x96 slice). Control flow is uniform over the cluster. */
+template <typename P>
+__global__ void __launch_bounds__(512, 1) k_chain_tc(const __grid_constant__ TcLoop lp, Step2DArgs a)
+{
+    const int rank = blockIdx.x % lp.cluster, slot = blockIdx.x / lp.cluster; /* clusters are consecutive blocks */
+    const ChainDesc cd = a.chains[a.order ? a.order[slot] : slot];
+    if (a.state && a.state[cd.instance].done) return; /* uniform over the cluster */
+    const int s_end = a.s_end < cd.len - 1 ? a.s_end : cd.len - 1;
+    if (a.s >= s_end) return;
+
+    extern __shared__ __align__(128) unsigned char smem[];
+    tc_begin(smem, lp.nax);
+    const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(smem);
+    if (threadIdx.x == 32)
+        for (int ax = 0; ax < lp.nax; ++ax) {
+            const TcGeom &g = lp.g[ax];
+            if (rank / g.parts >= lp.slots[ax]) continue;
+            if (g.nb == 4)
+                tc_start_op<P, 4>(g, cd.ops->tc[ax], rank % g.parts, sbase + lp.op_at[ax], sbase + SM_BAR + 8 * ax);
+            else
+                tc_start_op<P, 2>(g, cd.ops->tc[ax], rank % g.parts, sbase + lp.op_at[ax], sbase + SM_BAR + 8 * ax);
+        }
+    TcPhase ph = {0, true};
+#pragma unroll 1
+    for (int s = a.s; s < s_end; ++s) {
+        const P *bz = reinterpret_cast<const P *>(s < cd.seg_end ? cd.b0 : cd.b1);
+#pragma unroll 1
+        for (int ax = 0; ax < lp.nax; ++ax) {
+            const TcGeom &g = lp.g[ax];
+            const bool first = ax == 0, last = ax == lp.nax - 1;
+            const P *src = first ? reinterpret_cast<const P *>(cd.q) + (long)s * a.sstride : reinterpret_cast<const P *>(cd.tmp);
+            P *dst = last ? reinterpret_cast<P *>(cd.q) + (long)(s + 1) * a.sstride : reinterpret_cast<P *>(cd.tmp);
+            const int t0 = rank / g.parts, part = rank % g.parts;
+            if (t0 < lp.slots[ax])
+#pragma unroll 1
+                for (int t = t0; (long)t * g.tile < g.lines; t += lp.slots[ax]) {
+                    if (g.nb == 4)
+                        tc_tile<P, 4, 512, true>(g, src, dst, bz, first, last, t, part, smem, lp.op_at[ax], lp.tile_at,
+                                      sbase + SM_BAR + 8 * ax, ph);
+                    else
+                        tc_tile<P, 2, 512, true>(g, src, dst, bz, first, last, t, part, smem, lp.op_at[ax], lp.tile_at,
+                                      sbase + SM_BAR + 8 * ax, ph);
+                }
+            /* this axis' slice is complete before the next one reads it */
+            asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+        }
+    }
+    if (!ph.ok && threadIdx.x == 0) atomicExch(&g_scft_pass_fault, 1);
+}
+
+/* ------------------------------------------------------------- launchers */
+size_t scft_pass_tc_smem(int prec, const TcGeom &g)
+{
+    return SM_OP + g.op_part + (prec == SCFT_PREC_FP32 ? tile_bytes(g, Dig<float>::S)
+                                                      : tile_bytes(g, Dig<double>::S));
+}
+
+template <typename P>
+static cudaError_t launch_tc(const TcGeom &g, const PassArgs &a, cudaStream_t st)
+{
+    const size_t smem = SM_OP + g.op_part + tile_bytes(g, Dig<P>::S);
+    const dim3 grid((unsigned)((g.lines + g.tile - 1) / g.tile * g.parts), a.nchains);
+    if (g.tile < 8 || g.tile % 8 || g.tile > ROWS) return cudaErrorInvalidValue;
+    if (g.nb == 4)
+        k_pass_tc<P, 4><<<grid, 256, smem, st>>>(g, a);
+    else
+        k_pass_tc<P, 2><<<grid, 256, smem, st>>>(g, a);
+    return cudaGetLastError();
+}
+
+int scft_pass_tc_fits(int prec, const TcGeom &g, int smem_limit)
+{
+    return scft_pass_tc_smem(prec, g) <= (size_t)smem_limit;
+}
+
+cudaError_t scft_launch_pass_tc(int prec, const TcGeom &g, const PassArgs &a, cudaStream_t st)
+{
+    if (prec == SCFT_PREC_FP64) return launch_tc<double>(g, a, st);
+    if (prec == SCFT_PREC_FP32X2) return launch_tc<dfloat>(g, a, st);
+    return launch_tc<float>(g, a, st);
+}
+
+/* Shared-memory layout of the cluster loop, from the axes' tiles and parts;
+ * returns its bytes. */
+size_t scft_chain_tc_layout(int prec, TcLoop &lp)
+{
+    uint32_t at = SM_OP, tile = 0;
+    for (int ax = 0; ax < lp.nax; ++ax) {
+        lp.op_at[ax] = at;
+        at += (lp.g[ax].op_part + 127) / 128 * 128;
+        const uint32_t b = prec == SCFT_PREC_FP32 ? tile_bytes(lp.g[ax], Dig<float>::S) + exchange_bytes(lp.g[ax], 4)
+                                                  : tile_bytes(lp.g[ax], Dig<double>::S) + exchange_bytes(lp.g[ax], 8);
+        if (b > tile) tile = b;
+        lp.slots[ax] = lp.cluster / lp.g[ax].parts;
+    }
+    lp.tile_at = at;
+    return (size_t)at + tile;
+}
+
+template <typename P>
+static cudaError_t launch_chain(const TcLoop &lp, const Step2DArgs &a, int nchains, cudaStream_t st, int *clusters)
+{
+    TcLoop l = lp;
+    const int prec = std::is_same<P, double>::value ? SCFT_PREC_FP64 : std::is_same<P, float>::value ? SCFT_PREC_FP32 : SCFT_PREC_FP32X2;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(nchains * lp.cluster), 1, 1);
+    cfg.blockDim = dim3(512, 1, 1);
+    cfg.dynamicSmemBytes = scft_chain_tc_layout(prec, l);
+    cfg.stream = st;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = lp.cluster;
+    attr.val.clusterDim.y = 1;
+    attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    if (clusters) return cudaOccupancyMaxActiveClusters(clusters, k_chain_tc<P>, &cfg);
+    return cudaLaunchKernelEx(&cfg, k_chain_tc<P>, l, a);
+}
+
+/* Launches the contour loops of nchains chains; with clusters != NULL only asks
+ * how many clusters can be resident. */
+cudaError_t scft_launch_chain_tc(int prec, const TcLoop &lp, const Step2DArgs &a, int nchains, cudaStream_t st,
+                                 int *clusters)
+{
+    if (prec == SCFT_PREC_FP64) return launch_chain<double>(lp, a, nchains, st, clusters);
+    if (prec == SCFT_PREC_FP32X2) return launch_chain<dfloat>(lp, a, nchains, st, clusters);
+    return launch_chain<float>(lp, a, nchains, st, clusters);
+}
+
+template <typename P>
+static cudaError_t configure_tc(int smem_bytes)
+{
+    /* one carve-out for every pass, so the SMs keep their split between launches */
+    const void *k[] = {(const void *)k_pass_tc<P, 4>, (const void *)k_pass_tc<P, 2>, (const void *)k_chain_tc<P>};
+    cudaError_t e = cudaSuccess;
+    for (const void *f : k) {
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+    }
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_chain_tc<P>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    return e;
+}
+
+/* Raise the dynamic shared-memory limit once, outside any stream capture. */
+cudaError_t scft_pass_tc_configure(int smem_bytes)
+{
+    cudaError_t e = configure_tc<double>(smem_bytes);
+    if (e == cudaSuccess) e = configure_tc<dfloat>(smem_bytes);
+    if (e == cudaSuccess) e = configure_tc<float>(smem_bytes);
+    return e;
+}
+
+int scft_pass_tc_take_fault(void)
+{
+    int v = 0;
+    const int zero = 0;
+    if (cudaMemcpyFromSymbol(&v, g_scft_pass_fault, sizeof(int)) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    if (v) cudaMemcpyToSymbol(g_scft_pass_fault, &zero, sizeof(int));
+    return v;
+}

@@ -34,6 +34,7 @@
 #include <type_traits>
 
 #include "scft_internal.h"
+#include "scft_mbar.cuh"
 
 /* Build switches of the fused chain kernel. */
 #ifndef SCFT_F32X2
@@ -451,22 +452,6 @@ __device__ __forceinline__ void mma_bf16(uint32_t d, uint32_t a, uint64_t b, uin
                  "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d),
                  "r"(a), "l"(b), "r"(idesc), "r"(acc)
                  : "memory");
-}
-
-/* Bounded wait for the mbarrier phase of the given parity: false after ~0.1 s. */
-__device__ __forceinline__ bool mbar_wait(uint32_t mb, uint32_t parity)
-{
-    const long long t0 = clock64();
-    for (;;) {
-        uint32_t done;
-        asm volatile("{\n\t.reg .pred P1;\n\tmbarrier.try_wait.parity.shared::cta.b64 P1, [%1], %2;\n\t"
-                     "selp.b32 %0, 1, 0, P1;\n\t}"
-                     : "=r"(done)
-                     : "r"(mb), "r"(parity)
-                     : "memory");
-        if (done) return true;
-        if (clock64() - t0 > (1LL << 28)) return false;
-    }
 }
 
 /* u, v of one line split into bf16 pairs and stored to the A columns of its
