@@ -745,6 +745,7 @@ static int tc_apply(int prec, TcGeom &g, int tile, int parts, int smem_limit)
     if ((g.nchunks + g.cpp - 1) / g.cpp != parts) return 0;
     g.op_part = (unsigned)((size_t)g.nb * g.hp * tc_sk(prec) * g.cpp * g.w * 2);
     g.mag_nk8 = (unsigned)((0xFFFFFFFFull + g.hp / 8) / (g.hp / 8));
+    g.mag_og = (unsigned)((0xFFFFFFFFull + g.cpp * g.w / 4) / (g.cpp * g.w / 4));
     return scft_pass_tc_fits(prec, g, smem_limit);
 }
 
@@ -756,10 +757,15 @@ struct TcChoice {
 /* Clocks of a tile, roughly: loading and splitting per item of 2 NB points, 20 per
  * MMA (16 is the rate), joining and writing the outputs. In the loop (512 threads)
  * a warp multiplies one block at a time, in a pass of its own (256) all blocks. */
-static double tc_cta_cost(const TcGeom &g, int prec, int threads)
+static double tc_cta_cost(const TcGeom &g, int prec, int threads, int exchange = 0)
 {
     const double items = std::ceil(g.tile * (g.hp / 2) / (double)threads), mmas = prec == SCFT_PREC_FP32 ? 9.0 : 21.0;
     const double block = g.hp / 16 * mmas * 20.0 + 300.0, work = (g.tile + 15) / 16 * g.cpp, warps = threads / 32.0;
+    if (exchange) { /* blocks of 16 outputs x 8 lines, at the latency of one or the rate of all (~13 clocks an MMA) */
+        const double blocks = (g.tile + 7) / 8 * ((g.cpp + 1) / 2) * g.nb;
+        return 1500.0 + items * g.nb * 350.0 + std::max(std::ceil(blocks / warps) * block, blocks * g.hp / 16 * mmas * 13.0 / 4) +
+               std::max(1200.0, g.tile * g.cpp * 8 * g.nb * 2.0);
+    }
     if (threads == 512) /* loop: a block at a time, then the outputs */
         return 2000.0 + items * g.nb * 350.0 + std::ceil(work * g.nb / warps) * block +
                std::ceil(g.tile * g.cpp * 8 / (double)threads) * g.nb * 300.0;
@@ -1031,31 +1037,56 @@ static double tc_loop_plan(const scft_ctx *c, int cluster, int smem_limit, TcLoo
     return cost;
 }
 
+/* The 2D form with one tile per CTA and axis: nothing to choose but the cluster. */
+static double tc_exchange_plan(const scft_ctx *c, int cluster, int smem_limit, TcLoop &lp)
+{
+    const int prec = c->opt.precision;
+    memset(&lp, 0, sizeof(lp));
+    lp.nax = 2;
+    lp.cluster = cluster;
+    lp.exchange = 1;
+    double cost = 0.0;
+    for (int ax = 0; ax < 2; ++ax) {
+        lp.g[ax] = c->axes[ax].t;
+        const int tile = (int)(((lp.g[ax].lines + cluster - 1) / cluster + 7) / 8 * 8);
+        if (tile > 128 || !tc_apply(prec, lp.g[ax], tile, 1, smem_limit)) return -1.0;
+        cost += tc_cta_cost(lp.g[ax], prec, 512, 1);
+    }
+    return scft_chain_tc_layout(prec, lp) <= (size_t)smem_limit ? cost : -1.0;
+}
+
 struct LoopChoice {
     double cost; /* clocks of an iteration's contour steps */
     int resident; /* clusters that fit on the GPU */
     TcLoop lp;
 };
+static bool tc_loop_make(const scft_ctx *c, int cluster, int exchange, int smem_limit, LoopChoice &ch)
+{
+    if (exchange && c->axes.size() != 2) return false;
+    const double per = exchange ? tc_exchange_plan(c, cluster, smem_limit, ch.lp) : tc_loop_plan(c, cluster, smem_limit, ch.lp);
+    ch.cost = per * (c->maxlen - 1);
+    ch.resident = 0;
+    return per >= 0.0;
+}
+
 static std::vector<LoopChoice> tc_loops(const scft_ctx *c, int smem_limit)
 {
     std::vector<LoopChoice> out;
-    for (const Axis &A : c->axes)
-        if (!A.tc) return out;
-    if (c->axes.empty() || c->opt.kernel_path != 0) return out;
     double steps = 0.0;
     for (const ChainDesc &cd : c->chains_h) steps += cd.len - 1;
-    for (int cluster = 1; cluster <= 16; cluster *= 2) {
+    static const int sizes[] = {1, 2, 3, 4, 6, 8, 12, 16};
+    for (int k = 0; k < 16; ++k) {
+        const int cluster = sizes[k / 2], exchange = k % 2;
         LoopChoice ch;
-        const double per = tc_loop_plan(c, cluster, smem_limit, ch.lp);
-        if (per < 0.0) continue;
+        /* tiles of several slots and parts share out over powers of two */
+        if ((!exchange && (cluster & (cluster - 1)) != 0) || !tc_loop_make(c, cluster, exchange, smem_limit, ch)) continue;
         Step2DArgs a;
         memset(&a, 0, sizeof(a));
-        ch.resident = 0;
         if (scft_launch_chain_tc(c->opt.precision, ch.lp, a, 1, c->stream, &ch.resident) != cudaSuccess || ch.resident < 1) {
             cudaGetLastError();
             continue;
         }
-        ch.cost = per * std::max((double)(c->maxlen - 1), steps / std::min((double)ch.resident, (double)c->chains_h.size()));
+        ch.cost = std::max(ch.cost, ch.cost / (c->maxlen - 1) * steps / std::min((double)ch.resident, (double)c->chains_h.size()));
         out.push_back(ch);
     }
     return out;
@@ -1184,11 +1215,26 @@ static int choose_loop_tc(scft_ctx *c)
 {
     int optin = 0;
     CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device));
-    std::vector<LoopChoice> ch = tc_loops(c, optin);
-    if (ch.empty()) return SCFT_OK;
+    for (const Axis &A : c->axes)
+        if (!A.tc) return SCFT_OK;
     const int npass = (int)c->axes.size(), nch = (int)c->chains_h.size(), last = c->maxlen - 1;
+    if (npass == 0 || last < 1 || c->opt.kernel_path != 0) return SCFT_OK;
     double total = 0.0, passes = 0.0, ctas = 0.0;
     for (const ChainDesc &cd : c->chains_h) total += cd.len - 1;
+    char key[200];
+    snprintf(key, sizeof(key), "loop|%d|%d,%d,%d|%d|%d|%d,%.0f", c->opt.precision, c->nx, c->ny, c->nz, c->axes.back().dirichlet, nch,
+             c->maxlen, total);
+    if (c->opt.autotune) {
+        std::lock_guard<std::mutex> lk(g_tune_mu);
+        auto it = g_tune_cache.find(key);
+        if (it != g_tune_cache.end()) {
+            LoopChoice one;
+            c->loop_tc = it->second > 0 && tc_loop_make(c, it->second % 100, it->second / 100, optin, one);
+            if (c->loop_tc) c->loop = one.lp;
+            return SCFT_OK;
+        }
+    }
+    std::vector<LoopChoice> ch = tc_loops(c, optin);
     for (int ai = 0; ai < npass; ++ai) {
         const TcGeom &g = c->axes[ai].t;
         const std::vector<TcChoice> p = tc_choices(c, g, ai > 0 && ai < npass - 1, optin);
@@ -1196,22 +1242,7 @@ static int choose_loop_tc(scft_ctx *c)
         ctas += (double)((g.lines + g.tile - 1) / g.tile) * g.parts * nch / npass;
     }
     int best = -1;
-    if (c->opt.autotune && last > 0) {
-        char key[200];
-        snprintf(key, sizeof(key), "loop|%d|%d,%d,%d|%d|%d|%d,%.0f", c->opt.precision, c->nx, c->ny, c->nz,
-                 c->axes.back().dirichlet, nch, c->maxlen, total);
-        {
-            std::lock_guard<std::mutex> lk(g_tune_mu);
-            auto it = g_tune_cache.find(key);
-            if (it != g_tune_cache.end()) {
-                for (size_t k = 0; k < ch.size(); ++k)
-                    if (ch[k].lp.cluster == it->second) {
-                        c->loop_tc = 1;
-                        c->loop = ch[k].lp;
-                    }
-                return SCFT_OK;
-            }
-        }
+    if (c->opt.autotune) {
         const int steps = std::min(4, last);
         cudaEvent_t e0 = nullptr, e1 = nullptr;
         CK(cudaEventCreate(&e0));
@@ -1243,8 +1274,9 @@ static int choose_loop_tc(scft_ctx *c)
         cudaEventDestroy(e0);
         cudaEventDestroy(e1);
         if (rc) return rc;
+        scft_pass_tc_take_fault(); /* a wait that gave up on the timing runs is not an iteration's */
         std::lock_guard<std::mutex> lk(g_tune_mu);
-        g_tune_cache[key] = best < 0 ? 0 : ch[best].lp.cluster;
+        g_tune_cache[key] = best < 0 ? 0 : ch[best].lp.cluster + 100 * ch[best].lp.exchange;
     } else {
         for (size_t k = 0; k < ch.size(); ++k) {
             const double cost = ch[k].cost * (nch > ch[k].resident ? 2.0 : 1.3);

@@ -147,15 +147,20 @@ struct TcGeom {
     int tile, parts, cpp;
     unsigned op_part;  /* bytes of operator digits a CTA holds */
     unsigned mag_nk8;  /* ceil(2^32 / d), d = hp / 8 */
+    unsigned mag_og;   /* d = cpp w / 4 */
 };
 
-/* The cluster-resident contour loop over the same tiles (k_chain_tc). */
+/* The cluster-resident contour loop over the same tiles (k_chain_tc, k_chain2d_tc). */
 struct TcLoop {
     int nax, cluster; /* axes, CTAs per cluster */
+    int exchange;     /* 1: 2D, one tile per CTA and axis, lines passed through shared memory (k_chain2d_tc) */
     TcGeom g[3];
     int slots[3];      /* tiles taken side by side: cluster / parts */
     unsigned op_at[3]; /* shared-memory offsets of the axes' operator digits and of the tile region */
     unsigned tile_at;
+    /* exchange: the axes' lines in shared memory, values from line to line, ceil(2^32 / tile) */
+    unsigned buf_at[2], mag_tile[2];
+    int pitch[2];
 };
 
 size_t scft_pass_tc_smem(int prec, const TcGeom &g);

@@ -155,6 +155,36 @@ __device__ __forceinline__ uint32_t digit2(U ya, U yb, int i)
     return *reinterpret_cast<const uint32_t *>(&h);
 }
 
+/* the block operands of two points from the points' NB images, and their digits into the item's cells */
+template <typename P, int NB, typename Fix>
+__device__ __forceinline__ void put_digits(Fix (&X)[NB][2], unsigned char *cell)
+{
+    constexpr int S = Dig<P>::S;
+    using UFix = typename std::make_unsigned<Fix>::type;
+    constexpr UFix BIAS = S == 6 ? (UFix)0x0802008020080200ull : (UFix)0x20080200u; /* 512 in every field */
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+        if constexpr (NB == 4) { /* half-axis sums, then mirror sums */
+            const Fix a0 = X[0][q] + X[2][q], a1 = X[1][q] + X[3][q], b0 = X[0][q] - X[2][q], b1 = X[1][q] - X[3][q];
+            X[0][q] = a0 + a1;
+            X[1][q] = a0 - a1;
+            X[2][q] = b0 + b1;
+            X[3][q] = b0 - b1;
+        } else {
+            const Fix s = X[0][q] + X[1][q];
+            X[1][q] = X[0][q] - X[1][q];
+            X[0][q] = s;
+        }
+    }
+#pragma unroll
+    for (int b = 0; b < NB; ++b) {
+        const UFix ya = (UFix)X[b][0] + BIAS, yb = (UFix)X[b][1] + BIAS;
+#pragma unroll
+        for (int i = 0; i < S; ++i)
+            *reinterpret_cast<uint32_t *>(cell + (i * NB + b) * 128) = digit2<S, UFix>(ya, yb, i);
+    }
+}
+
 /* two consecutive values of a row, 16-byte aligned (FP32: 8) */
 __device__ __forceinline__ void ld2(const double *p, double (&v)[2])
 {
@@ -174,6 +204,25 @@ __device__ __forceinline__ void ld2(const float *p, float (&v)[2])
     v[0] = t.x;
     v[1] = t.y;
 }
+/* the same from shared memory */
+__device__ __forceinline__ void lds2(const double *p, double &a, double &b)
+{
+    const double2 t = *reinterpret_cast<const double2 *>(p);
+    a = t.x;
+    b = t.y;
+}
+__device__ __forceinline__ void lds2(const dfloat *p, dfloat &a, dfloat &b)
+{
+    const float4 t = *reinterpret_cast<const float4 *>(p);
+    a = dfloat(t.x, t.y);
+    b = dfloat(t.z, t.w);
+}
+__device__ __forceinline__ void lds2(const float *p, float &a, float &b)
+{
+    const float2 t = *reinterpret_cast<const float2 *>(p);
+    a = t.x;
+    b = t.y;
+}
 __device__ __forceinline__ void st2(double *p, double a, double b) { *reinterpret_cast<double2 *>(p) = make_double2(a, b); }
 __device__ __forceinline__ void st2(dfloat *p, dfloat a, dfloat b)
 {
@@ -188,6 +237,15 @@ __device__ __forceinline__ dfloat ld1(const dfloat *p)
     return dfloat(t.x, t.y);
 }
 
+/* factors that no one writes while the kernel runs: they may stay in L1 */
+__device__ __forceinline__ double ldc(const double *p) { return __ldg(p); }
+__device__ __forceinline__ float ldc(const float *p) { return __ldg(p); }
+__device__ __forceinline__ dfloat ldc(const dfloat *p)
+{
+    const float2 t = __ldg(reinterpret_cast<const float2 *>(p));
+    return dfloat(t.x, t.y);
+}
+
 /* four 8 x 8 matrices of 16-bit values from shared memory, rows of 16 bytes at each lane's address */
 __device__ __forceinline__ void ldsm4(uint32_t (&r)[4], uint32_t addr)
 {
@@ -196,7 +254,7 @@ __device__ __forceinline__ void ldsm4(uint32_t (&r)[4], uint32_t addr)
                  : "r"(addr)
                  : "memory");
 }
-/* c += a b: 16 lines x 8 outputs x 16 points */
+/* c += a b: 16 rows x 8 columns x 16 points */
 __device__ __forceinline__ void mma16816(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1)
 {
     asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
@@ -281,16 +339,20 @@ __device__ __forceinline__ void set_nan(float &y) { y = __int_as_float(0x7fc0000
  * operator digits (one region per axis), then the digits of a tile's lines. */
 constexpr uint32_t SM_BAR = 0, SM_FAIL = 32, SM_ELINE = 64, SM_OP = SM_ELINE + 2 * ROWS * 4;
 
-/* bytes of a tile's digits (an MMA reads 16 lines) */
-__host__ __device__ inline uint32_t tile_bytes(const TcGeom &g, int digits)
+/* bytes of a tile's digits (an MMA of a pass reads 16 lines, of k_chain2d_tc 8) */
+__host__ __device__ inline uint32_t tile_bytes(const TcGeom &g, int digits, int lines = 16)
 {
-    return (uint32_t)((g.tile + 15) / 16 * 16) * g.hp * g.nb * digits * 2;
+    return (uint32_t)((g.tile + lines - 1) / lines * lines) * g.hp * g.nb * digits * 2;
 }
 
-/* bytes of the exchange of block sums, for a part of the outputs */
+/* bytes of the exchange of block sums, for a part of the outputs (k_chain_tc, k_chain2d_tc) */
 __host__ __device__ inline uint32_t exchange_bytes(const TcGeom &g, int value)
 {
     return (uint32_t)((g.tile + 15) / 16 * 16) * (g.cpp * W * g.nb + 2) * value;
+}
+__host__ __device__ inline uint32_t exchange2d_bytes(const TcGeom &g, int value)
+{
+    return (uint32_t)g.tile * (g.cpp * W * g.nb + 4) * value;
 }
 
 /* Where a CTA is. */
@@ -299,12 +361,234 @@ struct TcPhase {
     bool ok;       /* no wait has given up */
 };
 
+/* ---- lines that pass between the CTAs of a cluster through shared memory (k_chain2d_tc) */
+
+/* Lines of one axis in this CTA's shared memory, and where its outputs go: lines of the other axis. */
+template <typename P>
+struct Exchange {
+    const P *in;       /* the tile's lines, `pitch` values apart */
+    const int *eline;  /* their largest exponents, below the step's number */
+    int pitch, tag;    /* tag: the number the receiver expects, in place */
+    uint32_t out, out_eline, bar; /* offsets in every CTA's shared memory */
+    int out_pitch, out_tile;
+    unsigned out_mag;  /* ceil(2^32 / out_tile) */
+    bool send;
+    const P *bz, *bnext; /* after the last axis: this and the next step's factors */
+    P *dst;              /* then q_{s+1} */
+};
+__device__ __forceinline__ uint32_t at_rank(uint32_t addr, uint32_t rank)
+{
+    uint32_t r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+    return r;
+}
+/* two neighbouring values into another CTA's shared memory, counted by its barrier (one store
+ * costs the same ~2 clocks a lane whatever its width) */
+__device__ __forceinline__ void send(uint32_t addr, uint32_t bar, unsigned long long a, unsigned long long b)
+{
+    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v2.b64 [%0], {%1, %2}, [%3];" ::"r"(addr), "l"(a), "l"(b), "r"(bar)
+                 : "memory");
+}
+__device__ __forceinline__ void send(uint32_t addr, uint32_t bar, double a, double b)
+{
+    send(addr, bar, (unsigned long long)__double_as_longlong(a), (unsigned long long)__double_as_longlong(b));
+}
+__device__ __forceinline__ void send(uint32_t addr, uint32_t bar, dfloat a, dfloat b)
+{
+    send(addr, bar, (unsigned long long)__float_as_uint(a.lo) << 32 | __float_as_uint(a.hi),
+         (unsigned long long)__float_as_uint(b.lo) << 32 | __float_as_uint(b.hi));
+}
+__device__ __forceinline__ void send(uint32_t addr, uint32_t bar, float a, float b)
+{
+    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v2.b32 [%0], {%1, %2}, [%3];" ::"r"(addr), "r"(__float_as_uint(a)),
+                 "r"(__float_as_uint(b)), "r"(bar)
+                 : "memory");
+}
+__device__ __forceinline__ double swap_rows(double v) { return __shfl_xor_sync(0xffffffffu, v, 4); }
+__device__ __forceinline__ float swap_rows(float v) { return __shfl_xor_sync(0xffffffffu, v, 4); }
+__device__ __forceinline__ dfloat swap_rows(dfloat v) { return dfloat(swap_rows(v.hi), swap_rows(v.lo)); }
+/* the largest of the values sent, counted by the barrier like them */
+__device__ __forceinline__ void send_max(uint32_t addr, uint32_t bar, uint32_t v)
+{
+    asm volatile("red.async.relaxed.cluster.mbarrier::complete_tx::bytes.shared::cluster.max.u32 [%0], %1, [%2];" ::"r"(addr), "r"(v), "r"(bar)
+                 : "memory");
+}
+constexpr int EBITS = 11; /* bits of an exponent */
+
+/* The tile of k_chain2d_tc: like tc_tile, from lines with their exponents in
+ * shared memory to lines of the other axis in their CTAs' shared memory. */
+template <typename P, int NB, int NT>
+__device__ __forceinline__ void tc_tile2d(const TcGeom &g, const Exchange<P> &xc, bool last, int tile_i, unsigned char *smem,
+                                          uint32_t sm_op, uint32_t sm_a, uint32_t bar_op, bool wait_op, bool &ok)
+{
+    constexpr int S = Dig<P>::S, SK = Dig<P>::SK, L = Dig<P>::L, CELL = S * NB * 128;
+    using Fix = typename FixT<P>::T;
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0); /* uniform */
+    const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(smem);
+    const int n = g.n, hb = g.hb, m = n / 2, nk8 = g.hp / 8, nc = g.nchunks;
+    const int L0 = tile_i * g.tile, nlines = (int)min((long)g.tile, g.lines - L0);
+    auto pos = [&](int p, int k) { /* as in tc_tile */
+        if (NB == 2) return p == 0 ? k : n - 1 - k;
+        return p == 0 ? k : p == 1 ? m - 1 - k : p == 2 ? k + m : n - 1 - k;
+    };
+
+    /* ---- digits: an item is two neighbouring points and their images of one line */
+#pragma unroll 1
+    for (int idx = tid; idx < g.tile * nk8 * 4; idx += NT) {
+        const int u = idx >> 5, rg = nk8 == 1 ? u : (int)__umulhi((unsigned)u, g.mag_nk8), k8 = u - rg * nk8;
+        const int r = rg * 8 + ((idx >> 2) & 7), k = k8 * 8 + 2 * (idx & 3);
+        const int em = xc.eline[r] & ((1 << EBITS) - 1);
+        const P *in = xc.in + r * xc.pitch;
+        Fix X[NB][2];
+#pragma unroll
+        for (int p = 0; p < NB; ++p) {
+            P v[2] = {P(0), P(0)};
+            if (r < nlines) {
+                if (n % 2 == 0 && k + 1 < hb) { /* pairs of an even axis are aligned */
+                    lds2(in + ((p & 1) ? pos(p, k + 1) : pos(p, k)), v[p & 1], v[1 - (p & 1)]);
+                } else {
+#pragma unroll
+                    for (int q = 0; q < 2; ++q)
+                        if (k + q < hb) v[q] = in[pos(p, k + q)];
+                }
+            }
+            X[p][0] = fix<NB>(v[0], em);
+            X[p][1] = fix<NB>(v[1], em);
+        }
+        put_digits<P, NB>(X, smem + sm_a + u * CELL + (idx & 31) * 4);
+    }
+    if (wait_op && tid == 0 && !(ok && mbar_wait(bar_op, 0))) *reinterpret_cast<volatile int *>(smem + SM_FAIL) = 1;
+    __syncthreads();
+    ok = *reinterpret_cast<volatile int *>(smem + SM_FAIL) == 0;
+
+    /* ---- products, 16 outputs x 8 lines of one block at a time: a tile of 8 lines fills the MMA.
+     * ldmatrix rows: operator (8 outputs, 8 points) cells at (output half, point half) =
+     * (lane >> 3 & 1, lane >> 4), line cells at (digit, point half) = (lane >> 4, lane >> 3 & 1).
+     * Accumulator v: output (lane >> 2) + 8 (v >> 1), line 2 (lane & 3) + (v & 1) */
+    using Acc = typename std::conditional<std::is_same<P, float>::value, float, long long>::type;
+    Acc *ex = reinterpret_cast<Acc *>(smem + sm_a + tile_bytes(g, S, 8));
+    const int pitch = nc * W * NB + 4; /* values of a line: block by block, shifted by four from line to line */
+    const int nr = (nlines + 7) / 8, np = (nc + 1) / 2, ks = g.hp / 16;
+#pragma unroll 1
+    for (int u = warp; u < nr * np * NB; u += NT / 32) {
+        const int b = u % NB, v = u / NB, rg = nr == 1 ? 0 : v / np, cp = v - rg * np;
+        const int cc = min(2 * cp + ((lane >> 3) & 1), nc - 1); /* an odd last chunk is read twice */
+        const uint32_t a0 = sbase + sm_op + (uint32_t)((cc * NB + b) * ks * SK * 256 + (lane >> 4) * 128 + (lane & 7) * 16);
+        const uint32_t b0 = sbase + sm_a + (uint32_t)((rg * nk8 + ((lane >> 3) & 1)) * CELL + b * 128 + (lane & 7) * 16);
+        float d[L][4];
+#pragma unroll
+        for (int l = 0; l < L; ++l)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) d[l][i] = 0.0f;
+#pragma unroll 1
+        for (int k = 0; k < ks; ++k) {
+            uint32_t bf[(S + 1) / 2][4]; /* line digits 2i, 2i + 1 */
+#pragma unroll
+            for (int i = 0; i < (S + 1) / 2; ++i)
+                ldsm4(bf[i], b0 + (uint32_t)(2 * k * CELL + min(2 * i + (lane >> 4), S - 1) * NB * 128));
+#pragma unroll
+            for (int j = 0; j < SK; ++j) {
+                uint32_t af[4];
+                ldsm4(af, a0 + (uint32_t)((k * SK + j) * 256));
+#pragma unroll
+                for (int i = 0; i < S; ++i)
+                    if (i + j < L) mma16816(d[i + j], af, bf[i / 2][2 * (i & 1)], bf[i / 2][2 * (i & 1) + 1]);
+            }
+        }
+        Acc *at = ex + (rg * 8 + 2 * (lane & 3)) * pitch + (b * nc + 2 * cp) * W + (lane >> 2);
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            if (i < 2 || 2 * cp + 1 < nc) at[(i & 1) * pitch + (i >> 1) * W] = join(d, i);
+    }
+    __syncthreads();
+
+    /* ---- outputs: a warp takes 8 lines x 4 block outputs, and of these all images, or a pair or one
+     * of them where there are too few to go round. Two neighbouring lines' values go in one store:
+     * of a pair of images the even line's thread sends the first, the odd one's the second. */
+    constexpr int NH = NB / 2; /* pairs of images */
+    const int og = nc * (W / 4), units = nr * og;
+    const int parts = units * NB <= NT / 32 ? NB : units * NH <= NT / 32 ? NH : 1;
+#pragma unroll 1
+    for (int w = warp; w < units * parts; w += NT / 32) {
+        const int u = parts == 1 ? w : parts == NB ? w / NB : w / NH, part = parts == 1 ? 0 : w - u * parts;
+        const int rg = nr == 1 ? 0 : (int)__umulhi((unsigned)u, g.mag_og), k = (u - rg * og) * 4 + (lane & 3), r = rg * 8 + (lane >> 2);
+        const bool in = r < nlines && k < hb;
+        const int em = xc.eline[r] & ((1 << EBITS) - 1);
+        const bool bad = em == ExpoMax<P>::v || !ok;
+        const int base = g.ls == 1 ? (L0 + r) * n : L0 + r;
+        const int odd = (lane >> 2) & 1;
+        const Acc *s = ex + r * pitch + k;
+        const Acc sm[2] = {s[0] + s[nc * W], s[0] - s[nc * W]};
+        Acc sp[2] = {0, 0};
+        if constexpr (NB == 4) {
+            sp[0] = s[2 * nc * W] + s[3 * nc * W];
+            sp[1] = s[2 * nc * W] - s[3 * nc * W];
+        }
+        /* image q of pair h: y = q_{s+1} (or the next axis' input) and z, what is sent */
+        auto point = [&](int h, int q, int x, bool on, P &y, P &z) {
+            P f = P(0);
+            if (last && on) f = ldc(xc.bz + base + g.ls * x);
+            from_fix(NB == 2 ? sm[q] : h ? sm[q] - sp[q] : sm[q] + sp[q], em, y);
+            if (bad) set_nan(y);
+            if (last) y = y * f;
+            z = y;
+            if (last && xc.send) z = y * (xc.bnext == xc.bz ? f : on ? ldc(xc.bnext + base + g.ls * x) : P(0));
+        };
+        auto put = [&](int x, P a, P b, unsigned e) {
+            const int to = xc.out_tile == 1 ? x : (int)__umulhi((unsigned)x, xc.out_mag), row = x - to * xc.out_tile;
+            const uint32_t there = at_rank(sbase, to);
+            send(there + xc.out + (uint32_t)((row * xc.out_pitch + L0 + r - odd) * sizeof(P)), there + xc.bar, a, b);
+            if (lane < 8) send_max(there + xc.out_eline + (uint32_t)row * 4, there + xc.bar, (uint32_t)xc.tag | e);
+        };
+        if (parts == NB) {
+            const int x = pos(part, k);
+            const bool line = k < hb && !(NB == 2 && part == 1 && x == k); /* odd n: one middle point */
+            P y, z;
+            if (part & 1)
+                point(part >> 1, 1, x, in && line, y, z);
+            else
+                point(part >> 1, 0, x, in && line, y, z);
+            if (xc.send && ok) { /* nothing is sent after a wait that ran out */
+                unsigned e = in ? (unsigned)expo(z) : 0u;
+                e = max(e, __shfl_xor_sync(0xffffffffu, e, 4));
+                e = max(e, __shfl_xor_sync(0xffffffffu, e, 8));
+                e = max(e, __shfl_xor_sync(0xffffffffu, e, 16));
+                const P got = swap_rows(z);
+                if (line && in && !odd) put(x, z, got, e);
+            }
+            if (last && in && line) xc.dst[base + g.ls * x] = y;
+        } else {
+#pragma unroll 1
+            for (int h = part; h < NH; h += parts) {
+                const int x0 = pos(2 * h, k), x1 = pos(2 * h + 1, k), x = odd ? x1 : x0;
+                const bool line1 = !(NB == 2 && x1 == k);
+                P y0, y1, z0, z1;
+                point(h, 0, x0, in, y0, z0);
+                point(h, 1, x1, in && line1, y1, z1);
+                if (xc.send && ok) {
+                    unsigned e = in ? (unsigned)expo(z0) | (unsigned)expo(z1) << 16 : 0u;
+                    e = __vmaxu2(e, __shfl_xor_sync(0xffffffffu, e, 4));
+                    e = __vmaxu2(e, __shfl_xor_sync(0xffffffffu, e, 8));
+                    e = __vmaxu2(e, __shfl_xor_sync(0xffffffffu, e, 16));
+                    const P got = swap_rows(odd ? z0 : z1);
+                    if (k < hb && r - odd < nlines && (!odd || line1)) put(x, odd ? got : z0, odd ? z1 : got, odd ? e >> 16 : e & 0xffffu);
+                }
+                if (last && in) {
+                    xc.dst[base + g.ls * x0] = y0;
+                    if (line1) xc.dst[base + g.ls * x1] = y1;
+                }
+            }
+        }
+    }
+}
+
 /* One tile of lines and one part of its outputs: y = K x (times b before the
  * first axis, after the last). Ends with every thread of the CTA past the digits. */
 template <typename P, int NB, int NT, bool SPLIT>
 __device__ __forceinline__ void tc_tile(const TcGeom &g, const P *src, P *dst, const P *__restrict__ bz,
                                         bool first, bool last, int tile_i, int part, unsigned char *smem,
-                                        uint32_t sm_op, uint32_t sm_a, uint32_t bar_op, TcPhase &ph)
+                                        uint32_t sm_op, uint32_t sm_a, uint32_t bar_op, bool wait_op, TcPhase &ph)
 {
     constexpr int S = Dig<P>::S, SK = Dig<P>::SK, L = Dig<P>::L;
     using Fix = typename FixT<P>::T;
@@ -415,31 +699,10 @@ __device__ __forceinline__ void tc_tile(const TcGeom &g, const P *src, P *dst, c
                 memcpy(&x, w, sizeof(P));
                 X[p][q] = fix<NB>(x, em);
             }
-        constexpr UFix BIAS = S == 6 ? (UFix)0x0802008020080200ull : (UFix)0x20080200u; /* 512 in every field */
-#pragma unroll
-        for (int q = 0; q < 2; ++q) {
-            if constexpr (NB == 4) { /* half-axis sums, then mirror sums */
-                const Fix a0 = X[0][q] + X[2][q], a1 = X[1][q] + X[3][q], b0 = X[0][q] - X[2][q], b1 = X[1][q] - X[3][q];
-                X[0][q] = a0 + a1;
-                X[1][q] = a0 - a1;
-                X[2][q] = b0 + b1;
-                X[3][q] = b0 - b1;
-            } else {
-                const Fix s = X[0][q] + X[1][q];
-                X[1][q] = X[0][q] - X[1][q];
-                X[0][q] = s;
-            }
-        }
-#pragma unroll
-        for (int b = 0; b < NB; ++b) {
-            const UFix ya = (UFix)X[b][0] + BIAS, yb = (UFix)X[b][1] + BIAS;
-#pragma unroll
-            for (int i = 0; i < S; ++i)
-                *reinterpret_cast<uint32_t *>(cell + (i * NB + b) * 128) = digit2<S, UFix>(ya, yb, i);
-        }
+        put_digits<P, NB>(X, cell);
     }
     /* the operator digits, loaded once: one thread waits for all */
-    if (tid == 0 && !(ph.ok && mbar_wait(bar_op, 0))) *reinterpret_cast<volatile int *>(smem + SM_FAIL) = 1;
+    if (wait_op && tid == 0 && !(ph.ok && mbar_wait(bar_op, 0))) *reinterpret_cast<volatile int *>(smem + SM_FAIL) = 1;
     __syncthreads();
     ph.ok = *reinterpret_cast<volatile int *>(smem + SM_FAIL) == 0;
 
@@ -630,7 +893,7 @@ __global__ void __launch_bounds__(256, 2) k_pass_tc(TcGeom g, PassArgs a)
     P *dst = a.last ? reinterpret_cast<P *>(cd.q) + (long)(a.s + 1) * a.sstride : reinterpret_cast<P *>(cd.tmp);
     const P *bz = reinterpret_cast<const P *>(a.s < cd.seg_end ? cd.b0 : cd.b1);
     TcPhase ph = {0, true};
-    tc_tile<P, NB, 256, false>(g, src, dst, bz, a.first, a.last, tile_i, part, smem, SM_OP, SM_OP + g.op_part, bar_op, ph);
+    tc_tile<P, NB, 256, false>(g, src, dst, bz, a.first, a.last, tile_i, part, smem, SM_OP, SM_OP + g.op_part, bar_op, true, ph);
     if (!ph.ok && threadIdx.x == 0) atomicExch(&g_scft_pass_fault, 1);
 }
 
@@ -678,16 +941,120 @@ __global__ void __launch_bounds__(512, 1) k_chain_tc(const __grid_constant__ TcL
                 for (int t = t0; (long)t * g.tile < g.lines; t += lp.slots[ax]) {
                     if (g.nb == 4)
                         tc_tile<P, 4, 512, true>(g, src, dst, bz, first, last, t, part, smem, lp.op_at[ax], lp.tile_at,
-                                      sbase + SM_BAR + 8 * ax, ph);
+                                                 sbase + SM_BAR + 8 * ax, s == a.s && t == t0, ph);
                     else
                         tc_tile<P, 2, 512, true>(g, src, dst, bz, first, last, t, part, smem, lp.op_at[ax], lp.tile_at,
-                                      sbase + SM_BAR + 8 * ax, ph);
+                                                 sbase + SM_BAR + 8 * ax, s == a.s && t == t0, ph);
                 }
             /* this axis' slice is complete before the next one reads it */
             asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
         }
     }
     if (!ph.ok && threadIdx.x == 0) atomicExch(&g_scft_pass_fault, 1);
+}
+
+/* The same loop on a 2D grid with one tile per CTA and axis, whose lines never
+ * leave shared memory: each output goes straight to the CTA whose line of the
+ * other axis it belongs to (st.async), with the largest exponent of the 8 lines a
+ * warp sends, and that CTA waits for its bytes on its own barrier. No CTA waits
+ * for stores to reach L2, for a cluster barrier and for the loads after it, nor
+ * looks for a line's largest value. A line of one axis has a point of every line
+ * of the other, so a CTA can only be sent lines again once all CTAs, itself
+ * included, have sent what they made of the last ones: one buffer per axis is
+ * enough. Only q_{s+1} goes to global memory, for the densities; what is sent
+ * after the last axis is b q_{s+1} already.
+ *
+ * A step is two serial phases of digits, products and outputs, each bounded by
+ * the latency of its own instructions on small grids (one item a thread) and on
+ * 192x96 by the integer pipe (digits ~1300 + 900 clocks, outputs 2700 + 3000)
+ * and the rate of mma.sync (2500 + 2500), with ~600 between them. FP64, a step:
+ * 32x16 7.0 -> 4.0 us, 64x64 6.9 -> 5.2, 192x96 10.8 -> 8.4 against the loop
+ * above, which stays for 3D grids and for slices that do not fit one tile a CTA. */
+template <typename P>
+__global__ void __launch_bounds__(512, 1) k_chain2d_tc(const __grid_constant__ TcLoop lp, Step2DArgs a)
+{
+    const int rank = blockIdx.x % lp.cluster, slot = blockIdx.x / lp.cluster; /* clusters are consecutive blocks */
+    const ChainDesc cd = a.chains[a.order ? a.order[slot] : slot];
+    if (a.state && a.state[cd.instance].done) return; /* uniform over the cluster */
+    const int s_end = a.s_end < cd.len - 1 ? a.s_end : cd.len - 1;
+    if (a.s >= s_end) return;
+
+    extern __shared__ __align__(128) unsigned char smem[];
+    tc_begin(smem, 4); /* operator digits of the two axes, lines of the two axes */
+    const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(smem), bars = sbase + SM_BAR;
+    bool mine[2], ok = true;
+    uint32_t bytes[2];
+#pragma unroll
+    for (int ax = 0; ax < 2; ++ax) {
+        const TcGeom &g = lp.g[ax];
+        mine[ax] = (long)rank * g.tile < g.lines;
+        /* a line's values, in pairs, and the largest exponent of each 8 of them that one warp sends */
+        bytes[ax] = mine[ax] ? (uint32_t)(min((long)g.tile, g.lines - (long)rank * g.tile) * ((g.n + 1) / 2 * 2 * sizeof(P) + (g.n + 7) / 8 * 4)) : 0u;
+        if (mine[ax] && threadIdx.x == 32) {
+            if (g.nb == 4)
+                tc_start_op<P, 4>(g, cd.ops->tc[ax], 0, sbase + lp.op_at[ax], bars + 8 * ax);
+            else
+                tc_start_op<P, 2>(g, cd.ops->tc[ax], 0, sbase + lp.op_at[ax], bars + 8 * ax);
+            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bars + 16 + 8 * ax), "r"(bytes[ax]) : "memory");
+        }
+    }
+    /* the first lines: b q_s from global memory */
+    if (mine[0]) {
+        const TcGeom &g = lp.g[0];
+        const P *src = reinterpret_cast<const P *>(cd.q) + (long)a.s * a.sstride;
+        const P *bz = reinterpret_cast<const P *>(a.s < cd.seg_end ? cd.b0 : cd.b1);
+        P *in = reinterpret_cast<P *>(smem + lp.buf_at[0]);
+        int *eline = reinterpret_cast<int *>(smem + SM_ELINE);
+        const int L0 = rank * g.tile, nlines = (int)min((long)g.tile, g.lines - L0);
+        for (int i = threadIdx.x; i < nlines * g.n; i += 512) {
+            const int x = i / nlines, r = i - x * nlines; /* lines of the slowest axis: neighbours in memory */
+            const long at = g.ls == 1 ? (long)(L0 + r) * g.n + x : (long)x * g.ls + L0 + r;
+            const P v = ld1(src + at) * ld1(bz + at);
+            in[r * lp.pitch[0] + x] = v;
+            atomicMax(&eline[r], expo(v));
+        }
+    }
+    /* every CTA's barriers are set up before anyone sends */
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+#pragma unroll 1
+    for (int s = a.s; s < s_end; ++s) {
+        const P *bz = reinterpret_cast<const P *>(s < cd.seg_end ? cd.b0 : cd.b1);
+#pragma unroll 1
+        for (int ax = 0; ax < 2; ++ax) {
+            if (!mine[ax]) continue;
+            const TcGeom &g = lp.g[ax], &o = lp.g[1 - ax];
+            const int t = s - a.s;
+            if (t > 0 || ax == 1) {
+                /* the lines are there; one thread re-arms the barrier for the next step */
+                const uint32_t bar = bars + 16 + 8 * ax;
+                const bool got = ok && mbar_wait<true>(bar, (uint32_t)(t - 1 + ax) & 1u);
+                if (!got) *reinterpret_cast<volatile int *>(smem + SM_FAIL) = 1;
+                if (got && s + 1 < s_end && threadIdx.x == 0)
+                    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes[ax]) : "memory");
+            }
+            const Exchange<P> xc = {reinterpret_cast<const P *>(smem + lp.buf_at[ax]),
+                                    reinterpret_cast<const int *>(smem + SM_ELINE) + ax * ROWS,
+                                    lp.pitch[ax],
+                                    (t + 1 + ax) << EBITS, /* larger than all before: the maxima need no reset */
+                                    lp.buf_at[1 - ax],
+                                    SM_ELINE + (1 - ax) * ROWS * 4,
+                                    SM_BAR + 16 + 8 * (1 - ax),
+                                    lp.pitch[1 - ax],
+                                    o.tile,
+                                    lp.mag_tile[1 - ax],
+                                    ax == 0 || s + 1 < s_end,
+                                    bz,
+                                    reinterpret_cast<const P *>(s + 1 < cd.seg_end ? cd.b0 : cd.b1),
+                                    reinterpret_cast<P *>(cd.q) + (long)(s + 1) * a.sstride};
+            if (g.nb == 4)
+                tc_tile2d<P, 4, 512>(g, xc, ax == 1, rank, smem, lp.op_at[ax], lp.tile_at, bars + 8 * ax, t == 0, ok);
+            else
+                tc_tile2d<P, 2, 512>(g, xc, ax == 1, rank, smem, lp.op_at[ax], lp.tile_at, bars + 8 * ax, t == 0, ok);
+        }
+    }
+    if (!ok && threadIdx.x == 0) atomicExch(&g_scft_pass_fault, 1);
+    /* no CTA leaves while another could still send to it */
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
 /* ------------------------------------------------------------- launchers */
@@ -730,10 +1097,17 @@ size_t scft_chain_tc_layout(int prec, TcLoop &lp)
     for (int ax = 0; ax < lp.nax; ++ax) {
         lp.op_at[ax] = at;
         at += (lp.g[ax].op_part + 127) / 128 * 128;
-        const uint32_t b = prec == SCFT_PREC_FP32 ? tile_bytes(lp.g[ax], Dig<float>::S) + exchange_bytes(lp.g[ax], 4)
-                                                  : tile_bytes(lp.g[ax], Dig<double>::S) + exchange_bytes(lp.g[ax], 8);
+        const int S = prec == SCFT_PREC_FP32 ? Dig<float>::S : Dig<double>::S, value = prec == SCFT_PREC_FP32 ? 4 : 8;
+        const uint32_t b = lp.exchange ? tile_bytes(lp.g[ax], S, 8) + exchange2d_bytes(lp.g[ax], value)
+                                       : tile_bytes(lp.g[ax], S) + exchange_bytes(lp.g[ax], value);
         if (b > tile) tile = b;
         lp.slots[ax] = lp.cluster / lp.g[ax].parts;
+        if (lp.exchange) { /* lines, shifted by half the banks from one to the next */
+            lp.pitch[ax] = (lp.g[ax].n + 15) / 16 * 16 + 8;
+            lp.buf_at[ax] = at;
+            lp.mag_tile[ax] = (unsigned)((0xFFFFFFFFull + lp.g[ax].tile) / lp.g[ax].tile);
+            at += (uint32_t)(lp.g[ax].tile * lp.pitch[ax] * value + 127) / 128 * 128;
+        }
     }
     lp.tile_at = at;
     return (size_t)at + tile;
@@ -756,6 +1130,10 @@ static cudaError_t launch_chain(const TcLoop &lp, const Step2DArgs &a, int nchai
     attr.val.clusterDim.z = 1;
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
+    if (lp.exchange) {
+        if (clusters) return cudaOccupancyMaxActiveClusters(clusters, k_chain2d_tc<P>, &cfg);
+        return cudaLaunchKernelEx(&cfg, k_chain2d_tc<P>, l, a);
+    }
     if (clusters) return cudaOccupancyMaxActiveClusters(clusters, k_chain_tc<P>, &cfg);
     return cudaLaunchKernelEx(&cfg, k_chain_tc<P>, l, a);
 }
@@ -774,13 +1152,15 @@ template <typename P>
 static cudaError_t configure_tc(int smem_bytes)
 {
     /* one carve-out for every pass, so the SMs keep their split between launches */
-    const void *k[] = {(const void *)k_pass_tc<P, 4>, (const void *)k_pass_tc<P, 2>, (const void *)k_chain_tc<P>};
+    const void *k[] = {(const void *)k_pass_tc<P, 4>, (const void *)k_pass_tc<P, 2>, (const void *)k_chain_tc<P>,
+                       (const void *)k_chain2d_tc<P>};
     cudaError_t e = cudaSuccess;
     for (const void *f : k) {
         if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
         if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
     }
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k_chain_tc<P>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_chain2d_tc<P>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     return e;
 }
 

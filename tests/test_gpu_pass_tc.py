@@ -73,3 +73,28 @@ def test_steps_against_dense_operators(srn, grid, prec):
         # levels and the rounding of the result, half an ulp of the largest value each
         # (their sums over blocks in FP32: as much again)
         assert err <= (t + 1) * (4 + 4 * naxes) * ULP[prec]
+
+
+@pytest.mark.parametrize("prec", ("fp64", "fp32x2", "fp32"))
+@pytest.mark.parametrize("grid", [(8, 9), (9, 11), (17, 33), (30, 15), (60, 64), (75, 26), (150, 75), (108, 100)])
+def test_solve_in_one_loop_equals_passes(srn, grid, prec):
+    """Whole iterations (two blocks' factors, both directions of a chain, a batch) with
+    the contour loop chosen by rule: ragged tiles of both axes, lines passed between
+    clusters of several sizes. The same integers are summed, so the bits are equal."""
+    nx, nz = grid
+    s = srn.configs.film2d(ns=32) if nx % 2 else srn.configs.bulk2d()
+    s.LX, s.LZ = nx * s.DR_TARGET * (1.02 if nx == 8 else 1.0), nz * s.DR_TARGET
+    out = {}
+    for path in ("auto", "passes"):
+        with srn.Solver([s, s], precision=prec, kernel_path=path, autotune=False) as sv:
+            assert sv.grid == (nx, 1, nz)
+            rng = np.random.default_rng(nx + nz)
+            for b in range(2):
+                sv.set_fields(rng.uniform(-1.0, 1.0, 14 * sv.M), b)
+                if nx % 2:
+                    sv.set_masks(srn.configs.substrate_mask(s), b)
+                sv.set_iteration(1, b)
+            res = sv.iterate(2)
+            out[path] = [sv.get_fields(b) for b in range(2)], [[r.free_energy for r in step] for step in res]
+    assert np.isfinite(out["auto"][0]).all()
+    assert np.array_equal(out["auto"][0], out["passes"][0]) and out["auto"][1] == out["passes"][1]
