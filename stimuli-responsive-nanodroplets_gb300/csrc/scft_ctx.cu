@@ -757,18 +757,15 @@ struct TcChoice {
 /* Clocks of a tile, roughly: loading and splitting per item of 2 NB points, 20 per
  * MMA (16 is the rate), joining and writing the outputs. In the loop (512 threads)
  * a warp multiplies one block at a time, in a pass of its own (256) all blocks. */
-static double tc_cta_cost(const TcGeom &g, int prec, int threads, int exchange = 0)
+static double tc_cta_cost(const TcGeom &g, int prec, int threads, int loop = 0)
 {
     const double items = std::ceil(g.tile * (g.hp / 2) / (double)threads), mmas = prec == SCFT_PREC_FP32 ? 9.0 : 21.0;
     const double block = g.hp / 16 * mmas * 20.0 + 300.0, work = (g.tile + 15) / 16 * g.cpp, warps = threads / 32.0;
-    if (exchange) { /* blocks of 16 outputs x 8 lines, at the latency of one or the rate of all (~13 clocks an MMA) */
+    if (loop) { /* blocks of 16 outputs x 8 lines, at the latency of one or the rate of all (~13 clocks an MMA) */
         const double blocks = (g.tile + 7) / 8 * ((g.cpp + 1) / 2) * g.nb;
         return 1500.0 + items * g.nb * 350.0 + std::max(std::ceil(blocks / warps) * block, blocks * g.hp / 16 * mmas * 13.0 / 4) +
                std::max(1200.0, g.tile * g.cpp * 8 * g.nb * 2.0);
     }
-    if (threads == 512) /* loop: a block at a time, then the outputs */
-        return 2000.0 + items * g.nb * 350.0 + std::ceil(work * g.nb / warps) * block +
-               std::ceil(g.tile * g.cpp * 8 / (double)threads) * g.nb * 300.0;
     return 2000.0 + items * g.nb * 350.0 + std::ceil(work / warps) * g.nb * (block + 500.0);
 }
 
@@ -1009,7 +1006,8 @@ static double tc_loop_plan(const scft_ctx *c, int cluster, int smem_limit, TcLoo
                 TcGeom g = g0;
                 if (!tc_apply(prec, g, t, parts, smem_limit)) continue;
                 const long slots = cluster / parts, tiles = (g.lines + t - 1) / t;
-                cand[ax].push_back({(double)((tiles + slots - 1) / slots) * tc_cta_cost(g, prec, 512) + 1500.0, g});
+                /* two groups share the SM: each tile takes ~1.5 times as long as alone */
+                cand[ax].push_back({(double)((tiles + 2 * slots - 1) / (2 * slots)) * (tiles > slots ? 1.5 : 1.0) * (1000.0 + tc_cta_cost(g, prec, 256, 1)) + 1500.0, g});
             }
         }
         std::stable_sort(cand[ax].begin(), cand[ax].end(), [](const std::pair<double, TcGeom> &x, const std::pair<double, TcGeom> &y) { return x.first < y.first; });

@@ -157,7 +157,7 @@ struct TcLoop {
     TcGeom g[3];
     int slots[3];      /* tiles taken side by side: cluster / parts */
     unsigned op_at[3]; /* shared-memory offsets of the axes' operator digits and of the tile region */
-    unsigned tile_at;
+    unsigned tile_at, tile_bytes;
     /* exchange: the axes' lines in shared memory, values from line to line, ceil(2^32 / tile) */
     unsigned buf_at[2], mag_tile[2];
     int pitch[2];

@@ -66,6 +66,7 @@ namespace {
 
 constexpr int W = 8;      /* block outputs of a chunk (the N of an MMA) */
 constexpr int ROWS = 128; /* lines of the largest tile */
+constexpr int GROUPS = 2; /* groups of warps of k_chain_tc, each with its own tiles */
 
 /* digits of the data, of the operator, and levels kept */
 template <typename P>
@@ -337,25 +338,54 @@ __device__ __forceinline__ void set_nan(float &y) { y = __int_as_float(0x7fc0000
 
 /* Shared memory (byte offsets): one barrier per axis, two sets of line exponents,
  * operator digits (one region per axis), then the digits of a tile's lines. */
-constexpr uint32_t SM_BAR = 0, SM_FAIL = 32, SM_ELINE = 64, SM_OP = SM_ELINE + 2 * ROWS * 4;
+constexpr uint32_t SM_BAR = 0, SM_FAIL = 32, SM_ELINE = 64, SM_OP = SM_ELINE + 4 * ROWS * 4;
 
-/* bytes of a tile's digits (an MMA of a pass reads 16 lines, of k_chain2d_tc 8) */
-__host__ __device__ inline uint32_t tile_bytes(const TcGeom &g, int digits, int lines = 16)
+/* bytes of a tile's digits (an MMA of a pass reads 16 lines, of the loops 8) */
+__host__ __device__ inline uint32_t tile_bytes(const TcGeom &g, int digits, int lines)
 {
     return (uint32_t)((g.tile + lines - 1) / lines * lines) * g.hp * g.nb * digits * 2;
 }
 
-/* bytes of the exchange of block sums, for a part of the outputs (k_chain_tc, k_chain2d_tc) */
+/* bytes of the exchange of block sums in the loops, for a part of the outputs */
 __host__ __device__ inline uint32_t exchange_bytes(const TcGeom &g, int value)
-{
-    return (uint32_t)((g.tile + 15) / 16 * 16) * (g.cpp * W * g.nb + 2) * value;
-}
-__host__ __device__ inline uint32_t exchange2d_bytes(const TcGeom &g, int value)
 {
     return (uint32_t)g.tile * (g.cpp * W * g.nb + 4) * value;
 }
 
-/* Where a CTA is. */
+/* Level sums of 16 outputs (chunks 2 cp, 2 cp + 1) x 8 lines (group rg) of block b: tiles of 8
+ * lines fill the MMA. ldmatrix rows: operator (8 outputs, 8 points) cells at (output half, point
+ * half) = (lane >> 3 & 1, lane >> 4), line cells at (digit, point half) = (lane >> 4, lane >> 3 & 1).
+ * d[.][v]: output (lane >> 2) + 8 (v >> 1), line 2 (lane & 3) + (v & 1). */
+template <typename P, int NB>
+__device__ __forceinline__ void products16x8(float (&d)[Dig<P>::L][4], uint32_t op, uint32_t lines, int nk8, int ks, int nc, int rg, int cp, int b)
+{
+    constexpr int S = Dig<P>::S, SK = Dig<P>::SK, L = Dig<P>::L, CELL = S * NB * 128;
+    const int lane = threadIdx.x & 31;
+    const int cc = min(2 * cp + ((lane >> 3) & 1), nc - 1); /* an odd last chunk is read twice */
+    const uint32_t a0 = op + (uint32_t)((cc * NB + b) * ks * SK * 256 + (lane >> 4) * 128 + (lane & 7) * 16);
+    const uint32_t b0 = lines + (uint32_t)((rg * nk8 + ((lane >> 3) & 1)) * CELL + b * 128 + (lane & 7) * 16);
+#pragma unroll
+    for (int l = 0; l < L; ++l)
+#pragma unroll
+        for (int v = 0; v < 4; ++v) d[l][v] = 0.0f;
+#pragma unroll 1
+    for (int k = 0; k < ks; ++k) {
+        uint32_t bf[(S + 1) / 2][4]; /* line digits 2i, 2i + 1 */
+#pragma unroll
+        for (int i = 0; i < (S + 1) / 2; ++i)
+            ldsm4(bf[i], b0 + (uint32_t)(2 * k * CELL + min(2 * i + (lane >> 4), S - 1) * NB * 128));
+#pragma unroll
+        for (int j = 0; j < SK; ++j) {
+            uint32_t af[4];
+            ldsm4(af, a0 + (uint32_t)((k * SK + j) * 256));
+#pragma unroll
+            for (int i = 0; i < S; ++i)
+                if (i + j < L) mma16816(d[i + j], af, bf[i / 2][2 * (i & 1)], bf[i / 2][2 * (i & 1) + 1]);
+        }
+    }
+}
+
+/* Where a CTA (or a group of its warps) is. */
 struct TcPhase {
     uint32_t tile; /* tiles done */
     bool ok;       /* no wait has given up */
@@ -421,7 +451,7 @@ template <typename P, int NB, int NT>
 __device__ __forceinline__ void tc_tile2d(const TcGeom &g, const Exchange<P> &xc, bool last, int tile_i, unsigned char *smem,
                                           uint32_t sm_op, uint32_t sm_a, uint32_t bar_op, bool wait_op, bool &ok)
 {
-    constexpr int S = Dig<P>::S, SK = Dig<P>::SK, L = Dig<P>::L, CELL = S * NB * 128;
+    constexpr int S = Dig<P>::S, L = Dig<P>::L, CELL = S * NB * 128;
     using Fix = typename FixT<P>::T;
     const int tid = threadIdx.x, lane = tid & 31;
     const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0); /* uniform */
@@ -462,10 +492,7 @@ __device__ __forceinline__ void tc_tile2d(const TcGeom &g, const Exchange<P> &xc
     __syncthreads();
     ok = *reinterpret_cast<volatile int *>(smem + SM_FAIL) == 0;
 
-    /* ---- products, 16 outputs x 8 lines of one block at a time: a tile of 8 lines fills the MMA.
-     * ldmatrix rows: operator (8 outputs, 8 points) cells at (output half, point half) =
-     * (lane >> 3 & 1, lane >> 4), line cells at (digit, point half) = (lane >> 4, lane >> 3 & 1).
-     * Accumulator v: output (lane >> 2) + 8 (v >> 1), line 2 (lane & 3) + (v & 1) */
+    /* ---- products, 16 outputs x 8 lines of one block at a time */
     using Acc = typename std::conditional<std::is_same<P, float>::value, float, long long>::type;
     Acc *ex = reinterpret_cast<Acc *>(smem + sm_a + tile_bytes(g, S, 8));
     const int pitch = nc * W * NB + 4; /* values of a line: block by block, shifted by four from line to line */
@@ -473,29 +500,8 @@ __device__ __forceinline__ void tc_tile2d(const TcGeom &g, const Exchange<P> &xc
 #pragma unroll 1
     for (int u = warp; u < nr * np * NB; u += NT / 32) {
         const int b = u % NB, v = u / NB, rg = nr == 1 ? 0 : v / np, cp = v - rg * np;
-        const int cc = min(2 * cp + ((lane >> 3) & 1), nc - 1); /* an odd last chunk is read twice */
-        const uint32_t a0 = sbase + sm_op + (uint32_t)((cc * NB + b) * ks * SK * 256 + (lane >> 4) * 128 + (lane & 7) * 16);
-        const uint32_t b0 = sbase + sm_a + (uint32_t)((rg * nk8 + ((lane >> 3) & 1)) * CELL + b * 128 + (lane & 7) * 16);
         float d[L][4];
-#pragma unroll
-        for (int l = 0; l < L; ++l)
-#pragma unroll
-            for (int i = 0; i < 4; ++i) d[l][i] = 0.0f;
-#pragma unroll 1
-        for (int k = 0; k < ks; ++k) {
-            uint32_t bf[(S + 1) / 2][4]; /* line digits 2i, 2i + 1 */
-#pragma unroll
-            for (int i = 0; i < (S + 1) / 2; ++i)
-                ldsm4(bf[i], b0 + (uint32_t)(2 * k * CELL + min(2 * i + (lane >> 4), S - 1) * NB * 128));
-#pragma unroll
-            for (int j = 0; j < SK; ++j) {
-                uint32_t af[4];
-                ldsm4(af, a0 + (uint32_t)((k * SK + j) * 256));
-#pragma unroll
-                for (int i = 0; i < S; ++i)
-                    if (i + j < L) mma16816(d[i + j], af, bf[i / 2][2 * (i & 1)], bf[i / 2][2 * (i & 1) + 1]);
-            }
-        }
+        products16x8<P, NB>(d, sbase + sm_op, sbase + sm_a, nk8, ks, nc, rg, cp, b);
         Acc *at = ex + (rg * 8 + 2 * (lane & 3)) * pitch + (b * nc + 2 * cp) * W + (lane >> 2);
 #pragma unroll
         for (int i = 0; i < 4; ++i)
@@ -593,11 +599,18 @@ __device__ __forceinline__ void tc_tile(const TcGeom &g, const P *src, P *dst, c
     constexpr int S = Dig<P>::S, SK = Dig<P>::SK, L = Dig<P>::L;
     using Fix = typename FixT<P>::T;
     using UFix = typename std::make_unsigned<Fix>::type;
-    const int tid = threadIdx.x, lane = tid & 31;
+    /* SPLIT: a group of NT threads with its own barrier */
+    const int tid = SPLIT ? threadIdx.x % NT : threadIdx.x, lane = tid & 31, group = SPLIT ? threadIdx.x / NT : 0;
     const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0); /* uniform */
+    auto sync = [&]() {
+        if (SPLIT)
+            asm volatile("bar.sync %0, %1;" ::"r"(1 + group), "n"(NT) : "memory");
+        else
+            __syncthreads();
+    };
     /* line exponents: one set in use, the other zeroed for the next tile */
-    int *eline = reinterpret_cast<int *>(smem + SM_ELINE) + (ph.tile & 1) * ROWS;
-    int *enext = reinterpret_cast<int *>(smem + SM_ELINE) + (~ph.tile & 1) * ROWS;
+    int *eline = reinterpret_cast<int *>(smem + SM_ELINE) + (2 * group + (ph.tile & 1)) * ROWS;
+    int *enext = reinterpret_cast<int *>(smem + SM_ELINE) + (2 * group + (~ph.tile & 1)) * ROWS;
     ++ph.tile;
     const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(smem);
     const int c0 = part * g.cpp, c1 = min(c0 + g.cpp, g.nchunks);
@@ -676,7 +689,7 @@ __device__ __forceinline__ void tc_tile(const TcGeom &g, const P *src, P *dst, c
             }
         atomicMax(&eline[r], em);
     }
-    __syncthreads();
+    sync();
 
     if (tid < ROWS) enext[tid] = 0;
     /* ---- digits of the block operands, over the item's own words */
@@ -703,42 +716,12 @@ __device__ __forceinline__ void tc_tile(const TcGeom &g, const P *src, P *dst, c
     }
     /* the operator digits, loaded once: one thread waits for all */
     if (wait_op && tid == 0 && !(ph.ok && mbar_wait(bar_op, 0))) *reinterpret_cast<volatile int *>(smem + SM_FAIL) = 1;
-    __syncthreads();
+    sync();
     ph.ok = *reinterpret_cast<volatile int *>(smem + SM_FAIL) == 0;
 
-    /* ---- products, 16 lines x 8 outputs at a time, and the levels joined in registers */
+    /* ---- products, and the levels joined in registers */
     using Acc = typename std::conditional<std::is_same<P, float>::value, float, long long>::type;
-    const int lt = (nlines + 15) / 16, nc = min(c1, (hb + W - 1) / W) - c0, ks = g.hp / 16;
-    /* ldmatrix rows: A (8 lines, 8 points) cells at (line half, point half) = (lane >> 3 & 1, lane >> 4),
-     * B (8 outputs, 8 points) cells at (digit, point half) = (lane >> 4, lane >> 3 & 1) */
-    const uint32_t a_lane = sbase + sm_a + (uint32_t)((((lane >> 3) & 1) * nk8 + (lane >> 4)) * CELL + (lane & 7) * 16);
-    const uint32_t b_lane = sbase + sm_op + (uint32_t)((lane >> 4) * 256 + ((lane >> 3) & 1) * 128 + (lane & 7) * 16);
-    /* accumulator v: line (lane >> 2) + 8 (v >> 1), output 2 (lane & 3) + (v & 1) */
-    auto products = [&](int l16, int cc, int b, Acc (&acc)[4]) {
-        const uint32_t a0 = a_lane + (uint32_t)(l16 * 2 * nk8 * CELL + b * 128);
-        const uint32_t b0 = b_lane + (uint32_t)((cc * NB + b) * ks * SK * 256);
-        float d[L][4];
-#pragma unroll
-        for (int l = 0; l < L; ++l)
-#pragma unroll
-            for (int v = 0; v < 4; ++v) d[l][v] = 0.0f;
-#pragma unroll 1
-        for (int k = 0; k < ks; ++k) {
-            uint32_t bf[SK / 2][4]; /* digits 2j, 2j + 1 */
-#pragma unroll
-            for (int j = 0; j < SK / 2; ++j) ldsm4(bf[j], b0 + (uint32_t)(k * SK * 256 + j * 512));
-#pragma unroll
-            for (int i = 0; i < S; ++i) {
-                uint32_t af[4];
-                ldsm4(af, a0 + (uint32_t)(2 * k * CELL + i * NB * 128));
-#pragma unroll
-                for (int j = 0; j < SK; ++j)
-                    if (i + j < L) mma16816(d[i + j], af, bf[j / 2][2 * (j & 1)], bf[j / 2][2 * (j & 1) + 1]);
-            }
-        }
-#pragma unroll
-        for (int v = 0; v < 4; ++v) acc[v] = join(d, v);
-    };
+    const int nc = min(c1, (hb + W - 1) / W) - c0, ks = g.hp / 16;
     /* block sums back to the NB points of an output */
     auto points = [&](const Acc (&s)[NB], int em, P (&y)[NB]) {
         Acc t[NB];
@@ -759,25 +742,28 @@ __device__ __forceinline__ void tc_tile(const TcGeom &g, const P *src, P *dst, c
         }
     };
     if constexpr (SPLIT) {
-        /* a warp takes one block of them, and the sums meet in shared memory: four (two) times as
-         * many, shorter pieces of work, for tiles that would leave warps without any */
-        Acc *ex = reinterpret_cast<Acc *>(smem + sm_a + tile_bytes(g, S));
-        const int pitch = nc * W * NB + 2; /* values of a line: 16-byte rows, shifted by a bank group */
+        /* a warp takes one block of 16 outputs x 8 lines, and the sums meet in shared memory: four
+         * (two) times as many, shorter pieces of work as with all blocks in one warp */
+        Acc *ex = reinterpret_cast<Acc *>(smem + sm_a + tile_bytes(g, S, 8));
+        const int pitch = nc * W * NB + 4; /* values of a line: block by block, shifted by four from line to line */
+        const int nr = (nlines + 7) / 8, np = (nc + 1) / 2;
 #pragma unroll 1
-        for (int u = warp; u < lt * nc * NB; u += NT / 32) {
-            const int b = u % NB, v = u / NB, cc = v / lt, l16 = v - cc * lt;
-            Acc acc[4];
-            products(l16, cc, b, acc);
+        for (int u = warp; u < nr * np * NB; u += NT / 32) {
+            const int b = u % NB, v = u / NB, rg = nr == 1 ? 0 : v / np, cp = v - rg * np;
+            float d[L][4];
+            products16x8<P, NB>(d, sbase + sm_op, sbase + sm_a, nk8, ks, nc, rg, cp, b);
+            Acc *at = ex + (rg * 8 + 2 * (lane & 3)) * pitch + (b * nc + 2 * cp) * W + (lane >> 2);
 #pragma unroll
-            for (int v4 = 0; v4 < 4; ++v4)
-                ex[(l16 * 16 + (lane >> 2) + 8 * (v4 >> 1)) * pitch + (cc * W + 2 * (lane & 3) + (v4 & 1)) * NB + b] = acc[v4];
+            for (int i = 0; i < 4; ++i)
+                if (i < 2 || 2 * cp + 1 < nc) at[(i & 1) * pitch + (i >> 1) * W] = join(d, i);
         }
-        __syncthreads();
+        sync();
         /* a warp takes 8 lines x 4 outputs: whole sectors along either direction */
-        const int og = nc * (W / 4);
+        const int og = g.cpp * (W / 4);
 #pragma unroll 1
-        for (int idx = tid; idx < (nlines + 7) / 8 * og * 32; idx += NT) {
-            const int u = idx >> 5, rg = u / og, o = (u - rg * og) * 4 + (idx & 3), r = rg * 8 + ((idx >> 2) & 7), k = c0 * W + o;
+        for (int u = warp; u < nr * og; u += NT / 32) {
+            const int rg = nr == 1 ? 0 : (int)__umulhi((unsigned)u, g.mag_og), o = (u - rg * og) * 4 + (lane & 3);
+            const int r = rg * 8 + (lane >> 2), k = c0 * W + o;
             if (r >= nlines || k >= hb) continue;
             const int base = line_base(r);
             P f[NB], y[NB];
@@ -787,12 +773,44 @@ __device__ __forceinline__ void tc_tile(const TcGeom &g, const P *src, P *dst, c
             }
             Acc s[NB];
 #pragma unroll
-            for (int b = 0; b < NB; ++b) s[b] = ex[r * pitch + o * NB + b];
+            for (int b = 0; b < NB; ++b) s[b] = ex[r * pitch + b * nc * W + o];
             points(s, eline[r], y);
 #pragma unroll
             for (int p = 0; p < NB; ++p) dst[base + ls * pos(p, k)] = last ? y[p] * f[p] : y[p];
         }
     } else {
+        /* 16 lines x 8 outputs at a time */
+        const int lt = (nlines + 15) / 16;
+        /* ldmatrix rows: A (8 lines, 8 points) cells at (line half, point half) = (lane >> 3 & 1, lane >> 4),
+         * B (8 outputs, 8 points) cells at (digit, point half) = (lane >> 4, lane >> 3 & 1) */
+        const uint32_t a_lane = sbase + sm_a + (uint32_t)((((lane >> 3) & 1) * nk8 + (lane >> 4)) * CELL + (lane & 7) * 16);
+        const uint32_t b_lane = sbase + sm_op + (uint32_t)((lane >> 4) * 256 + ((lane >> 3) & 1) * 128 + (lane & 7) * 16);
+        /* accumulator v: line (lane >> 2) + 8 (v >> 1), output 2 (lane & 3) + (v & 1) */
+        auto products = [&](int l16, int cc, int b, Acc (&acc)[4]) {
+            const uint32_t a0 = a_lane + (uint32_t)(l16 * 2 * nk8 * CELL + b * 128);
+            const uint32_t b0 = b_lane + (uint32_t)((cc * NB + b) * ks * SK * 256);
+            float d[L][4];
+#pragma unroll
+            for (int l = 0; l < L; ++l)
+#pragma unroll
+                for (int v = 0; v < 4; ++v) d[l][v] = 0.0f;
+#pragma unroll 1
+            for (int k = 0; k < ks; ++k) {
+                uint32_t bf[SK / 2][4]; /* digits 2j, 2j + 1 */
+#pragma unroll
+                for (int j = 0; j < SK / 2; ++j) ldsm4(bf[j], b0 + (uint32_t)(k * SK * 256 + j * 512));
+#pragma unroll
+                for (int i = 0; i < S; ++i) {
+                    uint32_t af[4];
+                    ldsm4(af, a0 + (uint32_t)(2 * k * CELL + i * NB * 128));
+#pragma unroll
+                    for (int j = 0; j < SK; ++j)
+                        if (i + j < L) mma16816(d[i + j], af, bf[j / 2][2 * (j & 1)], bf[j / 2][2 * (j & 1) + 1]);
+                }
+            }
+#pragma unroll
+            for (int v = 0; v < 4; ++v) acc[v] = join(d, v);
+        };
         /* a warp takes all blocks of them and writes the outputs from its registers */
 #pragma unroll 1
         for (int u = warp; u < lt * nc; u += NT / 32) {
@@ -841,7 +859,7 @@ __device__ __forceinline__ void tc_tile(const TcGeom &g, const P *src, P *dst, c
             }
         }
     }
-    __syncthreads();
+    sync();
 }
 
 /* This part's operator digits. */
@@ -862,7 +880,7 @@ __device__ __forceinline__ void tc_start_op(const TcGeom &g, const void *table, 
 /* Barriers and line exponents; ends with a CTA barrier. */
 __device__ __forceinline__ void tc_begin(unsigned char *smem, int nax)
 {
-    for (int i = threadIdx.x; i < 2 * ROWS; i += blockDim.x) reinterpret_cast<int *>(smem + SM_ELINE)[i] = 0;
+    for (int i = threadIdx.x; i < 4 * ROWS; i += blockDim.x) reinterpret_cast<int *>(smem + SM_ELINE)[i] = 0;
     if (threadIdx.x == 32) {
         *reinterpret_cast<volatile int *>(smem + SM_FAIL) = 0;
         for (int i = 0; i < nax; ++i)
@@ -903,7 +921,12 @@ __global__ void __launch_bounds__(256, 2) k_pass_tc(TcGeom g, PassArgs a)
  * one axis, then q_{s+1}), ordered by a cluster barrier after each axis. A step
  * thus costs two or three short phases per CTA, without the launches, the
  * set-up and the cold instruction cache that a pass of its own has (~4 of 8 us
- * on a 192x96 slice). Control flow is uniform over the cluster. */
+ * on a 192x96 slice). Two groups of warps with a barrier each take their own
+ * tiles, so that one splits or writes while the other multiplies: 46.5 -> 43.2 us a
+ * step for 192x96 chains of two CTAs with the GPU full, against one tile of all
+ * 512 threads at a time (three groups, or groups of 384 threads, do not fit or
+ * gain nothing: issue slots are ~45 % busy, shared memory 50 %, and neither more
+ * warps nor more overlap moves that). Control flow is uniform over the cluster. */
 template <typename P>
 __global__ void __launch_bounds__(512, 1) k_chain_tc(const __grid_constant__ TcLoop lp, Step2DArgs a)
 {
@@ -919,13 +942,15 @@ __global__ void __launch_bounds__(512, 1) k_chain_tc(const __grid_constant__ TcL
     if (threadIdx.x == 32)
         for (int ax = 0; ax < lp.nax; ++ax) {
             const TcGeom &g = lp.g[ax];
-            if (rank / g.parts >= lp.slots[ax]) continue;
+            if (rank / g.parts >= lp.slots[ax] || (long)(rank / g.parts) * g.tile >= g.lines) continue;
             if (g.nb == 4)
                 tc_start_op<P, 4>(g, cd.ops->tc[ax], rank % g.parts, sbase + lp.op_at[ax], sbase + SM_BAR + 8 * ax);
             else
                 tc_start_op<P, 2>(g, cd.ops->tc[ax], rank % g.parts, sbase + lp.op_at[ax], sbase + SM_BAR + 8 * ax);
         }
     TcPhase ph = {0, true};
+    const int group = threadIdx.x / (512 / GROUPS);
+    const uint32_t tile_at = lp.tile_at + (uint32_t)group * lp.tile_bytes;
 #pragma unroll 1
     for (int s = a.s; s < s_end; ++s) {
         const P *bz = reinterpret_cast<const P *>(s < cd.seg_end ? cd.b0 : cd.b1);
@@ -935,22 +960,22 @@ __global__ void __launch_bounds__(512, 1) k_chain_tc(const __grid_constant__ TcL
             const bool first = ax == 0, last = ax == lp.nax - 1;
             const P *src = first ? reinterpret_cast<const P *>(cd.q) + (long)s * a.sstride : reinterpret_cast<const P *>(cd.tmp);
             P *dst = last ? reinterpret_cast<P *>(cd.q) + (long)(s + 1) * a.sstride : reinterpret_cast<P *>(cd.tmp);
-            const int t0 = rank / g.parts, part = rank % g.parts;
-            if (t0 < lp.slots[ax])
+            const int t0 = rank / g.parts + group * lp.slots[ax], part = rank % g.parts;
+            if (rank / g.parts < lp.slots[ax])
 #pragma unroll 1
-                for (int t = t0; (long)t * g.tile < g.lines; t += lp.slots[ax]) {
+                for (int t = t0; (long)t * g.tile < g.lines; t += GROUPS * lp.slots[ax]) {
                     if (g.nb == 4)
-                        tc_tile<P, 4, 512, true>(g, src, dst, bz, first, last, t, part, smem, lp.op_at[ax], lp.tile_at,
+                        tc_tile<P, 4, 512 / GROUPS, true>(g, src, dst, bz, first, last, t, part, smem, lp.op_at[ax], tile_at,
                                                  sbase + SM_BAR + 8 * ax, s == a.s && t == t0, ph);
                     else
-                        tc_tile<P, 2, 512, true>(g, src, dst, bz, first, last, t, part, smem, lp.op_at[ax], lp.tile_at,
+                        tc_tile<P, 2, 512 / GROUPS, true>(g, src, dst, bz, first, last, t, part, smem, lp.op_at[ax], tile_at,
                                                  sbase + SM_BAR + 8 * ax, s == a.s && t == t0, ph);
                 }
             /* this axis' slice is complete before the next one reads it */
             asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
         }
     }
-    if (!ph.ok && threadIdx.x == 0) atomicExch(&g_scft_pass_fault, 1);
+    if (!ph.ok && threadIdx.x % (512 / GROUPS) == 0) atomicExch(&g_scft_pass_fault, 1);
 }
 
 /* The same loop on a 2D grid with one tile per CTA and axis, whose lines never
@@ -1060,14 +1085,14 @@ __global__ void __launch_bounds__(512, 1) k_chain2d_tc(const __grid_constant__ T
 /* ------------------------------------------------------------- launchers */
 size_t scft_pass_tc_smem(int prec, const TcGeom &g)
 {
-    return SM_OP + g.op_part + (prec == SCFT_PREC_FP32 ? tile_bytes(g, Dig<float>::S)
-                                                      : tile_bytes(g, Dig<double>::S));
+    return SM_OP + g.op_part + (prec == SCFT_PREC_FP32 ? tile_bytes(g, Dig<float>::S, 16)
+                                                      : tile_bytes(g, Dig<double>::S, 16));
 }
 
 template <typename P>
 static cudaError_t launch_tc(const TcGeom &g, const PassArgs &a, cudaStream_t st)
 {
-    const size_t smem = SM_OP + g.op_part + tile_bytes(g, Dig<P>::S);
+    const size_t smem = SM_OP + g.op_part + tile_bytes(g, Dig<P>::S, 16);
     const dim3 grid((unsigned)((g.lines + g.tile - 1) / g.tile * g.parts), a.nchains);
     if (g.tile < 8 || g.tile % 8 || g.tile > ROWS) return cudaErrorInvalidValue;
     if (g.nb == 4)
@@ -1098,8 +1123,7 @@ size_t scft_chain_tc_layout(int prec, TcLoop &lp)
         lp.op_at[ax] = at;
         at += (lp.g[ax].op_part + 127) / 128 * 128;
         const int S = prec == SCFT_PREC_FP32 ? Dig<float>::S : Dig<double>::S, value = prec == SCFT_PREC_FP32 ? 4 : 8;
-        const uint32_t b = lp.exchange ? tile_bytes(lp.g[ax], S, 8) + exchange2d_bytes(lp.g[ax], value)
-                                       : tile_bytes(lp.g[ax], S) + exchange_bytes(lp.g[ax], value);
+        const uint32_t b = tile_bytes(lp.g[ax], S, 8) + exchange_bytes(lp.g[ax], value);
         if (b > tile) tile = b;
         lp.slots[ax] = lp.cluster / lp.g[ax].parts;
         if (lp.exchange) { /* lines, shifted by half the banks from one to the next */
@@ -1110,7 +1134,8 @@ size_t scft_chain_tc_layout(int prec, TcLoop &lp)
         }
     }
     lp.tile_at = at;
-    return (size_t)at + tile;
+    lp.tile_bytes = (tile + 127) / 128 * 128;
+    return (size_t)at + (lp.exchange ? 1 : GROUPS) * lp.tile_bytes;
 }
 
 template <typename P>
