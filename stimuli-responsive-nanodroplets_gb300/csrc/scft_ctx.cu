@@ -137,7 +137,8 @@ struct scft_ctx {
     int hist_cap = 0;
     int pending = 0; /* iterations enqueued and not yet collected */
     cudaEvent_t chunk_done = nullptr; /* recorded after the records copy of the enqueued chunk */
-    int nparts = 0;
+    UpdateTable *table = nullptr;
+    int nparts = 0, qparts = 0;
     size_t device_bytes = 0;
     std::vector<void *> allocs;
     /* host mirrors */
@@ -1584,7 +1585,9 @@ extern "C" int scft_ctx_create(const scft_surface *surfaces, const scft_options 
     ALLOC(c->mask, sizeof(double) * B * 3 * sm);
     ALLOC(c->bz, (size_t)c->psize * B * SCFT_NFIELDS * sm);
     c->nparts = scft_post_nparts(c->m, c->sms);
-    ALLOC(c->partial, sizeof(double) * B * SCFT_NSPECIES * c->nparts);
+    c->qparts = scft_post_qparts(c->m, opt.precision, c->sms);
+    ALLOC(c->partial, sizeof(double) * B * (SCFT_NSPECIES * c->qparts + 3 * c->nparts));
+    ALLOC(c->table, sizeof(UpdateTable) * B);
     ALLOC(c->noise, sizeof(double) * B * d.n_active * sm);
     c->hist_cap = SCFT_HIST_CAP;
     ALLOC(c->hist, sizeof(scft_iter_out) * c->hist_cap * B);
@@ -1697,7 +1700,7 @@ extern "C" int scft_ctx_create(const scft_surface *surfaces, const scft_options 
     c->rng.assign(3 * B, 0);
     c->fields_set.assign(B, 0);
     c->prop_launches_per_iter = (c->fused2d || c->fused3d || c->loop_tc) ? 1L : (long)(c->maxlen - 1) * (long)c->axes.size();
-    c->launches_per_iter = c->prop_launches_per_iter + 2 + 6 + (opt.noise_mode == SCFT_NOISE_DRAND48 ? 5 : 0);
+    c->launches_per_iter = c->prop_launches_per_iter + 2 + 3 + (opt.noise_mode == SCFT_NOISE_DRAND48 ? 5 : 0);
     if (cudaStreamSynchronize(c->stream) != cudaSuccess) {
         set_err("context set-up failed: %s", cudaGetErrorString(cudaGetLastError()));
         scft_ctx_destroy(c);
@@ -1930,6 +1933,11 @@ static PostArgs post_args(scft_ctx *c, const double *noise_dev)
     a.bz = c->bz;
     a.field_use = c->field_use;
     a.partial = c->partial;
+    a.upd_partial = c->partial + (size_t)c->B * SCFT_NSPECIES * c->qparts;
+    a.table = c->table;
+    a.qparts = c->qparts;
+    for (int sp = 0; sp < SCFT_NSPECIES; ++sp)
+        if (c->species_h[sp].present) a.q_species[a.nq_species++] = sp;
     a.nparts = c->nparts;
     a.noise = noise_dev;
     a.hist = c->hist;

@@ -175,6 +175,15 @@ cudaError_t scft_launch_chain_tc(int prec, const TcLoop &lp, const Step2DArgs &a
 int scft_pass_tc_take_fault(void);
 
 /* Arguments shared by the non-propagator kernels (scft_post.cu). */
+/* What the update of an instance needs besides its fields, and the arrival counters of the
+ * launches whose last CTA finishes an instance (zero between launches). */
+struct UpdateTable {
+    double coef[SCFT_MAX_BLOCKS];
+    double chi[SCFT_NFIELDS][SCFT_NFIELDS], pavg[SCFT_NFIELDS], c[SCFT_NFIELDS], e[SCFT_NFIELDS], ctot;
+    int f[SCFT_NFIELDS]; /* active fields */
+    unsigned q_arrived, u_arrived;
+};
+
 struct PostArgs {
     const InstParams *params;   /* [B] */
     InstState *state;           /* [B] */
@@ -192,8 +201,11 @@ struct PostArgs {
     const double *mask;         /* [B][3][sm] */
     void *bz;                   /* [B][13][sm] P */
     unsigned field_use;         /* bit f: some chain propagates with field f */
-    double *partial;            /* [B][nparts][...] */
-    int nparts;
+    double *partial;            /* [B][17][qparts]: partial sums of Q */
+    UpdateTable *table;         /* [B] */
+    double *upd_partial;        /* [B][nparts][3]: of H, p and (phi_tot - 1)^2 */
+    int nparts, qparts;
+    int q_species[SCFT_NSPECIES], nq_species; /* the species present */
     const double *noise;        /* [B][n_active][sm] or NULL */
     scft_iter_out *hist;        /* [cap][B] */
     scft_iter_out *last;        /* [B]: the latest record (repeated while frozen) */
@@ -211,6 +223,7 @@ cudaError_t scft_post_iter_end(const PostArgs &a, int prec, int sms, cudaStream_
 /* k_density alone (the unit entry point scft_density) */
 cudaError_t scft_density_launch(const PostArgs &a, int prec, int sms, cudaStream_t st);
 int scft_post_nparts(long m, int sms);
+int scft_post_qparts(long m, int prec, int sms);
 cudaError_t scft_convert(int prec, const double *src, void *dst, long n, int to_p, cudaStream_t st);
 cudaError_t scft_boltz_one(int prec, const double *w, void *bz, double ds, long m, cudaStream_t st);
 

@@ -14,7 +14,8 @@
 #include "scft_internal.h"
 
 #define POST_THREADS 256
-
+#define DENSITY_THREADS 64
+#define UPDATE_THREADS 128
 
 
 __device__ __forceinline__ double warp_sum(double v)
@@ -82,72 +83,122 @@ __device__ __forceinline__ P boltz(double ds, double w)
         return P(exp(arg)); /* FP64, or the FP32 pair nearest the FP64 value */
 }
 
-/* b for the fields chains use, and the initial slice of every chain: 1, the
- * grafting mask (SCFT.c:2441) or the single-point seed while iIter <=
- * SEED_STEPS (SCFT.c:2346-2367). */
+/* b for the fields chains use, and the initial slice of every chain: 1, the grafting
+ * mask (SCFT.c:2441) or the single-point seed while iIter <= SEED_STEPS
+ * (SCFT.c:2346-2367). Where the grid leaves SMs idle, one field or the initial slices
+ * per blockIdx.z, so that a thread waits for one exponential and not for all in turn
+ * (one 32x16 film, 2 CTAs: 11.9 -> 6.0 us; 256 films of 192x96, 18432 CTAs: 128 us
+ * with all in one thread, 241 us apart). */
 template <typename P>
 __global__ void k_boltz_init(PostArgs a)
 {
     const int b = blockIdx.y;
     if (a.state[b].done) return;
     const InstParams &ip = a.params[b];
-    const unsigned long iter = a.state[b].iter;
-    const bool seed_on = ip.enable_seed && iter <= (unsigned long)ip.seed_steps;
-    P *bz = reinterpret_cast<P *>(a.bz) + (long)b * SCFT_NFIELDS * a.sm;
-    const double *w = a.w + (long)b * 14 * a.sm;
-    for (long idx = blockIdx.x * (long)blockDim.x + threadIdx.x; idx < a.m; idx += (long)gridDim.x * blockDim.x) {
-        for (int f = 0; f < SCFT_NFIELDS; ++f)
-            if (a.field_use >> f & 1u) bz[f * a.sm + idx] = boltz<P>(ip.ds, w[f * a.sm + idx]);
-        const int k = (int)(idx % a.nz);
-        const int j = (int)((idx / a.nz) % a.ny);
-        const int i = (int)(idx / ((long)a.nz * a.ny));
-        for (int c = 0; c < a.nchains; ++c) {
-            const ChainDesc &cd = a.chains[b * a.nchains + c];
+    const long first = blockIdx.x * (long)blockDim.x + threadIdx.x, step = (long)gridDim.x * blockDim.x;
+    const bool apart = gridDim.z > 1;
+    unsigned z = 0;
+    for (unsigned use = a.field_use; use; use &= use - 1, ++z) {
+        if (apart && z != blockIdx.z) continue;
+        const int f = __ffs(use) - 1;
+        P *bz = reinterpret_cast<P *>(a.bz) + ((long)b * SCFT_NFIELDS + f) * a.sm;
+        const double *w = a.w + ((long)b * 14 + f) * a.sm;
+        for (long idx = first; idx < a.m; idx += step) bz[idx] = boltz<P>(ip.ds, w[idx]);
+    }
+    if (apart && blockIdx.z + 1 < gridDim.z) return;
+    const bool seed_on = ip.enable_seed && a.state[b].iter <= (unsigned long)ip.seed_steps;
+    for (int c = 0; c < a.nchains; ++c) {
+        const ChainDesc &cd = a.chains[b * a.nchains + c];
+        P *q = reinterpret_cast<P *>(cd.q);
+        for (long idx = first; idx < a.m; idx += step) {
             P v = (P)1;
             if (cd.init == SCFT_INIT_MASK) {
                 v = (P)a.mask[((long)b * 3 + cd.init_arg) * a.sm + idx];
             } else if (cd.init == SCFT_INIT_SEED && seed_on) {
+                const int k = (int)(idx % a.nz);
+                const int j = (int)((idx / a.nz) % a.ny);
+                const int i = (int)(idx / ((long)a.nz * a.ny));
                 const int D = ip.seed_area_delta;
                 const bool in = i > (a.nx / 2 - D) && i < (a.nx / 2 + D) && j > (a.ny / 2 - D) && j < (a.ny / 2 + D) &&
                                 k > (a.nz / 4 - D) && k < (a.nz / 4 + D);
                 v = in ? (P)1 : (P)0;
             }
-            reinterpret_cast<P *>(cd.q)[idx] = v;
+            q[idx] = v;
         }
     }
 }
 
 /* ------------------------------------------------------------------ Q */
-/* Partial sums of q(r, NS_EFF-1) per species (funChemPotential, SCFT.c:1837-1859). */
-template <typename P>
-__global__ void __launch_bounds__(POST_THREADS) k_q_partial(PostArgs a)
+/* Whether this CTA is the last of `total` to arrive at the counter, which then
+ * starts over. What the others wrote before is visible to all its threads. */
+__device__ __forceinline__ bool last_cta(unsigned *counter, unsigned total)
 {
-    __shared__ double sh[32];
-    const int sp = blockIdx.y, b = blockIdx.z;
-    const SpeciesDesc sd = a.species[b * SCFT_NSPECIES + sp];
-    if (!sd.present || a.state[b].done) return;
-    const ChainDesc &cd = a.chains[b * a.nchains + sd.q_chain];
-    const P *q = reinterpret_cast<const P *>(cd.q) + (long)(sd.len - 1) * a.sm;
-    double v[1] = {0.0};
-    for (long idx = blockIdx.x * (long)blockDim.x + threadIdx.x; idx < a.m; idx += (long)gridDim.x * blockDim.x)
-        v[0] += (double)q[idx];
-    block_sum<1>(v, sh);
-    if (threadIdx.x == 0) a.partial[((long)b * SCFT_NSPECIES + sp) * gridDim.x + blockIdx.x] = v[0];
+    __shared__ int s_last;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        s_last = atomicInc(counter, total - 1) == total - 1;
+        __threadfence();
+    }
+    __syncthreads();
+    return s_last != 0;
 }
 
-__global__ void k_q_final(PostArgs a, int nparts)
+/* One instance's Q of every species, by a warp each, and what the update needs of
+ * them and of the parameters: once, and not in every CTA of the update. */
+__device__ __noinline__ void prepare_update(const PostArgs &a, int b)
 {
-    const int sp = blockIdx.x, b = blockIdx.y;
-    if (threadIdx.x != 0 || a.state[b].done) return;
-    const SpeciesDesc sd = a.species[b * SCFT_NSPECIES + sp];
-    double q = 0.0;
-    if (sd.present) {
-        const double *p = a.partial + ((long)b * SCFT_NSPECIES + sp) * nparts;
+    InstState &st = a.state[b];
+    const InstParams &ip = a.params[b];
+    UpdateTable &u = a.table[b];
+    const int lane = threadIdx.x & 31, warps = blockDim.x / 32;
+    __shared__ double s_q[SCFT_NSPECIES];
+    __shared__ int s_act[SCFT_NFIELDS];
+    for (int sp = threadIdx.x; sp < SCFT_NSPECIES; sp += blockDim.x) s_q[sp] = 0.0;
+    __syncthreads();
+    for (int k = threadIdx.x / 32; k < a.nq_species; k += warps) {
+        const int sp = a.q_species[k];
+        const double *p = a.partial + ((long)b * SCFT_NSPECIES + sp) * a.qparts;
         double s = 0.0;
-        for (int k = 0; k < nparts; ++k) s += p[k];
-        q = s / (double)a.m; /* qrsum / dVol, SCFT.c:1861 */
+        for (int i = lane; i < a.qparts; i += 32) s += __ldcg(p + i);
+        s = warp_sum(s);
+        if (lane == 0) s_q[sp] = s / (double)a.m; /* qrsum / dVol, SCFT.c:1861 */
     }
-    a.state[b].q[sp] = q;
+    if (threadIdx.x < 32) {
+        const bool on = lane < SCFT_NFIELDS && ip.active[lane];
+        const unsigned act = __ballot_sync(0xffffffffu, on);
+        if (on) s_act[__popc(act & ((1u << lane) - 1))] = lane;
+    }
+    __syncthreads();
+    for (int sp = threadIdx.x; sp < SCFT_NSPECIES; sp += blockDim.x) st.q[sp] = s_q[sp];
+    for (int k = threadIdx.x; k < a.nblocks; k += blockDim.x) {
+        const BlockDesc bd = a.blocks[b * a.nblocks + k];
+        const double ds_eff = 1.0 / (bd.len - 1);
+        /* frac * ((raw / 3) * (DS_EFF / Q)) as one factor */
+        u.coef[k] = ip.frac[k] * ((ds_eff / s_q[bd.species]) / 3.0);
+    }
+    const int na = a.n_active;
+    for (int i = threadIdx.x; i < na; i += blockDim.x) {
+        double c = 0.0, e = 0.0;
+        for (int j = 0; j < na; ++j) {
+            const double x = ip.chi[s_act[i]][s_act[j]];
+            u.chi[i][j] = x;
+            if (j != i) {
+                c += x;
+                e += x * ip.phi_avg[s_act[j]];
+            }
+        }
+        u.pavg[i] = ip.phi_avg[s_act[i]];
+        u.c[i] = c;
+        u.e[i] = e;
+        u.f[i] = s_act[i];
+    }
+    if (threadIdx.x == blockDim.x - 1) {
+        double c = 0.0;
+        for (int i = 0; i < na; ++i)
+            for (int j = i + 1; j < na; ++j) c += ip.chi[s_act[i]][s_act[j]];
+        u.ctot = c;
+    }
 }
 
 /* ------------------------------------------------------------- density */
@@ -228,13 +279,49 @@ __device__ __forceinline__ void load_p(const P *p, P (&o)[V])
     }
 }
 
+/* Rows behind the blocks: partial sums of q(r, NS_EFF-1) of the species present
+ * (funChemPotential, SCFT.c:1837-1859), one row each, by the first a.qparts CTAs; the
+ * last of an instance's finishes Q. */
+template <typename P, int V>
+__device__ __forceinline__ void q_partial(const PostArgs &a, int b, int sp)
+{
+    __shared__ double sh[32];
+    const SpeciesDesc sd = a.species[b * SCFT_NSPECIES + sp];
+    const P *q = reinterpret_cast<const P *>(a.chains[b * a.nchains + sd.q_chain].q) + (long)(sd.len - 1) * a.sm;
+    double v[1] = {0.0};
+    for (long iv = blockIdx.x * (long)blockDim.x + threadIdx.x; iv < (a.m + V - 1) / V; iv += (long)a.qparts * blockDim.x) {
+        const long idx = iv * V;
+        if (idx + V <= a.m) {
+            P x[V];
+            load_p<P, V>(q + idx, x);
+#pragma unroll
+            for (int k = 0; k < V; ++k) v[0] += (double)x[k];
+        } else {
+            for (long i = idx; i < a.m; ++i) v[0] += (double)q[i];
+        }
+    }
+    block_sum<1>(v, sh);
+    if (threadIdx.x == 0) a.partial[((long)b * SCFT_NSPECIES + sp) * a.qparts + blockIdx.x] = v[0];
+    if (last_cta(&a.table[b].q_arrived, (unsigned)(a.qparts * a.nq_species))) prepare_update(a, b);
+}
+
+/* CTAs of 64 threads: a small grid's FP64 sums spread over four times as many SMs.
+ * Both contour loops run together, for more slices in flight per thread; the rows of
+ * Q take no launch of their own. 256 films of 192x96 in FP32, bounded by the slices
+ * read from HBM: densities and Q 1794 -> 1768 us (in launches for all 17 species, Q
+ * took 275 of them); one 32x16 film, bounded by latency and launches: with the update
+ * below, 341 -> 307 us an iteration. */
 template <typename P>
-__global__ void __launch_bounds__(POST_THREADS) k_density(PostArgs a)
+__global__ void __launch_bounds__(DENSITY_THREADS) k_density(PostArgs a)
 {
     constexpr int V = sizeof(P) == 4 ? 4 : 2;
     using Acc = typename AccOf<P>::T;
     const int blk = blockIdx.y, b = blockIdx.z;
     if (a.state[b].done) return;
+    if (blk >= a.nblocks) {
+        if (blockIdx.x < a.qparts) q_partial<P, V>(a, b, a.q_species[blk - a.nblocks]);
+        return;
+    }
     const BlockDesc bd = a.blocks[b * a.nblocks + blk];
     const P *qf = reinterpret_cast<const P *>(a.chains[b * a.nchains + bd.chain_f].q);
     const P *qb = reinterpret_cast<const P *>(a.chains[b * a.nchains + bd.chain_b].q);
@@ -263,19 +350,25 @@ __global__ void __launch_bounds__(POST_THREADS) k_density(PostArgs a)
             load_p<P, V>(qf + (long)top * a.sm + idx, y);
 #pragma unroll
             for (int v = 0; v < V; ++v) e2[v].add(x[v], y[v]);
+            int s = 1;
 #pragma unroll 4
-            for (int s = 1; s < mid; s += 2) {
+            for (; s + 1 < mid; s += 2) {
+                P x2[V], y2[V];
+                load_p<P, V>(qf + (long)s * a.sm + idx, x);
+                load_p<P, V>(qf + (long)(top - s) * a.sm + idx, y);
+                load_p<P, V>(qf + (long)(s + 1) * a.sm + idx, x2);
+                load_p<P, V>(qf + (long)(top - s - 1) * a.sm + idx, y2);
+#pragma unroll
+                for (int v = 0; v < V; ++v) {
+                    h4[v].add(x[v], y[v]);
+                    h2[v].add(x2[v], y2[v]);
+                }
+            }
+            if (s < mid) {
                 load_p<P, V>(qf + (long)s * a.sm + idx, x);
                 load_p<P, V>(qf + (long)(top - s) * a.sm + idx, y);
 #pragma unroll
                 for (int v = 0; v < V; ++v) h4[v].add(x[v], y[v]);
-            }
-#pragma unroll 4
-            for (int s = 2; s < mid; s += 2) {
-                load_p<P, V>(qf + (long)s * a.sm + idx, x);
-                load_p<P, V>(qf + (long)(top - s) * a.sm + idx, y);
-#pragma unroll
-                for (int v = 0; v < V; ++v) h2[v].add(x[v], y[v]);
             }
             if (mid > 0) {
                 load_p<P, V>(qf + (long)mid * a.sm + idx, x);
@@ -303,19 +396,25 @@ __global__ void __launch_bounds__(POST_THREADS) k_density(PostArgs a)
             load_p<P, V>(qb + (long)(top - bd.stop) * a.sm + idx, y);
 #pragma unroll
             for (int v = 0; v < V; ++v) ends[v].add(x[v], y[v]);
+            int s = bd.start + 1;
 #pragma unroll 4
-            for (int s = bd.start + 1; s <= bd.stop - 1; s += 2) {
+            for (; s + 1 <= bd.stop - 2; s += 2) {
+                P x2[V], y2[V];
+                load_p<P, V>(qf + (long)s * a.sm + idx, x);
+                load_p<P, V>(qb + (long)(top - s) * a.sm + idx, y);
+                load_p<P, V>(qf + (long)(s + 1) * a.sm + idx, x2);
+                load_p<P, V>(qb + (long)(top - s - 1) * a.sm + idx, y2);
+#pragma unroll
+                for (int v = 0; v < V; ++v) {
+                    a4[v].add(x[v], y[v]);
+                    a2[v].add(x2[v], y2[v]);
+                }
+            }
+            if (s <= bd.stop - 1) {
                 load_p<P, V>(qf + (long)s * a.sm + idx, x);
                 load_p<P, V>(qb + (long)(top - s) * a.sm + idx, y);
 #pragma unroll
                 for (int v = 0; v < V; ++v) a4[v].add(x[v], y[v]);
-            }
-#pragma unroll 4
-            for (int s = bd.start + 2; s <= bd.stop - 2; s += 2) {
-                load_p<P, V>(qf + (long)s * a.sm + idx, x);
-                load_p<P, V>(qb + (long)(top - s) * a.sm + idx, y);
-#pragma unroll
-                for (int v = 0; v < V; ++v) a2[v].add(x[v], y[v]);
             }
 #pragma unroll
             for (int v = 0; v < V; ++v) out[idx + v] = ends[v].value() + 4.0 * a4[v].value() + 2.0 * a2[v].value();
@@ -337,6 +436,75 @@ __global__ void __launch_bounds__(POST_THREADS) k_density(PostArgs a)
     }
 }
 
+/* Reduce the update partials of one instance, finish H (ln Q terms,
+ * SCFT.c:1528-1555), mu (SCFT.c:1862-1869), RMS and <p>; write the record. A lane
+ * for each logarithm: with all in one thread 12 of 15 us. */
+__device__ __noinline__ void finish_iteration(const PostArgs &a, int b, int nparts, double *sh)
+{
+    __shared__ double s_q[SCFT_NSPECIES], s_lnq[SCFT_NSPECIES], s_mu[SCFT_NSPECIES];
+    InstState &st = a.state[b];
+    const InstParams &ip = a.params[b];
+    const long slot = (long)st.tick - 1;
+    double v[3] = {0.0, 0.0, 0.0};
+    /* fixed assignment of partials to threads keeps the order deterministic */
+    for (int k = threadIdx.x; k < nparts; k += blockDim.x) {
+        const double *pp = a.upd_partial + ((long)b * nparts + k) * 3;
+        v[0] += __ldcg(pp);
+        v[1] += __ldcg(pp + 1);
+        v[2] += __ldcg(pp + 2);
+    }
+    if (threadIdx.x >= 32 && threadIdx.x < 32 + 2 * SCFT_NSPECIES) {
+        const int t = threadIdx.x - 32, sp = t >> 1;
+        const double q = st.q[sp], qm = q * q;
+        const int present = a.species[b * SCFT_NSPECIES + sp].present;
+        if (t & 1) {
+            s_lnq[sp] = present ? ip.lnq_coef[sp] * log(q) : 0.0;
+            s_q[sp] = q;
+        } else {
+            s_mu[sp] = !present || qm == 0.0 ? 0.0 : -log(qm) / 2.0;
+        }
+    }
+    block_sum<3>(v, sh);
+    if (threadIdx.x != 0) return;
+    const double dvol = (double)a.m;
+    double H = v[0] / dvol;
+    double frac = 0.0;
+    int bad = 0;
+    scft_iter_out rec;
+    for (int sp = 0; sp < SCFT_NSPECIES; ++sp) {
+        rec.q[sp] = s_q[sp];
+        rec.mu[sp] = s_mu[sp];
+    }
+    for (int k = 0; k < a.nq_species; ++k) {
+        const int sp = a.q_species[k];
+        frac += s_lnq[sp];
+        if (!isfinite(s_q[sp])) bad = 1;
+    }
+    H -= frac;
+    const double pavg = v[1] / dvol;
+    const double rms = sqrt(v[2] / dvol);
+    if (!isfinite(H) || !isfinite(rms) || !isfinite(pavg)) bad = 1;
+    st.p_avg = pavg;
+    if (bad) st.status = SCFT_ERR_NONFINITE; /* keeps an error set earlier in the iteration */
+    rec.iter = st.iter;
+    rec.free_energy = H;
+    rec.rms = rms;
+    rec.mf = (st.iter > (unsigned long)ip.relaxation) ? 0.0 : 1.0;
+    rec.status = st.status;
+    rec.converged = 0;
+    if (st.stop_rms > 0.0 && st.status == SCFT_OK && rms < st.stop_rms) {
+        st.done = 2; /* frozen from the next iteration on; this one still ends with the p shift */
+        rec.converged = 1;
+    }
+    /* with a stop criterion (batch and serving forms) a non-finite instance is
+     * frozen too: its records repeat the failing iteration and it costs nothing
+     * until its slot is re-armed; without one (the fixed-ITER drop-in) it keeps
+     * iterating as the reference does */
+    if (st.stop_rms > 0.0 && st.status != SCFT_OK) st.done = 2;
+    a.last[b] = rec;
+    if (slot >= 0 && slot < a.hist_cap) a.hist[slot * a.B + b] = rec;
+}
+
 /* -------------------------------------------------------- fused update */
 /* Per grid point: block densities (funDensity normalisation SCFT.c:2299 and
  * funVolFrac SCFT.c:1458-1482), totals (funAddArray SCFT.c:1486-1512), the free
@@ -349,69 +517,44 @@ __global__ void __launch_bounds__(POST_THREADS) k_density(PostArgs a)
  * factors sit in shared memory; per-point values stay in registers because all
  * register-array indices are loop counters of fully unrolled loops.
  * Block partials of H, p and (phi_tot-1)^2 go to a.partial. The pass is bound
- * by the FP64 pipe's latency, so it is built for three CTAs per SM with up to
- * four active fields and two otherwise (a few registers spill; measured faster
- * than one or two CTAs without spills). */
+ * by the FP64 pipe's latency, so it is built for 768 threads per SM with up to
+ * four active fields and 512 otherwise (a few registers spill; measured faster
+ * than fewer threads without spills), in CTAs of 128, so that one grid's points
+ * spread over twice the SMs. The last CTA of an instance ends the iteration: it
+ * has the partials in L2 and needs no launch of its own. */
 template <int NA>
-__global__ void __launch_bounds__(POST_THREADS, (NA <= 4 ? 3 : 2)) k_update(PostArgs a)
+__global__ void __launch_bounds__(UPDATE_THREADS, (NA <= 4 ? 6 : 4)) k_update(PostArgs a)
 {
     __shared__ double sh[3 * 32];
     __shared__ double coef[SCFT_MAX_BLOCKS];
-    __shared__ double chiA[SCFT_NFIELDS][SCFT_NFIELDS];
-    __shared__ double pavgA[SCFT_NFIELDS];
-    __shared__ double cA[SCFT_NFIELDS], eA[SCFT_NFIELDS]; /* row sums of chi, of chi . phi_avg */
-    __shared__ double s_ctot;                             /* sum over pairs of chi */
-    __shared__ int actf[SCFT_NFIELDS], p0[SCFT_NFIELDS], p1[SCFT_NFIELDS];
-    __shared__ int s_na;
+    __shared__ double chiA[NA][NA];
+    __shared__ double pavgA[NA], cA[NA], eA[NA]; /* row sums of chi, of chi . phi_avg */
+    __shared__ int actf[NA], p0[NA], p1[NA];
     const int b = blockIdx.y;
-    if (a.state[b].done) return;
+    if (a.state[b].done) {
+        /* frozen: repeat the converging iteration's record */
+        const long slot = (long)a.state[b].tick - 1;
+        if (blockIdx.x == 0 && threadIdx.x == 0 && slot >= 0 && slot < a.hist_cap) a.hist[slot * a.B + b] = a.last[b];
+        return;
+    }
     const InstParams &ip = a.params[b];
     const InstState &st = a.state[b];
+    const UpdateTable &ut = a.table[b];
     const double mf = (st.iter > (unsigned long)ip.relaxation) ? 0.0 : 1.0; /* SCFT.c:1515-1522 */
-    if (threadIdx.x < a.nblocks) {
-        const BlockDesc bd = a.blocks[b * a.nblocks + threadIdx.x];
-        const double ds_eff = 1.0 / (bd.len - 1);
-        /* frac * ((raw / 3) * (DS_EFF / Q)) as one factor: the FP64 divisions
-         * would otherwise dominate this kernel's FP64 pipe time */
-        coef[threadIdx.x] = ip.frac[threadIdx.x] * ((ds_eff / st.q[bd.species]) / 3.0);
-    }
-    if (threadIdx.x == 0) {
-        int n = 0;
-        for (int f = 0; f < SCFT_NFIELDS; ++f)
-            if (ip.active[f]) {
-                actf[n] = f;
-                p0[n] = a.part0[f];
-                p1[n] = a.part1[f];
-                pavgA[n] = ip.phi_avg[f];
-                ++n;
-            }
-        s_na = n;
-    }
-    __syncthreads();
     /* every instance of a context has NA active fields (checked at creation) */
     constexpr int na = NA;
-    for (int e = threadIdx.x; e < na * na; e += blockDim.x) {
-        const int i = e / na, j = e - i * na;
-        chiA[i][j] = ip.chi[actf[i]][actf[j]];
+    for (int e = threadIdx.x; e < na * na; e += UPDATE_THREADS) chiA[e / na][e % na] = ut.chi[e / na][e % na];
+    if (threadIdx.x < a.nblocks) coef[threadIdx.x] = ut.coef[threadIdx.x];
+    if (threadIdx.x >= 32 && threadIdx.x < 32 + na) {
+        const int i = threadIdx.x - 32, f = ut.f[i];
+        actf[i] = f;
+        p0[i] = a.part0[f];
+        p1[i] = a.part1[f];
+        pavgA[i] = ut.pavg[i];
+        cA[i] = ut.c[i];
+        eA[i] = ut.e[i];
     }
-    __syncthreads();
-    if (threadIdx.x < na) {
-        const int i = threadIdx.x;
-        double c = 0.0, e = 0.0;
-        for (int j = 0; j < na; ++j)
-            if (j != i) {
-                c += chiA[i][j];
-                e += chiA[i][j] * pavgA[j];
-            }
-        cA[i] = c;
-        eA[i] = e;
-    }
-    if (threadIdx.x == 0) {
-        double c = 0.0;
-        for (int i = 0; i < na; ++i)
-            for (int j = i + 1; j < na; ++j) c += chiA[i][j];
-        s_ctot = c;
-    }
+    const double s_ctot = ut.ctot; /* sum over pairs of chi */
     __syncthreads();
     const double g1 = ip.g1, g2 = ip.g2, g12 = g1 - g2, dt = ip.dt_noise;
     const double inv_na = 1.0 / na;
@@ -495,75 +638,12 @@ __global__ void __launch_bounds__(POST_THREADS, (NA <= 4 ? 3 : 2)) k_update(Post
     }
     block_sum<3>(acc, sh);
     if (threadIdx.x == 0) {
-        double *pp = a.partial + ((long)b * gridDim.x + blockIdx.x) * 3;
+        double *pp = a.upd_partial + ((long)b * gridDim.x + blockIdx.x) * 3;
         pp[0] = acc[0];
         pp[1] = acc[1];
         pp[2] = acc[2];
     }
-}
-
-/* Reduce the update partials of one instance, finish H (ln Q terms,
- * SCFT.c:1528-1555), mu (SCFT.c:1862-1869), RMS and <p>; write the record. */
-__global__ void k_finalize(PostArgs a, int nparts)
-{
-    const int b = blockIdx.x;
-    __shared__ double sh[3 * 32];
-    InstState &st = a.state[b];
-    const long slot = (long)st.tick - 1;
-    if (st.done) {
-        /* frozen: repeat the converging iteration's record */
-        if (threadIdx.x == 0 && slot >= 0 && slot < a.hist_cap) a.hist[slot * a.B + b] = a.last[b];
-        return;
-    }
-    double v[3] = {0.0, 0.0, 0.0};
-    /* fixed assignment of partials to threads keeps the order deterministic */
-    for (int k = threadIdx.x; k < nparts; k += blockDim.x) {
-        const double *pp = a.partial + ((long)b * nparts + k) * 3;
-        v[0] += pp[0];
-        v[1] += pp[1];
-        v[2] += pp[2];
-    }
-    block_sum<3>(v, sh);
-    if (threadIdx.x != 0) return;
-    const InstParams &ip = a.params[b];
-    const double dvol = (double)a.m;
-    double H = v[0] / dvol;
-    double frac = 0.0;
-    int bad = 0;
-    scft_iter_out rec;
-    for (int sp = 0; sp < SCFT_NSPECIES; ++sp) {
-        const double q = st.q[sp];
-        rec.q[sp] = q;
-        rec.mu[sp] = 0.0;
-        if (!a.species[b * SCFT_NSPECIES + sp].present) continue;
-        const double qm = q * q;
-        rec.mu[sp] = (qm == 0.0) ? 0.0 : -log(qm) / 2.0;
-        frac += ip.lnq_coef[sp] * log(q);
-        if (!isfinite(q)) bad = 1;
-    }
-    H -= frac;
-    const double pavg = v[1] / dvol;
-    const double rms = sqrt(v[2] / dvol);
-    if (!isfinite(H) || !isfinite(rms) || !isfinite(pavg)) bad = 1;
-    st.p_avg = pavg;
-    if (bad) st.status = SCFT_ERR_NONFINITE; /* keeps an error set earlier in the iteration */
-    rec.iter = st.iter;
-    rec.free_energy = H;
-    rec.rms = rms;
-    rec.mf = (st.iter > (unsigned long)ip.relaxation) ? 0.0 : 1.0;
-    rec.status = st.status;
-    rec.converged = 0;
-    if (st.stop_rms > 0.0 && st.status == SCFT_OK && rms < st.stop_rms) {
-        st.done = 2; /* frozen from the next iteration on; this one still ends with the p shift */
-        rec.converged = 1;
-    }
-    /* with a stop criterion (batch and serving forms) a non-finite instance is
-     * frozen too: its records repeat the failing iteration and it costs nothing
-     * until its slot is re-armed; without one (the fixed-ITER drop-in) it keeps
-     * iterating as the reference does */
-    if (st.stop_rms > 0.0 && st.status != SCFT_OK) st.done = 2;
-    a.last[b] = rec;
-    if (slot >= 0 && slot < a.hist_cap) a.hist[slot * a.B + b] = rec;
+    if (last_cta(&a.table[b].u_arrived, gridDim.x)) finish_iteration(a, b, gridDim.x, sh);
 }
 
 /* p -= <p> (SCFT.c:2119-2123). */
@@ -578,10 +658,9 @@ __global__ void k_p_shift(PostArgs a)
 }
 
 /* ------------------------------------------------------------ launchers */
-static int grid_for(long m, int sms)
+static int grid_for(long m, int threads, int cap)
 {
-    long g = (m + POST_THREADS - 1) / POST_THREADS;
-    long cap = (long)sms * 4;
+    long g = (m + threads - 1) / threads;
     if (g > cap) g = cap;
     return (int)(g < 1 ? 1 : g);
 }
@@ -589,7 +668,10 @@ static int grid_for(long m, int sms)
 cudaError_t scft_post_iter_begin(const PostArgs &a, int prec, int sms, cudaStream_t st)
 {
     k_iter_begin<<<(a.B + 127) / 128, 128, 0, st>>>(a);
-    dim3 g(grid_for(a.m, sms), a.B);
+    dim3 g(grid_for(a.m, POST_THREADS, 4 * sms), a.B, 1);
+    if ((long)g.x * a.B < sms) {
+        for (unsigned u = a.field_use; u; u &= u - 1) ++g.z; /* and the initial slices */
+    }
     if (prec == SCFT_PREC_FP64)
         k_boltz_init<double><<<g, POST_THREADS, 0, st>>>(a);
     else if (prec == SCFT_PREC_FP32X2)
@@ -605,61 +687,57 @@ cudaError_t scft_post_mark_start(const PostArgs &a, cudaStream_t st)
     return cudaGetLastError();
 }
 
-int scft_post_nparts(long m, int sms) { return grid_for(m, sms); }
+static int density_grid(long m, int prec, int sms)
+{
+    const int v = prec == SCFT_PREC_FP32 ? 4 : 2;
+    return grid_for((m + v - 1) / v, DENSITY_THREADS, 16 * sms);
+}
+
+/* Partial sums of a species' Q: few, as every CTA of the update adds them up again. */
+int scft_post_qparts(long m, int prec, int sms)
+{
+    const int g = density_grid(m, prec, sms);
+    return g < 64 ? g : 64;
+}
+int scft_post_nparts(long m, int sms) { return grid_for(m, UPDATE_THREADS, 4 * sms); }
 
 cudaError_t scft_density_launch(const PostArgs &a, int prec, int sms, cudaStream_t st)
 {
-    const int vw = prec == SCFT_PREC_FP32 ? 4 : 2;
-    dim3 gd(grid_for((a.m + vw - 1) / vw, sms), a.nblocks, a.B);
+    dim3 gd(density_grid(a.m, prec, sms), a.nblocks + a.nq_species, a.B);
     if (prec == SCFT_PREC_FP64)
-        k_density<double><<<gd, POST_THREADS, 0, st>>>(a);
+        k_density<double><<<gd, DENSITY_THREADS, 0, st>>>(a);
     else if (prec == SCFT_PREC_FP32X2)
-        k_density<dfloat><<<gd, POST_THREADS, 0, st>>>(a);
+        k_density<dfloat><<<gd, DENSITY_THREADS, 0, st>>>(a);
     else
-        k_density<float><<<gd, POST_THREADS, 0, st>>>(a);
+        k_density<float><<<gd, DENSITY_THREADS, 0, st>>>(a);
     return cudaGetLastError();
 }
 
 cudaError_t scft_post_iter_end(const PostArgs &a, int prec, int sms, cudaStream_t st)
 {
-    const int gp = grid_for(a.m, sms);
-    dim3 gq(gp, SCFT_NSPECIES, a.B);
-    if (prec == SCFT_PREC_FP64)
-        k_q_partial<double><<<gq, POST_THREADS, 0, st>>>(a);
-    else if (prec == SCFT_PREC_FP32X2)
-        k_q_partial<dfloat><<<gq, POST_THREADS, 0, st>>>(a);
-    else
-        k_q_partial<float><<<gq, POST_THREADS, 0, st>>>(a);
-    k_q_final<<<dim3(SCFT_NSPECIES, a.B), 32, 0, st>>>(a, gp);
-    const int vw = prec == SCFT_PREC_FP32 ? 4 : 2;
-    dim3 gd(grid_for((a.m + vw - 1) / vw, sms), a.nblocks, a.B);
-    if (prec == SCFT_PREC_FP64)
-        k_density<double><<<gd, POST_THREADS, 0, st>>>(a);
-    else if (prec == SCFT_PREC_FP32X2)
-        k_density<dfloat><<<gd, POST_THREADS, 0, st>>>(a);
-    else
-        k_density<float><<<gd, POST_THREADS, 0, st>>>(a);
+    cudaError_t e = scft_density_launch(a, prec, sms, st);
+    if (e != cudaSuccess) return e;
+    const int gp = scft_post_nparts(a.m, sms);
     {
         const dim3 gu(gp, a.B);
         switch (a.n_active) {
-        case 1: k_update<1><<<gu, POST_THREADS, 0, st>>>(a); break;
-        case 2: k_update<2><<<gu, POST_THREADS, 0, st>>>(a); break;
-        case 3: k_update<3><<<gu, POST_THREADS, 0, st>>>(a); break;
-        case 4: k_update<4><<<gu, POST_THREADS, 0, st>>>(a); break;
-        case 5: k_update<5><<<gu, POST_THREADS, 0, st>>>(a); break;
-        case 6: k_update<6><<<gu, POST_THREADS, 0, st>>>(a); break;
-        case 7: k_update<7><<<gu, POST_THREADS, 0, st>>>(a); break;
-        case 8: k_update<8><<<gu, POST_THREADS, 0, st>>>(a); break;
-        case 9: k_update<9><<<gu, POST_THREADS, 0, st>>>(a); break;
-        case 10: k_update<10><<<gu, POST_THREADS, 0, st>>>(a); break;
-        case 11: k_update<11><<<gu, POST_THREADS, 0, st>>>(a); break;
-        case 12: k_update<12><<<gu, POST_THREADS, 0, st>>>(a); break;
-        case 13: k_update<13><<<gu, POST_THREADS, 0, st>>>(a); break;
+        case 1: k_update<1><<<gu, UPDATE_THREADS, 0, st>>>(a); break;
+        case 2: k_update<2><<<gu, UPDATE_THREADS, 0, st>>>(a); break;
+        case 3: k_update<3><<<gu, UPDATE_THREADS, 0, st>>>(a); break;
+        case 4: k_update<4><<<gu, UPDATE_THREADS, 0, st>>>(a); break;
+        case 5: k_update<5><<<gu, UPDATE_THREADS, 0, st>>>(a); break;
+        case 6: k_update<6><<<gu, UPDATE_THREADS, 0, st>>>(a); break;
+        case 7: k_update<7><<<gu, UPDATE_THREADS, 0, st>>>(a); break;
+        case 8: k_update<8><<<gu, UPDATE_THREADS, 0, st>>>(a); break;
+        case 9: k_update<9><<<gu, UPDATE_THREADS, 0, st>>>(a); break;
+        case 10: k_update<10><<<gu, UPDATE_THREADS, 0, st>>>(a); break;
+        case 11: k_update<11><<<gu, UPDATE_THREADS, 0, st>>>(a); break;
+        case 12: k_update<12><<<gu, UPDATE_THREADS, 0, st>>>(a); break;
+        case 13: k_update<13><<<gu, UPDATE_THREADS, 0, st>>>(a); break;
         default: return cudaErrorInvalidValue;
         }
     }
-    k_finalize<<<a.B, POST_THREADS, 0, st>>>(a, gp);
-    k_p_shift<<<dim3(gp, a.B), POST_THREADS, 0, st>>>(a);
+    k_p_shift<<<dim3(grid_for(a.m, POST_THREADS, 4 * sms), a.B), POST_THREADS, 0, st>>>(a);
     return cudaGetLastError();
 }
 
