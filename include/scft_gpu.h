@@ -305,7 +305,7 @@ typedef struct scft_timing {
                           2 the 64^3 cluster kernel; 0 per-axis passes (prop_launches tells whether
                           each is a launch or a chain's passes run in one) */
     int threads_per_line; /* fused 2D kernel: 2 when a batch of at most one chain per SM gives each
-                             line two threads (bit-identical results), else 1 */
+                             line two threads, or each chain several CTAs (bit-identical results), else 1 */
 } scft_timing;
 int scft_enable_timing(scft_ctx *ctx, int on);
 int scft_get_timing(const scft_ctx *ctx, scft_timing *t);

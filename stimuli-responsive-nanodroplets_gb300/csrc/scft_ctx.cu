@@ -113,7 +113,7 @@ struct scft_ctx {
     std::vector<ChainSpec> cs0; /* instance 0's chains: the composition every instance shares */
     /* fused contour loops: 2D (scft_step2d.cu), 64^3 clusters (scft_step3d.cu) */
     int fused2d = 0;
-    int wide2d = 0; /* fused 2D loop with two threads per line (batches of at most one chain per SM) */
+    int wide2d = 0; /* fused 2D loop: 1 two threads per line, 4 or 8 a cluster of CTAs per chain, for small batches */
     int fused3d = 0;
     int loop_tc = 0; /* the cluster contour loop on the tensor-core tiles (k_chain_tc) */
     TcLoop loop;
@@ -569,6 +569,17 @@ static int fused2d_tables(scft_ctx *c, const scft_derived &d, InstOps &o)
     return SCFT_OK;
 }
 
+/* Clusters of g CTAs for each chain of the fused 2D loop: at most one CTA per SM. One
+ * film of 192x96 takes 1121 us a loop with two threads per line, 693 with g = 4 and 491
+ * with g = 8; 4 films 1144, 698 and 736. Two CTAs per SM can gain too where the batch
+ * is alone (8 films, g = 4: 702), but five batches side by side then get in each
+ * other's way (64 mixed instances: 16.8 -> 17.7 ms for 8 iterations). */
+static bool cluster2d_ok(const scft_ctx *c, int g)
+{
+    return (long)c->B * c->nchains * g <= c->sms &&
+           scft_step2d_cluster(c->opt.precision, c->der[0].nx, c->der[0].nz, g);
+}
+
 /* The fused 2D step: z operator rows (A then B, row-major) and the x factor
  * E(k)/NX per operator set, the four-step twiddles along x once. */
 static int build_fused2d(scft_ctx *c)
@@ -600,7 +611,10 @@ static int build_fused2d(scft_ctx *c)
     c->fused2d = 1;
     /* a batch with at most one chain per SM runs one CTA per SM either way: twice
      * the threads per chain shortens each step, with bit-identical results */
-    c->wide2d = scft_step2d_wide(c->opt.precision, nx, d0.nz) && (long)c->B * c->nchains <= c->sms;
+    const long chains = (long)c->B * c->nchains;
+    c->wide2d = scft_step2d_wide(c->opt.precision, nx, d0.nz) && chains <= c->sms;
+    for (int g = 8; g >= 4; g /= 2)
+        if (c->wide2d < 2 && cluster2d_ok(c, g)) c->wide2d = g;
     return SCFT_OK;
 }
 /* Blocks of a tensor-core pass: half-axis and mirror symmetry on periodic axes of
@@ -1325,7 +1339,10 @@ static int autotune_fused2d(scft_ctx *c)
     float best_ms = 1e30f;
     int best = c->wide2d;
     cudaError_t e = cudaSuccess;
-    for (int wide = 0; wide <= 1 && e == cudaSuccess; ++wide) {
+    static const int forms[] = {0, 1, 4, 8};
+    for (int wide : forms) {
+        if (e != cudaSuccess) break;
+        if (wide > 1 && !cluster2d_ok(c, wide)) continue;
         e = scft_launch_step2d(c->opt.precision, c->nx, c->nz, a, total, c->stream, 0, wide); /* warm-up */
         if (e == cudaSuccess) e = cudaEventRecord(e0, c->stream);
         for (int r = 0; r < 2 && e == cudaSuccess; ++r)

@@ -251,6 +251,7 @@ cudaError_t scft_launch_step2d(int prec, int nx, int nz, const Step2DArgs &a, in
                                int configure, int wide);
 /* 1 if (nx, nz) has the two-threads-per-line form of the fused 2D loop */
 int scft_step2d_wide(int prec, int nx, int nz);
+int scft_step2d_cluster(int prec, int nx, int nz, int g);
 /* 1 if the fused 2D loop of (nx, nz) runs the z tail on the tensor cores */
 int scft_step2d_ztc(int prec, int nx, int nz);
 /* 1 if a tensor-core wait of the 2D loop gave up since the last call (clears it) */

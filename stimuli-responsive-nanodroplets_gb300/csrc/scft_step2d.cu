@@ -454,41 +454,46 @@ __device__ __forceinline__ void mma_bf16(uint32_t d, uint32_t a, uint64_t b, uin
                  : "memory");
 }
 
-/* u, v of one line split into bf16 pairs and stored to the A columns of its
- * TMEM lane (ta = lane address of column COL_A); the line is read from shared
- * memory 16 columns (and their mirror images) at a time. */
+/* 16 columns of u, v of one line (chunk c) split into bf16 pairs and stored to the
+ * A columns of its TMEM lane (ta = lane address of column COL_A); pair(k) returns
+ * the line's columns 2k, 2k + 1. */
+template <int NZ, typename Pair>
+__device__ __forceinline__ void ztc_store_chunk(const Pair &pair, int c, uint32_t ta)
+{
+    using Z = ZTail<NZ>;
+    float lo[16], hi[16]; /* x[16c + i], x[NZ - 16 - 16c + i] */
+#pragma unroll
+    for (int i = 0; i < 16; i += 2) {
+        const float2 a = pair(8 * c + i / 2);
+        const float2 m = pair(NZ / 2 - 8 - 8 * c + i / 2);
+        lo[i] = a.x;
+        lo[i + 1] = a.y;
+        hi[i] = m.x;
+        hi[i + 1] = m.y;
+    }
+    uint32_t u1[8], u2[8], v1[8], v2[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        /* k = 16c + 2j: x[k], x[k+1] and their mirrors x[NZ-1-k], x[NZ-2-k] */
+        const float xa = lo[2 * j], xb = lo[2 * j + 1], ma = hi[15 - 2 * j], mb = hi[14 - 2 * j];
+        const float ua = xa + ma, ub = xb + mb, va = xa - ma, vb = xb - mb;
+        u1[j] = bf16x2_rn(ub, ua); /* even k in the low half */
+        v1[j] = bf16x2_rn(vb, va);
+        u2[j] = bf16x2_rn(ub - bf16_hi(u1[j]), ua - bf16_lo(u1[j]));
+        v2[j] = bf16x2_rn(vb - bf16_hi(v1[j]), va - bf16_lo(v1[j]));
+    }
+    tm_st8(ta + 0 * Z::PC + 8 * c, u1);
+    tm_st8(ta + 1 * Z::PC + 8 * c, u2);
+    tm_st8(ta + 2 * Z::PC + 8 * c, v1);
+    tm_st8(ta + 3 * Z::PC + 8 * c, v2);
+}
+/* A whole line, from shared memory. */
 template <int NZ>
 __device__ __forceinline__ void ztc_store_a(const float *row, uint32_t ta)
 {
-    using Z = ZTail<NZ>;
+    auto pair = [&](int k) { return *reinterpret_cast<const float2 *>(row + 2 * k); };
 #pragma unroll
-    for (int c = 0; c < Z::H / 16; ++c) {
-        float lo[16], hi[16]; /* x[16c + i], x[NZ - 16 - 16c + i] */
-#pragma unroll
-        for (int i = 0; i < 16; i += 2) {
-            const float2 a = *reinterpret_cast<const float2 *>(row + 16 * c + i);
-            const float2 m = *reinterpret_cast<const float2 *>(row + NZ - 16 - 16 * c + i);
-            lo[i] = a.x;
-            lo[i + 1] = a.y;
-            hi[i] = m.x;
-            hi[i + 1] = m.y;
-        }
-        uint32_t u1[8], u2[8], v1[8], v2[8];
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            /* k = 16c + 2j: x[k], x[k+1] and their mirrors x[NZ-1-k], x[NZ-2-k] */
-            const float xa = lo[2 * j], xb = lo[2 * j + 1], ma = hi[15 - 2 * j], mb = hi[14 - 2 * j];
-            const float ua = xa + ma, ub = xb + mb, va = xa - ma, vb = xb - mb;
-            u1[j] = bf16x2_rn(ub, ua); /* even k in the low half */
-            v1[j] = bf16x2_rn(vb, va);
-            u2[j] = bf16x2_rn(ub - bf16_hi(u1[j]), ua - bf16_lo(u1[j]));
-            v2[j] = bf16x2_rn(vb - bf16_hi(v1[j]), va - bf16_lo(v1[j]));
-        }
-        tm_st8(ta + 0 * Z::PC + 8 * c, u1);
-        tm_st8(ta + 1 * Z::PC + 8 * c, u2);
-        tm_st8(ta + 2 * Z::PC + 8 * c, v1);
-        tm_st8(ta + 3 * Z::PC + 8 * c, v2);
-    }
+    for (int c = 0; c < ZTail<NZ>::H / 16; ++c) ztc_store_chunk<NZ>(pair, c, ta);
     asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
 
@@ -613,6 +618,40 @@ __device__ __forceinline__ void ztc_band(float *row, const float *bt)
         pair_rows(j, j - NZ + 2 * R0);
         shift();
     }
+}
+
+/* Band rows j, j + 1 alone, from x = x[j - 3 .. j + 5] (the sums of ztc_band). */
+template <int NZ>
+__device__ __forceinline__ float2 ztc_band_pair(const float *x0, int j, const float4 *b4)
+{
+    constexpr int R0 = ZTail<NZ>::R0;
+    float y[2];
+    if (j >= R0 && j < NZ - R0) {
+        const float4 cc = b4[4 * R0];
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            const float *x = x0 + e;
+            float t = cc.w * (x[0] + x[6]);
+            t = fmaf(cc.z, x[1] + x[5], t);
+            t = fmaf(cc.y, x[2] + x[4], t);
+            y[e] = fmaf(cc.x, x[3], t);
+        }
+    } else {
+        const int r = j < R0 ? j : j - NZ + 2 * R0;
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            const float4 ca = b4[2 * (r + e)], cb = b4[2 * (r + e) + 1];
+            const float *x = x0 + e;
+            float t = ca.x * x[0];
+            t = fmaf(cb.z, x[6], t);
+            t = fmaf(ca.y, x[1], t);
+            t = fmaf(cb.y, x[5], t);
+            t = fmaf(ca.z, x[2], t);
+            t = fmaf(cb.x, x[4], t);
+            y[e] = fmaf(ca.w, x[3], t);
+        }
+    }
+    return make_float2(y[0], y[1]);
 }
 
 /* Adds the tail (Pe + Po on top, Pe - Po mirrored below) to the band values of
@@ -1106,6 +1145,290 @@ __global__ void __launch_bounds__(NX * TM, (MinBlocks2D<P, NX, NZ, TM>::value)) 
     }
 }
 
+/* --------------------------------------------------- a cluster per chain
+ * The same contour loop with a chain's slice spread over G CTAs, for batches that
+ * leave SMs idle: a CTA has NZ/2/G complex columns for the x phases and NX/G rows
+ * for the z phase, each with the arithmetic of k_chain2d, so that the bits do not
+ * depend on G. Between the two the slice changes hands in G x G blocks of rows and
+ * columns, copied from shared memory to shared memory (cp.async.bulk) and counted by
+ * the receiver's barrier; a CTA's rows are kept block by block as they come and go.
+ * A block is only sent again once its receiver, and with it every CTA, has sent what
+ * it made of the last ones, so one buffer each way is enough.
+ * A step is bounded by the latency of its phases (the DFT of a column pair in one
+ * thread, the tail's MMAs) and of the two exchanges: 192x96, one film, 8.9 -> 3.9 us a
+ * step with G = 8 (5.5 with G = 4; with G = 2 no faster than two threads per line). */
+template <int NX, int NZ, int G>
+struct Cl2D {
+    static constexpr int H = NZ / 2, CW = NZ / 2 / G, RW = NX / G;
+    static constexpr int T = 128 * (H / 16);         /* a warp of each TMEM lane quadrant for every 16 columns */
+    static constexpr uint32_t BLOCK = RW * CW * 8;   /* bytes that one CTA sends another */
+    static constexpr uint32_t XC = 0;                /* complex [NX][CW] */
+    static constexpr uint32_t R = XC + NX * CW * 8;  /* complex [G][RW][CW] */
+    static constexpr int TP = NZ + 1;                /* pitch of the tails */
+    static constexpr uint32_t TB = R + NX * CW * 8;  /* [RW][TP] */
+    static constexpr uint32_t KP = (TB + RW * TP * 4 + 127) / 128 * 128; /* operator pieces */
+    static constexpr uint32_t TW = KP + 8 * H * H;
+    static constexpr uint32_t EX = TW + 8 * NX;
+    static constexpr uint32_t BAND = EX + 4 * NX;
+    static constexpr uint32_t BARS = (BAND + ZTail<NZ>::BAND_BYTES + 15) / 16 * 16; /* tail, rows, columns */
+    static constexpr uint32_t END = BARS + 32;
+    /* no more CTAs on an SM than its TMEM serves, whatever else runs there: a CTA that
+     * holds columns never waits for one that wants them */
+    static constexpr uint32_t SHARE = 233472 / 512 * ZTail<NZ>::TCOLS - 1024;
+    static constexpr uint32_t SMEM = END > SHARE ? END : SHARE;
+    static constexpr bool ok = (NZ / 2) % G == 0 && NX % G == 0 && BLOCK % 16 == 0 && RW <= 64;
+};
+
+__device__ __forceinline__ uint32_t cluster_addr(uint32_t addr, uint32_t rank)
+{
+    uint32_t r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+    return r;
+}
+/* bytes from this CTA's shared memory to another's, counted by its barrier */
+__device__ __forceinline__ void copy_to(uint32_t rank, uint32_t dst, uint32_t src, uint32_t bytes, uint32_t bar)
+{
+    asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(cluster_addr(dst, rank)),
+                 "r"(src), "r"(bytes), "r"(cluster_addr(bar, rank))
+                 : "memory");
+}
+__device__ __forceinline__ void expect(uint32_t bar, uint32_t bytes)
+{
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+
+template <int NX, int NZ, int N1, int N2, int G>
+__global__ void __launch_bounds__(Cl2D<NX, NZ, G>::T, 1) k_chain2d_cl(Step2DArgs a)
+{
+    using L = Cl2D<NX, NZ, G>;
+    using Z = ZTail<NZ>;
+    constexpr int T = L::T, CW = L::CW, RW = L::RW, NZ2 = NZ / 2;
+    constexpr int PAIRS = RW * NZ2, PER = (PAIRS + T - 1) / T; /* row pairs, per thread */
+    const int rank = blockIdx.x % G, slot = blockIdx.x / G; /* clusters are consecutive blocks */
+    const ChainDesc cd = a.chains[a.order ? a.order[slot] : slot];
+    if (a.state && a.state[cd.instance].done) return; /* uniform over the cluster */
+    const int s_end = a.s_end < cd.len - 1 ? a.s_end : cd.len - 1;
+    if (a.s >= s_end) return;
+
+    extern __shared__ __align__(128) unsigned char smem[];
+    const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(smem);
+    Cx<float> *XC = reinterpret_cast<Cx<float> *>(smem + L::XC);
+    float2 *R = reinterpret_cast<float2 *>(smem + L::R);
+    float *TB = reinterpret_cast<float *>(smem + L::TB);
+    const Cx<float> *TW = reinterpret_cast<const Cx<float> *>(smem + L::TW);
+    const float *EX = reinterpret_cast<const float *>(smem + L::EX);
+    const uint32_t bar_tail = sbase + L::BARS, bar_rows = bar_tail + 8, bar_cols = bar_tail + 16;
+    uint32_t *tslot = reinterpret_cast<uint32_t *>(smem + L::BARS + 24);
+    const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
+
+    /* operators and tables, once per chain */
+    {
+        constexpr int NB = Z::BAND_BYTES / 16, NP = 8 * Z::H * Z::H / 16;
+        const unsigned char *g = reinterpret_cast<const unsigned char *>(cd.ops->kz);
+        for (int e = tid; e < NB; e += T) cp_async16(smem + L::BAND + 16 * e, g + 16 * e);
+        for (int e = tid; e < NP; e += T) cp_async16(smem + L::KP + 16 * e, g + 16 * NB + 16 * e);
+        for (int e = tid; e < NX / 2; e += T) cp_async16(smem + L::TW + 16 * e, reinterpret_cast<const unsigned char *>(cd.ops->twx) + 16 * e);
+        for (int e = tid; e < NX / 4; e += T) cp_async16(smem + L::EX + 16 * e, reinterpret_cast<const unsigned char *>(cd.ops->ex) + 16 * e);
+        asm volatile("cp.async.commit_group;\n" ::);
+    }
+    if (tid == 0) {
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 2;" ::"r"(bar_tail) : "memory");
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar_rows) : "memory");
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar_cols) : "memory");
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        expect(bar_rows, G * L::BLOCK);
+        expect(bar_cols, G * L::BLOCK);
+    }
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"((uint32_t)__cvta_generic_to_shared(tslot)),
+                     "r"(Z::TCOLS)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    /* the first columns: b . q_s from global memory */
+    {
+        const float2 *q = reinterpret_cast<const float2 *>(reinterpret_cast<const float *>(cd.q) + (long)a.s * a.sstride) + rank * CW;
+        const float2 *b = reinterpret_cast<const float2 *>(a.s < cd.seg_end ? cd.b0 : cd.b1) + rank * CW;
+        for (int e = tid; e < NX * CW; e += T) {
+            const int x = e / CW, c = e - x * CW;
+            const float2 qv = q[x * NZ2 + c], bv = b[x * NZ2 + c];
+            XC[e] = {qv.x * bv.x, qv.y * bv.y};
+        }
+    }
+    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); /* the tensor cores read the operator pieces */
+    tc_fence_before();
+    /* every CTA's barriers are set up before anyone sends, and its columns allocated before anyone waits */
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    tc_fence_after();
+    const uint32_t tmem = *tslot;
+    const int quad = warp & 3, zc = warp >> 2; /* TMEM lanes and 16-column chunk of this warp */
+    const bool row_warp = quad * 32 < RW;
+    auto pair_at = [&](int r, int c) { /* columns 2c, 2c + 1 of row r */
+        const int g = c / CW;
+        return (g * RW + r) * CW + (c - g * CW);
+    };
+    float2 bres[PER];
+    const void *bres_src = nullptr;
+    int failed = 0;
+
+#pragma unroll 1
+    for (int s = a.s; s < s_end; ++s) {
+        const uint32_t phase = (uint32_t)(s - a.s) & 1u;
+        const float2 *bz = reinterpret_cast<const float2 *>(s < cd.seg_end ? cd.b0 : cd.b1) + rank * PAIRS;
+        const float2 *bnext = reinterpret_cast<const float2 *>(s + 1 < cd.seg_end ? cd.b0 : cd.b1) + rank * PAIRS;
+        float2 *qn = reinterpret_cast<float2 *>(reinterpret_cast<float *>(cd.q) + (long)(s + 1) * a.sstride) + rank * PAIRS;
+        if (bres_src != bz) {
+#pragma unroll
+            for (int i = 0; i < PER; ++i)
+                if (PAIRS % T == 0 || tid + i * T < PAIRS) bres[i] = bz[tid + i * T];
+            bres_src = bz;
+        }
+        bool ok = true;
+        if (s > a.s) { /* columns of b . q_s */
+            ok = mbar_wait<true>(bar_cols, phase ^ 1u);
+            if (ok && tid == 0 && s + 1 < s_end) expect(bar_cols, G * L::BLOCK);
+        }
+        /* x: A, B, C as in k_chain2d, on this CTA's columns */
+        for (int w = tid; w < N2 * CW; w += T) {
+            const int n2 = w / CW;
+            Cx<float> v[N1];
+#pragma unroll
+            for (int n1 = 0; n1 < N1; ++n1) v[n1] = XC[N2 * CW * n1 + w];
+            Dft<float, N1, false>::run(v);
+#pragma unroll
+            for (int k1 = 1; k1 < N1; ++k1) v[k1] = cmul(v[k1], TW[n2 * N1 + k1]);
+#pragma unroll
+            for (int k1 = 0; k1 < N1; ++k1) XC[N2 * CW * k1 + w] = v[k1];
+        }
+        __syncthreads();
+        for (int w = tid; w < N1 * CW; w += T) {
+            const int k1 = w / CW, c = w - k1 * CW;
+            Cx<float> u[N2];
+#pragma unroll
+            for (int n2 = 0; n2 < N2; ++n2) u[n2] = XC[(N2 * k1 + n2) * CW + c];
+            Dft<float, N2, false>::run(u);
+#pragma unroll
+            for (int k2 = 0; k2 < N2; ++k2) {
+                if (k2 == 0 && k1 == 0) { /* mean mode: a division, as in k_chain2d */
+                    u[0].x = u[0].x / (float)NX;
+                    u[0].y = u[0].y / (float)NX;
+                    continue;
+                }
+                const float f = EX[k1 + N1 * k2];
+                u[k2].x *= f;
+                u[k2].y *= f;
+            }
+            Dft<float, N2, true>::run(u);
+#pragma unroll
+            for (int n2 = 1; n2 < N2; ++n2) u[n2] = cmulc(u[n2], TW[n2 * N1 + k1]);
+#pragma unroll
+            for (int n2 = 0; n2 < N2; ++n2) XC[(N2 * k1 + n2) * CW + c] = u[n2];
+        }
+        __syncthreads();
+        for (int w = tid; w < N2 * CW; w += T) {
+            Cx<float> v[N1];
+#pragma unroll
+            for (int k1 = 0; k1 < N1; ++k1) v[k1] = XC[N2 * CW * k1 + w];
+            Dft<float, N1, true>::run(v);
+#pragma unroll
+            for (int n1 = 0; n1 < N1; ++n1) XC[N2 * CW * n1 + w] = v[n1];
+        }
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        failed = __syncthreads_or(!ok);
+        if (failed) break; /* the others' waits run out too */
+        /* rows x of block g to CTA g, which has them as its block `rank` */
+        if (tid < G) copy_to(tid, sbase + L::R + rank * L::BLOCK, sbase + L::XC + tid * L::BLOCK, L::BLOCK, bar_rows);
+
+        /* z: band on the FP32 pipe, tail on the tensor cores */
+        ok = mbar_wait<true>(bar_rows, phase);
+        if (ok && tid == 0 && s + 1 < s_end) expect(bar_rows, G * L::BLOCK);
+        if (row_warp) {
+            const int r = min(quad * 32 + lane, RW - 1);
+            auto pair = [&](int k) { return R[pair_at(r, k)]; };
+            ztc_store_chunk<NZ>(pair, zc, tmem + ((uint32_t)(quad * 32) << 16) + Z::COL_A);
+            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+        }
+        tc_fence_before();
+        __syncthreads();
+        tc_fence_after();
+        ztc_issue_tile<NZ, T>(tid, 2, tmem, sbase + L::KP, bar_tail);
+        float2 y[PER];
+#pragma unroll
+        for (int i = 0; i < PER; ++i) {
+            const int e = tid + i * T;
+            if (PAIRS % T != 0 && e >= PAIRS) break;
+            const int r = e / NZ2, c = e - r * NZ2, j = 2 * c;
+            float w[10]; /* x[j - 4 .. j + 5] */
+#pragma unroll
+            for (int d = 0; d < 5; ++d) {
+                int p = c + d - 2;
+                p = p < 0 ? p + NZ2 : p >= NZ2 ? p - NZ2 : p;
+                const float2 v = R[pair_at(r, p)];
+                w[2 * d] = v.x;
+                w[2 * d + 1] = v.y;
+            }
+            y[i] = ztc_band_pair<NZ>(w + 1, j, reinterpret_cast<const float4 *>(smem + L::BAND));
+        }
+        const bool tail = mbar_wait(bar_tail, phase);
+        ok = __all_sync(0xffffffffu, ok && tail);
+        tc_fence_after();
+        if (row_warp && ok) {
+            const int r = quad * 32 + lane;
+            uint32_t pe[16], po[16];
+            tm_ld16(tmem + ((uint32_t)(quad * 32) << 16) + Z::COL_PE + 16 * zc, pe);
+            tm_ld16(tmem + ((uint32_t)(quad * 32) << 16) + Z::COL_PO + 16 * zc, po);
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+            if (r < RW) {
+#pragma unroll
+                for (int i = 0; i < 16; ++i) {
+                    const float ev = __uint_as_float(pe[i]), od = __uint_as_float(po[i]);
+                    TB[r * L::TP + 16 * zc + i] = ev + od;
+                    TB[r * L::TP + NZ - 1 - 16 * zc - i] = ev - od;
+                }
+            }
+        }
+        tc_fence_before();
+        failed = __syncthreads_or(!ok);
+        tc_fence_after();
+        if (failed) break;
+        /* q_{s+1} = b . y to HBM, and b_next . q_{s+1} back to the owners of its columns */
+#pragma unroll
+        for (int i = 0; i < PER; ++i) {
+            const int e = tid + i * T;
+            if (PAIRS % T != 0 && e >= PAIRS) break;
+            const int r = e / NZ2, c = e - r * NZ2;
+            const float yx = y[i].x + TB[r * L::TP + 2 * c], yy = y[i].y + TB[r * L::TP + 2 * c + 1];
+            const float2 o = make_float2(yx * bres[i].x, yy * bres[i].y);
+            qn[e] = o;
+            if (s + 1 < s_end) {
+                const float2 nb = bnext == bz ? bres[i] : bnext[e];
+                R[pair_at(r, c)] = make_float2(o.x * nb.x, o.y * nb.y);
+            }
+        }
+        if (s + 1 < s_end) {
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncthreads();
+            if (tid < G) copy_to(tid, sbase + L::XC + rank * L::BLOCK, sbase + L::R + tid * L::BLOCK, L::BLOCK, bar_cols);
+        }
+    }
+    if (failed) {
+        /* a wait that gave up: the last slice goes out as NaN (the instance then reports a
+         * non-finite status) and the chain stops, after its own copies have had time to land */
+        if (tid == 0) atomicExch(&g_scft_tc_fault, 1);
+        float2 *qn = reinterpret_cast<float2 *>(reinterpret_cast<float *>(cd.q) + (long)s_end * a.sstride) + rank * PAIRS;
+        for (int e = tid; e < PAIRS; e += T) qn[e] = make_float2(__int_as_float(0x7fc00000), __int_as_float(0x7fc00000));
+        for (const long long t0 = clock64(); clock64() - t0 < (1 << 20);) {}
+    }
+    tc_fence_before();
+    /* no CTA leaves while another could still send to it */
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    if (warp == 0) {
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(Z::TCOLS) : "memory");
+    }
+}
+
 /* ---------------------------------------------------------------- dispatch */
 template <typename P, int NX, int NZ, int N1, int N2>
 static size_t smem_bytes_t()
@@ -1147,6 +1470,35 @@ struct WideOk {
     static constexpr bool value = (NZ / 2) % 8 == 0 && SCFT_F32X2;
 };
 
+template <typename P, int NX, int NZ, int G>
+struct ClOk {
+    static constexpr bool value = ZTcOk<P, NX, NZ>::value && Cl2D<NX, NZ, G>::ok;
+};
+
+template <typename P, int NX, int NZ, int N1, int N2, int G>
+static cudaError_t launch_cl(const Step2DArgs &a, int nchains, cudaStream_t st, int configure)
+{
+    if constexpr (ClOk<P, NX, NZ, G>::value) {
+        using L = Cl2D<NX, NZ, G>;
+        if (configure)
+            return cudaFuncSetAttribute(k_chain2d_cl<NX, NZ, N1, N2, G>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::SMEM);
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)(nchains * G), 1, 1);
+        cfg.blockDim = dim3(L::T, 1, 1);
+        cfg.dynamicSmemBytes = L::SMEM;
+        cfg.stream = st;
+        cudaLaunchAttribute attr;
+        attr.id = cudaLaunchAttributeClusterDimension;
+        attr.val.clusterDim.x = G;
+        attr.val.clusterDim.y = 1;
+        attr.val.clusterDim.z = 1;
+        cfg.attrs = &attr;
+        cfg.numAttrs = 1;
+        return cudaLaunchKernelEx(&cfg, k_chain2d_cl<NX, NZ, N1, N2, G>, a);
+    }
+    return configure ? cudaSuccess : cudaErrorInvalidValue;
+}
+
 template <typename P, int NX, int NZ, int N1, int N2>
 static cudaError_t launch_t(const Step2DArgs &a, int nblocks, cudaStream_t st, int configure, int wide)
 {
@@ -1158,7 +1510,13 @@ static cudaError_t launch_t(const Step2DArgs &a, int nblocks, cudaStream_t st, i
             if (e == cudaSuccess)
                 e = cudaFuncSetAttribute(k_chain2d<P, NX, NZ, N1, N2, 2>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e == cudaSuccess) e = launch_cl<P, NX, NZ, N1, N2, 4>(a, 0, st, 1);
+        if (e == cudaSuccess) e = launch_cl<P, NX, NZ, N1, N2, 8>(a, 0, st, 1);
         return e;
+    }
+    if (wide > 1) {
+        if (wide == 4) return launch_cl<P, NX, NZ, N1, N2, 4>(a, nblocks, st, 0);
+        return launch_cl<P, NX, NZ, N1, N2, 8>(a, nblocks, st, 0);
     }
     if constexpr (WideOk<NX, NZ>::value) {
         if (wide) {
@@ -1221,9 +1579,21 @@ int scft_step2d_wide(int prec, int nx, int nz)
     return 0;
 }
 
+/* 1 if the shape has the loop of clusters of g CTAs a chain (the same bits). */
+int scft_step2d_cluster(int prec, int nx, int nz, int g)
+{
+    if (prec != SCFT_PREC_FP32) return 0;
+#define X(NX_, NZ_, A_, B_)                                                                                           \
+    if (nx == NX_ && nz == NZ_)                                                                                       \
+        return g == 4 ? ClOk<float, NX_, NZ_, 4>::value : g == 8 ? ClOk<float, NX_, NZ_, 8>::value : 0;
+    SCFT_STEP2D_SHAPES(X)
+#undef X
+    return 0;
+}
+
 /* configure = 1 raises the kernels' shared-memory limit (call once, outside
  * any stream capture); configure = 0 launches, with two threads per line if
- * wide is set and the shape has that kernel. */
+ * wide is 1 and the shape has that kernel, or clusters of `wide` CTAs a chain. */
 cudaError_t scft_launch_step2d(int prec, int nx, int nz, const Step2DArgs &a, int nblocks, cudaStream_t st,
                                int configure, int wide)
 {

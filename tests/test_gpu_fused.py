@@ -91,3 +91,29 @@ def test_two_threads_per_line_bit_identical(srn, nx, nz):
     np.testing.assert_array_equal(w1, wb)
     np.testing.assert_array_equal(p1, pb)
     np.testing.assert_array_equal(s1, sb)
+
+
+@pytest.mark.parametrize("B", [1, 5])
+@pytest.mark.parametrize("nx,nz", [(192, 96), (192, 128), (128, 96), (96, 64), (64, 64), (64, 32), (32, 32)])
+def test_cluster_per_chain_bit_identical(srn, nx, nz, B):
+    """Small batches spread each chain over a cluster of CTAs (8 for one film of five
+    chains, 4 for five films): bit for bit the one-CTA loop of a large batch, diblock
+    junction and chains of different lengths included."""
+    s = srn.configs.film2d(nx=nx, nz=nz, ns=40, iters=3)
+    w = srn.configs.droplet_fields(s, seed=9, radius=nx * 0.125 / 5)
+    m = srn.configs.substrate_mask(s)
+
+    def run(n):
+        with srn.Solver([s] * n, precision="fp32", autotune=False) as sv:
+            for b in range(n):
+                sv.set_fields(w, b)
+                sv.set_masks(m, b)
+                sv.set_iteration(1, b)
+            out = sv.iterate(3)
+            assert sv.timing()["fused_chain"] == 1
+            return [(r[n - 1].free_energy, r[n - 1].rms, tuple(r[n - 1].q)) for r in out], sv.get_fields(n - 1), sv.get_densities(n - 1)
+
+    small, large = run(B), run(40)
+    assert small[0] == large[0]
+    np.testing.assert_array_equal(small[1], large[1])
+    np.testing.assert_array_equal(small[2][0], large[2][0])
