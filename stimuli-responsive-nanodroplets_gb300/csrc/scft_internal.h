@@ -174,7 +174,6 @@ cudaError_t scft_launch_chain_tc(int prec, const TcLoop &lp, const Step2DArgs &a
 /* 1 if a tensor-core wait of a pass gave up since the last call (clears it) */
 int scft_pass_tc_take_fault(void);
 
-/* Arguments shared by the non-propagator kernels (scft_post.cu). */
 /* What the update of an instance needs besides its fields, and the arrival counters of the
  * launches whose last CTA finishes an instance (zero between launches). */
 struct UpdateTable {
@@ -184,6 +183,7 @@ struct UpdateTable {
     unsigned q_arrived, u_arrived;
 };
 
+/* Arguments shared by the non-propagator kernels (scft_post.cu). */
 struct PostArgs {
     const InstParams *params;   /* [B] */
     InstState *state;           /* [B] */
@@ -228,8 +228,12 @@ cudaError_t scft_convert(int prec, const double *src, void *dst, long n, int to_
 cudaError_t scft_boltz_one(int prec, const double *w, void *bz, double ds, long m, cudaStream_t st);
 
 /* Arguments of the fused 2D contour step (scft_step2d.cu). */
+struct StepUnit {
+    int chain, s0, s1; /* contour steps s0 .. s1 - 1 of a chain */
+};
 struct Step2DArgs {
     const ChainDesc *chains;
+    const StepUnit *units; /* loops over clusters: each cluster's part of a chain (or NULL: order, s, s_end) */
     const int *order;  /* chain indices, longest first (or NULL) */
     const InstState *state; /* [B]: chains of frozen instances return at once (NULL: no check) */
     int s;             /* first contour step: reads slice s */
@@ -246,6 +250,18 @@ size_t scft_step2d_smem(int prec, int nx, int nz);
 /* 64^3 periodic FP32 grids: one 8-CTA cluster per chain (scft_step3d.cu) */
 size_t scft_step3d_smem(int prec, int nx, int ny, int nz);
 cudaError_t scft_launch_step3d(const Step2DArgs &a, int nchains, cudaStream_t st, int configure);
+int scft_step3d_resident(void); /* clusters that fit on the GPU */
+/* What cluster `slot` of a launch runs: chain and contour steps. */
+struct StepRange {
+    int chain, s, s_end;
+};
+#ifdef __CUDACC__
+__device__ __forceinline__ StepRange step_range(const Step2DArgs &a, int slot)
+{
+    if (a.units) return {a.units[slot].chain, a.units[slot].s0, a.units[slot].s1};
+    return {a.order ? a.order[slot] : slot, a.s, a.s_end};
+}
+#endif
 int scft_step2d_n1(int nx);
 cudaError_t scft_launch_step2d(int prec, int nx, int nz, const Step2DArgs &a, int nblocks, cudaStream_t st,
                                int configure, int wide);

@@ -931,10 +931,11 @@ template <typename P>
 __global__ void __launch_bounds__(512, 1) k_chain_tc(const __grid_constant__ TcLoop lp, Step2DArgs a)
 {
     const int rank = blockIdx.x % lp.cluster, slot = blockIdx.x / lp.cluster; /* clusters are consecutive blocks */
-    const ChainDesc cd = a.chains[a.order ? a.order[slot] : slot];
+    const StepRange run = step_range(a, slot);
+    const ChainDesc cd = a.chains[run.chain];
     if (a.state && a.state[cd.instance].done) return; /* uniform over the cluster */
-    const int s_end = a.s_end < cd.len - 1 ? a.s_end : cd.len - 1;
-    if (a.s >= s_end) return;
+    const int s_end = run.s_end < cd.len - 1 ? run.s_end : cd.len - 1;
+    if (run.s >= s_end) return;
 
     extern __shared__ __align__(128) unsigned char smem[];
     tc_begin(smem, lp.nax);
@@ -952,7 +953,7 @@ __global__ void __launch_bounds__(512, 1) k_chain_tc(const __grid_constant__ TcL
     const int group = threadIdx.x / (512 / GROUPS);
     const uint32_t tile_at = lp.tile_at + (uint32_t)group * lp.tile_bytes;
 #pragma unroll 1
-    for (int s = a.s; s < s_end; ++s) {
+    for (int s = run.s; s < s_end; ++s) {
         const P *bz = reinterpret_cast<const P *>(s < cd.seg_end ? cd.b0 : cd.b1);
 #pragma unroll 1
         for (int ax = 0; ax < lp.nax; ++ax) {
@@ -966,10 +967,10 @@ __global__ void __launch_bounds__(512, 1) k_chain_tc(const __grid_constant__ TcL
                 for (int t = t0; (long)t * g.tile < g.lines; t += GROUPS * lp.slots[ax]) {
                     if (g.nb == 4)
                         tc_tile<P, 4, 512 / GROUPS, true>(g, src, dst, bz, first, last, t, part, smem, lp.op_at[ax], tile_at,
-                                                 sbase + SM_BAR + 8 * ax, s == a.s && t == t0, ph);
+                                                 sbase + SM_BAR + 8 * ax, s == run.s && t == t0, ph);
                     else
                         tc_tile<P, 2, 512 / GROUPS, true>(g, src, dst, bz, first, last, t, part, smem, lp.op_at[ax], tile_at,
-                                                 sbase + SM_BAR + 8 * ax, s == a.s && t == t0, ph);
+                                                 sbase + SM_BAR + 8 * ax, s == run.s && t == t0, ph);
                 }
             /* this axis' slice is complete before the next one reads it */
             asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
@@ -999,10 +1000,11 @@ template <typename P>
 __global__ void __launch_bounds__(512, 1) k_chain2d_tc(const __grid_constant__ TcLoop lp, Step2DArgs a)
 {
     const int rank = blockIdx.x % lp.cluster, slot = blockIdx.x / lp.cluster; /* clusters are consecutive blocks */
-    const ChainDesc cd = a.chains[a.order ? a.order[slot] : slot];
+    const StepRange run = step_range(a, slot);
+    const ChainDesc cd = a.chains[run.chain];
     if (a.state && a.state[cd.instance].done) return; /* uniform over the cluster */
-    const int s_end = a.s_end < cd.len - 1 ? a.s_end : cd.len - 1;
-    if (a.s >= s_end) return;
+    const int s_end = run.s_end < cd.len - 1 ? run.s_end : cd.len - 1;
+    if (run.s >= s_end) return;
 
     extern __shared__ __align__(128) unsigned char smem[];
     tc_begin(smem, 4); /* operator digits of the two axes, lines of the two axes */
@@ -1026,8 +1028,8 @@ __global__ void __launch_bounds__(512, 1) k_chain2d_tc(const __grid_constant__ T
     /* the first lines: b q_s from global memory */
     if (mine[0]) {
         const TcGeom &g = lp.g[0];
-        const P *src = reinterpret_cast<const P *>(cd.q) + (long)a.s * a.sstride;
-        const P *bz = reinterpret_cast<const P *>(a.s < cd.seg_end ? cd.b0 : cd.b1);
+        const P *src = reinterpret_cast<const P *>(cd.q) + (long)run.s * a.sstride;
+        const P *bz = reinterpret_cast<const P *>(run.s < cd.seg_end ? cd.b0 : cd.b1);
         P *in = reinterpret_cast<P *>(smem + lp.buf_at[0]);
         int *eline = reinterpret_cast<int *>(smem + SM_ELINE);
         const int L0 = rank * g.tile, nlines = (int)min((long)g.tile, g.lines - L0);
@@ -1042,13 +1044,13 @@ __global__ void __launch_bounds__(512, 1) k_chain2d_tc(const __grid_constant__ T
     /* every CTA's barriers are set up before anyone sends */
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 #pragma unroll 1
-    for (int s = a.s; s < s_end; ++s) {
+    for (int s = run.s; s < s_end; ++s) {
         const P *bz = reinterpret_cast<const P *>(s < cd.seg_end ? cd.b0 : cd.b1);
 #pragma unroll 1
         for (int ax = 0; ax < 2; ++ax) {
             if (!mine[ax]) continue;
             const TcGeom &g = lp.g[ax], &o = lp.g[1 - ax];
-            const int t = s - a.s;
+            const int t = s - run.s;
             if (t > 0 || ax == 1) {
                 /* the lines are there; one thread re-arms the barrier for the next step */
                 const uint32_t bar = bars + 16 + 8 * ax;

@@ -233,11 +233,12 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(NT, 1) k_chain3d(St
     cg::cluster_group cl = cg::this_cluster();
     const int rank = (int)cl.block_rank();
     const int slot = blockIdx.x / CL;
-    const ChainDesc cd = a.chains[a.order ? a.order[slot] : slot];
+    const StepRange run = step_range(a, slot);
+    const ChainDesc cd = a.chains[run.chain];
     /* uniform over the cluster: every CTA reads the same descriptor and state */
     if (a.state && a.state[cd.instance].done) return;
-    const int s_end = a.s_end < cd.len - 1 ? a.s_end : cd.len - 1;
-    if (a.s >= s_end) return;
+    const int s_end = run.s_end < cd.len - 1 ? run.s_end : cd.len - 1;
+    if (run.s >= s_end) return;
 
     extern __shared__ __align__(16) unsigned char smem_raw[];
     float *Q = reinterpret_cast<float *>(smem_raw);
@@ -248,8 +249,8 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(NT, 1) k_chain3d(St
 
     /* Q = b_s . q_s in D1 */
     {
-        const float *q = reinterpret_cast<const float *>(cd.q) + (long)a.s * a.sstride;
-        const float *b = reinterpret_cast<const float *>(a.s < cd.seg_end ? cd.b0 : cd.b1);
+        const float *q = reinterpret_cast<const float *>(cd.q) + (long)run.s * a.sstride;
+        const float *b = reinterpret_cast<const float *>(run.s < cd.seg_end ? cd.b0 : cd.b1);
         for (int base = tid; base < PL * N3 * N3 / 4; base += NT * UB) {
             float4 qv[UB], bv[UB];
 #pragma unroll
@@ -269,7 +270,7 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(NT, 1) k_chain3d(St
     __syncthreads();
 
     int d = 0; /* current distribution */
-    for (int s = a.s; s < s_end; ++s) {
+    for (int s = run.s; s < s_end; ++s) {
         /* z lines: plane `warp`, rows lane and lane+32 */
         {
             float *r0 = Q + warp * PP + lane * RP;
@@ -349,24 +350,39 @@ size_t scft_step3d_smem(int prec, int nx, int ny, int nz)
 
 /* configure = 1: raise the shared-memory limit and check that an 8-CTA cluster
  * with this footprint can be resident (returns cudaErrorNotSupported if not). */
+static cudaError_t resident_clusters(int *nclusters)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(CL, 1, 1);
+    cfg.blockDim = dim3(NT, 1, 1);
+    cfg.dynamicSmemBytes = STEP3D_SMEM;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = CL;
+    attr.val.clusterDim.y = 1;
+    attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaOccupancyMaxActiveClusters(nclusters, k_chain3d, &cfg);
+}
+
+int scft_step3d_resident(void)
+{
+    int n = 0;
+    if (resident_clusters(&n) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    return n;
+}
+
 cudaError_t scft_launch_step3d(const Step2DArgs &a, int nchains, cudaStream_t st, int configure)
 {
     if (configure) {
         cudaError_t e = cudaFuncSetAttribute(k_chain3d, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)STEP3D_SMEM);
         if (e != cudaSuccess) return e;
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(CL, 1, 1);
-        cfg.blockDim = dim3(NT, 1, 1);
-        cfg.dynamicSmemBytes = STEP3D_SMEM;
-        cudaLaunchAttribute attr;
-        attr.id = cudaLaunchAttributeClusterDimension;
-        attr.val.clusterDim.x = CL;
-        attr.val.clusterDim.y = 1;
-        attr.val.clusterDim.z = 1;
-        cfg.attrs = &attr;
-        cfg.numAttrs = 1;
         int nclusters = 0;
-        e = cudaOccupancyMaxActiveClusters(&nclusters, k_chain3d, &cfg);
+        e = resident_clusters(&nclusters);
         if (e != cudaSuccess) return e;
         return nclusters > 0 ? cudaSuccess : cudaErrorNotSupported;
     }
