@@ -1191,9 +1191,11 @@ static int autotune_axes(scft_ctx *c)
                 pa.even = A.even;
                 const int nt = A.tc ? 0 : (int)(lines / t);
                 if (A.tc) adopt(t);
+                /* tensor-core passes overlap their neighbours' ends, so they are timed in
+                 * whole steps, with the other axes as they are so far */
                 auto launch = [&]() {
-                    return A.tc ? scft_launch_pass_tc(c->opt.precision, A.t, pa, c->stream)
-                                : scft_launch_pass(c->opt.precision, A.g, pa, nt, c->stream);
+                    if (!A.tc) return scft_launch_pass(c->opt.precision, A.g, pa, nt, c->stream);
+                    return launch_steps(c, c->chains, total, std::min(c->maxlen, 5)) == SCFT_OK ? cudaSuccess : cudaErrorUnknown;
                 };
                 cudaError_t e = launch(); /* warm-up */
                 if (e == cudaSuccess) e = cudaEventRecord(e0, c->stream);

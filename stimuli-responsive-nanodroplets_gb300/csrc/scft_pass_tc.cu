@@ -58,6 +58,7 @@
 #include "scft_dfloat.cuh"
 #include "scft_internal.h"
 #include "scft_mbar.cuh"
+#include "scft_pdl.cuh"
 
 /* Set when a tensor-core wait of a pass gave up (the tile is then written as NaN). */
 __device__ int g_scft_pass_fault;
@@ -719,6 +720,8 @@ __device__ __forceinline__ void tc_tile(const TcGeom &g, const P *src, P *dst, c
     sync();
     ph.ok = *reinterpret_cast<volatile int *>(smem + SM_FAIL) == 0;
 
+    if (!SPLIT) pdl_trigger(); /* the next pass' CTAs may set themselves up where there is room */
+
     /* ---- products, and the levels joined in registers */
     using Acc = typename std::conditional<std::is_same<P, float>::value, float, long long>::type;
     const int nc = min(c1, (hb + W - 1) / W) - c0, ks = g.hp / 16;
@@ -897,15 +900,22 @@ template <typename P, int NB>
 __global__ void __launch_bounds__(256, 2) k_pass_tc(TcGeom g, PassArgs a)
 {
     const ChainDesc cd = a.chains[blockIdx.y];
-    if (a.s >= cd.len - 1) return; /* uniform over the CTA */
-    if (a.state && a.state[cd.instance].done) return;
+    const bool active = a.s < cd.len - 1; /* uniform over the CTA */
 
     extern __shared__ __align__(128) unsigned char smem[];
     const int part = blockIdx.x % g.parts, tile_i = blockIdx.x / g.parts;
     tc_begin(smem, 1);
     const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(smem), bar_op = sbase + SM_BAR;
-    if (threadIdx.x == 32) /* in flight until the products need them */
+    if (active && threadIdx.x == 32) /* in flight until the products need them */
         tc_start_op<P, NB>(g, cd.ops->tc[a.axis], part, sbase + SM_OP, bar_op);
+    /* what is read up to here no kernel writes. Every CTA waits, so that a pass ends after the
+     * one before it */
+    pdl_wait();
+    if (!active) return;
+    if (a.state && a.state[cd.instance].done) {
+        mbar_wait(bar_op, 0); /* for its own copy */
+        return;
+    }
     const P *src = a.first ? reinterpret_cast<const P *>(cd.q) + (long)a.s * a.sstride
                            : reinterpret_cast<const P *>(cd.tmp);
     P *dst = a.last ? reinterpret_cast<P *>(cd.q) + (long)(a.s + 1) * a.sstride : reinterpret_cast<P *>(cd.tmp);
@@ -933,14 +943,13 @@ __global__ void __launch_bounds__(512, 1) k_chain_tc(const __grid_constant__ TcL
     const int rank = blockIdx.x % lp.cluster, slot = blockIdx.x / lp.cluster; /* clusters are consecutive blocks */
     const StepRange run = step_range(a, slot);
     const ChainDesc cd = a.chains[run.chain];
-    if (a.state && a.state[cd.instance].done) return; /* uniform over the cluster */
     const int s_end = run.s_end < cd.len - 1 ? run.s_end : cd.len - 1;
-    if (run.s >= s_end) return;
+    const bool any = run.s < s_end; /* uniform over the cluster */
 
     extern __shared__ __align__(128) unsigned char smem[];
     tc_begin(smem, lp.nax);
     const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(smem);
-    if (threadIdx.x == 32)
+    if (any && threadIdx.x == 32)
         for (int ax = 0; ax < lp.nax; ++ax) {
             const TcGeom &g = lp.g[ax];
             if (rank / g.parts >= lp.slots[ax] || (long)(rank / g.parts) * g.tile >= g.lines) continue;
@@ -949,11 +958,20 @@ __global__ void __launch_bounds__(512, 1) k_chain_tc(const __grid_constant__ TcL
             else
                 tc_start_op<P, 2>(g, cd.ops->tc[ax], rank % g.parts, sbase + lp.op_at[ax], sbase + SM_BAR + 8 * ax);
         }
+    pdl_wait();
+    if (!any) return;
+    if (a.state && a.state[cd.instance].done) { /* uniform over the cluster */
+        for (int ax = 0; ax < lp.nax; ++ax) /* its own copies */
+            if (rank / lp.g[ax].parts < lp.slots[ax] && (long)(rank / lp.g[ax].parts) * lp.g[ax].tile < lp.g[ax].lines)
+                mbar_wait(sbase + SM_BAR + 8 * ax, 0);
+        return;
+    }
     TcPhase ph = {0, true};
     const int group = threadIdx.x / (512 / GROUPS);
     const uint32_t tile_at = lp.tile_at + (uint32_t)group * lp.tile_bytes;
 #pragma unroll 1
     for (int s = run.s; s < s_end; ++s) {
+        if (s + 1 == s_end) pdl_trigger();
         const P *bz = reinterpret_cast<const P *>(s < cd.seg_end ? cd.b0 : cd.b1);
 #pragma unroll 1
         for (int ax = 0; ax < lp.nax; ++ax) {
@@ -1002,9 +1020,8 @@ __global__ void __launch_bounds__(512, 1) k_chain2d_tc(const __grid_constant__ T
     const int rank = blockIdx.x % lp.cluster, slot = blockIdx.x / lp.cluster; /* clusters are consecutive blocks */
     const StepRange run = step_range(a, slot);
     const ChainDesc cd = a.chains[run.chain];
-    if (a.state && a.state[cd.instance].done) return; /* uniform over the cluster */
     const int s_end = run.s_end < cd.len - 1 ? run.s_end : cd.len - 1;
-    if (run.s >= s_end) return;
+    const bool any = run.s < s_end; /* uniform over the cluster */
 
     extern __shared__ __align__(128) unsigned char smem[];
     tc_begin(smem, 4); /* operator digits of the two axes, lines of the two axes */
@@ -1014,7 +1031,7 @@ __global__ void __launch_bounds__(512, 1) k_chain2d_tc(const __grid_constant__ T
 #pragma unroll
     for (int ax = 0; ax < 2; ++ax) {
         const TcGeom &g = lp.g[ax];
-        mine[ax] = (long)rank * g.tile < g.lines;
+        mine[ax] = any && (long)rank * g.tile < g.lines;
         /* a line's values, in pairs, and the largest exponent of each 8 of them that one warp sends */
         bytes[ax] = mine[ax] ? (uint32_t)(min((long)g.tile, g.lines - (long)rank * g.tile) * ((g.n + 1) / 2 * 2 * sizeof(P) + (g.n + 7) / 8 * 4)) : 0u;
         if (mine[ax] && threadIdx.x == 32) {
@@ -1024,6 +1041,13 @@ __global__ void __launch_bounds__(512, 1) k_chain2d_tc(const __grid_constant__ T
                 tc_start_op<P, 2>(g, cd.ops->tc[ax], 0, sbase + lp.op_at[ax], bars + 8 * ax);
             asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bars + 16 + 8 * ax), "r"(bytes[ax]) : "memory");
         }
+    }
+    pdl_wait();
+    if (!any) return;
+    if (a.state && a.state[cd.instance].done) { /* uniform over the cluster */
+        for (int ax = 0; ax < 2; ++ax)
+            if (mine[ax]) mbar_wait(bars + 8 * ax, 0); /* its own copies */
+        return;
     }
     /* the first lines: b q_s from global memory */
     if (mine[0]) {
@@ -1045,6 +1069,7 @@ __global__ void __launch_bounds__(512, 1) k_chain2d_tc(const __grid_constant__ T
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 #pragma unroll 1
     for (int s = run.s; s < s_end; ++s) {
+        if (s + 1 == s_end) pdl_trigger();
         const P *bz = reinterpret_cast<const P *>(s < cd.seg_end ? cd.b0 : cd.b1);
 #pragma unroll 1
         for (int ax = 0; ax < 2; ++ax) {
@@ -1097,11 +1122,7 @@ static cudaError_t launch_tc(const TcGeom &g, const PassArgs &a, cudaStream_t st
     const size_t smem = SM_OP + g.op_part + tile_bytes(g, Dig<P>::S, 16);
     const dim3 grid((unsigned)((g.lines + g.tile - 1) / g.tile * g.parts), a.nchains);
     if (g.tile < 8 || g.tile % 8 || g.tile > ROWS) return cudaErrorInvalidValue;
-    if (g.nb == 4)
-        k_pass_tc<P, 4><<<grid, 256, smem, st>>>(g, a);
-    else
-        k_pass_tc<P, 2><<<grid, 256, smem, st>>>(g, a);
-    return cudaGetLastError();
+    return g.nb == 4 ? pdl_launch(k_pass_tc<P, 4>, grid, 256, smem, st, g, a) : pdl_launch(k_pass_tc<P, 2>, grid, 256, smem, st, g, a);
 }
 
 int scft_pass_tc_fits(int prec, const TcGeom &g, int smem_limit)
@@ -1150,13 +1171,15 @@ static cudaError_t launch_chain(const TcLoop &lp, const Step2DArgs &a, int nchai
     cfg.blockDim = dim3(512, 1, 1);
     cfg.dynamicSmemBytes = scft_chain_tc_layout(prec, l);
     cfg.stream = st;
-    cudaLaunchAttribute attr;
-    attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = lp.cluster;
-    attr.val.clusterDim.y = 1;
-    attr.val.clusterDim.z = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = lp.cluster;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 2;
     if (lp.exchange) {
         if (clusters) return cudaOccupancyMaxActiveClusters(clusters, k_chain2d_tc<P>, &cfg);
         return cudaLaunchKernelEx(&cfg, k_chain2d_tc<P>, l, a);

@@ -12,6 +12,7 @@
 
 #include "scft_dfloat.cuh"
 #include "scft_internal.h"
+#include "scft_pdl.cuh"
 
 #define POST_THREADS 256
 #define DENSITY_THREADS 64
@@ -49,6 +50,8 @@ __device__ void block_sum(double (&v)[NV], double *sh)
 /* ---------------------------------------------------------- iteration begin */
 __global__ void k_iter_begin(PostArgs a)
 {
+    pdl_wait();
+    pdl_trigger();
     const int b = blockIdx.x * blockDim.x + threadIdx.x;
     if (b < a.B) {
         a.state[b].tick += 1;
@@ -92,6 +95,8 @@ __device__ __forceinline__ P boltz(double ds, double w)
 template <typename P>
 __global__ void k_boltz_init(PostArgs a)
 {
+    pdl_wait();
+    pdl_trigger();
     const int b = blockIdx.y;
     if (a.state[b].done) return;
     const InstParams &ip = a.params[b];
@@ -317,6 +322,7 @@ __global__ void __launch_bounds__(DENSITY_THREADS) k_density(PostArgs a)
     constexpr int V = sizeof(P) == 4 ? 4 : 2;
     using Acc = typename AccOf<P>::T;
     const int blk = blockIdx.y, b = blockIdx.z;
+    pdl_wait();
     if (a.state[b].done) return;
     if (blk >= a.nblocks) {
         if (blockIdx.x < a.qparts) q_partial<P, V>(a, b, a.q_species[blk - a.nblocks]);
@@ -531,6 +537,7 @@ __global__ void __launch_bounds__(UPDATE_THREADS, (NA <= 4 ? 6 : 4)) k_update(Po
     __shared__ double pavgA[NA], cA[NA], eA[NA]; /* row sums of chi, of chi . phi_avg */
     __shared__ int actf[NA], p0[NA], p1[NA];
     const int b = blockIdx.y;
+    pdl_wait();
     if (a.state[b].done) {
         /* frozen: repeat the converging iteration's record */
         const long slot = (long)a.state[b].tick - 1;
@@ -636,6 +643,7 @@ __global__ void __launch_bounds__(UPDATE_THREADS, (NA <= 4 ? 6 : 4)) k_update(Po
         acc[1] += pn;
         acc[2] += (tot - 1.0) * (tot - 1.0);
     }
+    pdl_trigger();
     block_sum<3>(acc, sh);
     if (threadIdx.x == 0) {
         double *pp = a.upd_partial + ((long)b * gridDim.x + blockIdx.x) * 3;
@@ -650,6 +658,8 @@ __global__ void __launch_bounds__(UPDATE_THREADS, (NA <= 4 ? 6 : 4)) k_update(Po
 __global__ void k_p_shift(PostArgs a)
 {
     const int b = blockIdx.y;
+    pdl_wait();
+    pdl_trigger();
     if (a.state[b].done == 1) return;
     const double pavg = a.state[b].p_avg;
     double *p = a.w + ((long)b * 14 + 13) * a.sm;
@@ -667,18 +677,15 @@ static int grid_for(long m, int threads, int cap)
 
 cudaError_t scft_post_iter_begin(const PostArgs &a, int prec, int sms, cudaStream_t st)
 {
-    k_iter_begin<<<(a.B + 127) / 128, 128, 0, st>>>(a);
+    cudaError_t e = pdl_launch(k_iter_begin, dim3((a.B + 127) / 128), 128, 0, st, a);
+    if (e != cudaSuccess) return e;
     dim3 g(grid_for(a.m, POST_THREADS, 4 * sms), a.B, 1);
     if ((long)g.x * a.B < sms) {
         for (unsigned u = a.field_use; u; u &= u - 1) ++g.z; /* and the initial slices */
     }
-    if (prec == SCFT_PREC_FP64)
-        k_boltz_init<double><<<g, POST_THREADS, 0, st>>>(a);
-    else if (prec == SCFT_PREC_FP32X2)
-        k_boltz_init<dfloat><<<g, POST_THREADS, 0, st>>>(a);
-    else
-        k_boltz_init<float><<<g, POST_THREADS, 0, st>>>(a);
-    return cudaGetLastError();
+    if (prec == SCFT_PREC_FP64) return pdl_launch(k_boltz_init<double>, g, POST_THREADS, 0, st, a);
+    if (prec == SCFT_PREC_FP32X2) return pdl_launch(k_boltz_init<dfloat>, g, POST_THREADS, 0, st, a);
+    return pdl_launch(k_boltz_init<float>, g, POST_THREADS, 0, st, a);
 }
 
 cudaError_t scft_post_mark_start(const PostArgs &a, cudaStream_t st)
@@ -704,13 +711,9 @@ int scft_post_nparts(long m, int sms) { return grid_for(m, UPDATE_THREADS, 4 * s
 cudaError_t scft_density_launch(const PostArgs &a, int prec, int sms, cudaStream_t st)
 {
     dim3 gd(density_grid(a.m, prec, sms), a.nblocks + a.nq_species, a.B);
-    if (prec == SCFT_PREC_FP64)
-        k_density<double><<<gd, DENSITY_THREADS, 0, st>>>(a);
-    else if (prec == SCFT_PREC_FP32X2)
-        k_density<dfloat><<<gd, DENSITY_THREADS, 0, st>>>(a);
-    else
-        k_density<float><<<gd, DENSITY_THREADS, 0, st>>>(a);
-    return cudaGetLastError();
+    if (prec == SCFT_PREC_FP64) return pdl_launch(k_density<double>, gd, DENSITY_THREADS, 0, st, a);
+    if (prec == SCFT_PREC_FP32X2) return pdl_launch(k_density<dfloat>, gd, DENSITY_THREADS, 0, st, a);
+    return pdl_launch(k_density<float>, gd, DENSITY_THREADS, 0, st, a);
 }
 
 cudaError_t scft_post_iter_end(const PostArgs &a, int prec, int sms, cudaStream_t st)
@@ -721,24 +724,24 @@ cudaError_t scft_post_iter_end(const PostArgs &a, int prec, int sms, cudaStream_
     {
         const dim3 gu(gp, a.B);
         switch (a.n_active) {
-        case 1: k_update<1><<<gu, UPDATE_THREADS, 0, st>>>(a); break;
-        case 2: k_update<2><<<gu, UPDATE_THREADS, 0, st>>>(a); break;
-        case 3: k_update<3><<<gu, UPDATE_THREADS, 0, st>>>(a); break;
-        case 4: k_update<4><<<gu, UPDATE_THREADS, 0, st>>>(a); break;
-        case 5: k_update<5><<<gu, UPDATE_THREADS, 0, st>>>(a); break;
-        case 6: k_update<6><<<gu, UPDATE_THREADS, 0, st>>>(a); break;
-        case 7: k_update<7><<<gu, UPDATE_THREADS, 0, st>>>(a); break;
-        case 8: k_update<8><<<gu, UPDATE_THREADS, 0, st>>>(a); break;
-        case 9: k_update<9><<<gu, UPDATE_THREADS, 0, st>>>(a); break;
-        case 10: k_update<10><<<gu, UPDATE_THREADS, 0, st>>>(a); break;
-        case 11: k_update<11><<<gu, UPDATE_THREADS, 0, st>>>(a); break;
-        case 12: k_update<12><<<gu, UPDATE_THREADS, 0, st>>>(a); break;
-        case 13: k_update<13><<<gu, UPDATE_THREADS, 0, st>>>(a); break;
+        case 1: e = pdl_launch(k_update<1>, gu, UPDATE_THREADS, 0, st, a); break;
+        case 2: e = pdl_launch(k_update<2>, gu, UPDATE_THREADS, 0, st, a); break;
+        case 3: e = pdl_launch(k_update<3>, gu, UPDATE_THREADS, 0, st, a); break;
+        case 4: e = pdl_launch(k_update<4>, gu, UPDATE_THREADS, 0, st, a); break;
+        case 5: e = pdl_launch(k_update<5>, gu, UPDATE_THREADS, 0, st, a); break;
+        case 6: e = pdl_launch(k_update<6>, gu, UPDATE_THREADS, 0, st, a); break;
+        case 7: e = pdl_launch(k_update<7>, gu, UPDATE_THREADS, 0, st, a); break;
+        case 8: e = pdl_launch(k_update<8>, gu, UPDATE_THREADS, 0, st, a); break;
+        case 9: e = pdl_launch(k_update<9>, gu, UPDATE_THREADS, 0, st, a); break;
+        case 10: e = pdl_launch(k_update<10>, gu, UPDATE_THREADS, 0, st, a); break;
+        case 11: e = pdl_launch(k_update<11>, gu, UPDATE_THREADS, 0, st, a); break;
+        case 12: e = pdl_launch(k_update<12>, gu, UPDATE_THREADS, 0, st, a); break;
+        case 13: e = pdl_launch(k_update<13>, gu, UPDATE_THREADS, 0, st, a); break;
         default: return cudaErrorInvalidValue;
         }
     }
-    k_p_shift<<<dim3(grid_for(a.m, POST_THREADS, 4 * sms), a.B), POST_THREADS, 0, st>>>(a);
-    return cudaGetLastError();
+    if (e != cudaSuccess) return e;
+    return pdl_launch(k_p_shift, dim3(grid_for(a.m, POST_THREADS, 4 * sms), a.B), POST_THREADS, 0, st, a);
 }
 
 /* ----------------------------------------------------- unit-entry helpers */
