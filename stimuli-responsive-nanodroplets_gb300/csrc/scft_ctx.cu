@@ -235,26 +235,26 @@ static void dense_operator(int n, double alpha, int dirichlet, std::vector<long 
             const double kz = kval(m, N);
             E[m] = expl(-(long double)alpha * (long double)kz * (long double)kz);
         }
-        for (int d = 0; d < N; ++d) cs[d] = cosl(pi * d / L);
-        for (int d = 0; d < N; ++d) {
+        for (int d = 0; d <= L; ++d) cs[d] = cs[(N - d) % N] = cosl(pi * d / L);
+        for (int d = 0; d <= L; ++d) {
             long double s = 0.0L;
             for (int m = 1; m <= n; ++m) s += E[m] * cs[(m * d) % N];
-            f[d] = s / L;
+            f[d] = f[(N - d) % N] = s / L;
         }
         for (int a = 0; a < n; ++a)
             for (int b = 0; b < n; ++b) K[(size_t)a * n + b] = f[a < b ? b - a : a - b] - f[a + b + 2];
     } else {
         /* circulant: K[i][j] = (1/n) sum_t E_t cos(2 pi t (i-j) / n) */
         std::vector<long double> c(n), E(n), cs(n);
-        for (int t = 0; t < n; ++t) {
+        for (int t = 0; t <= n / 2; ++t) { /* modes t and n - t are one */
             const double k = kval(t, n);
-            E[t] = expl(-(long double)alpha * k * k);
-            cs[t] = cosl(2.0L * pi * t / n);
+            E[t] = expl(-(long double)alpha * k * k) * (t == 0 || 2 * t == n ? 1 : 2);
+            cs[t] = cs[(n - t) % n] = cosl(2.0L * pi * t / n);
         }
-        for (int d = 0; d < n; ++d) {
+        for (int d = 0; d <= n / 2; ++d) {
             long double s = 0.0L;
-            for (int t = 0; t < n; ++t) s += E[t] * cs[(t * d) % n];
-            c[d] = s / n;
+            for (int t = 0; t <= n / 2; ++t) s += E[t] * cs[(t * d) % n];
+            c[d] = c[(n - d) % n] = s / n;
         }
         for (int i = 0; i < n; ++i)
             for (int j = 0; j < n; ++j) K[(size_t)i * n + j] = c[(i - j + n) % n];
