@@ -203,7 +203,7 @@ def measure_form(srn, surfaces, precision: str, steps: int, warmup: int, device:
         "threads_per_line": int(t["threads_per_line"]),
         "kernel": {1: f"k_chain2d<float,{sv.grid[0]},{sv.grid[2]}> (persistent fused contour loop)",
                    2: "k_chain3d (64^3 contour loop, one 8-CTA cluster per chain)"}.get(
-                       t["fused_chain"], "k_pass_fft + k_pass_dense (per-axis passes)"),
+                       t["fused_chain"], "k_pass_tc / k_chain_tc / k_chain2d_tc (axis contractions on the tensor cores)"),
     }
     res["achieved_gbs"] = bytes_iter * B / (t["prop_ms"] * 1e-3 / steps) / 1e9
     # end to end through the C ABI with pinned host buffers: per step the restart

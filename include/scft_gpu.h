@@ -115,7 +115,7 @@ typedef struct scft_options {
     int autotune;    /* 1 (default): time the launch forms on the context's own chains at
                         creation and keep the fastest (cached per shape and batch size): per-axis
                         pass tiles, passes as launches or as one loop, the fused 2D loop's one or
-                        two threads per line; 0: heuristics.
+                        two threads per line or several CTAs per chain; 0: heuristics.
                         Every candidate gives bit-identical results. The timing is taken with the
                         context alone on the GPU: contexts whose iterations are kept in flight side
                         by side (pipelined parts of one batch, serving pools) run better on the

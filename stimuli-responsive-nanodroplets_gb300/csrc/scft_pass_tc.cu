@@ -39,12 +39,12 @@
  * 8-48 of the 64 rows. 192x96 film, FP64, 32 instances: 16.3 ms an iteration
  * against 12.7; 64^3 blend: 18.4 against 14.3. The passes are bound by the
  * integer pipe (splitting, joining: ~100 operations per value, 2 issue slots
- * each) and by the rate of mma.sync (16 clocks each).
+ * each) and by the rate of mma.sync (~13 clocks each on an SM quarter).
  * Measured against the FP64 and double-float passes (FFT along periodic axes,
  * dense products along the others), ms per iteration, contour steps and all:
- * 192x96 film, one FP64 instance 4.36 -> 1.49, 32 FP64 instances 45.8 -> 12.7,
- * 16 FP32x2 instances 11.4 -> 6.1; 64^3 four-diblock blend, FP64, 55.9 -> 15.2;
- * 150x75 film, FP32, 4 instances 2.65 -> 1.8. Errors against 64-bit references
+ * 192x96 film, one FP64 instance 4.36 -> 1.15, 32 FP64 instances 46.5 -> 10.9,
+ * 16 FP32x2 instances 11.4 -> 5.8; 64^3 four-diblock blend, FP64, 56.0 -> 14.1;
+ * 150x75 film, FP32, 4 instances 2.65 -> 1.22. Errors against 64-bit references
  * are no larger than before in every form.
  *
  * A line with a NaN or an infinity comes out as NaN.

@@ -19,6 +19,10 @@
  * instance that is active at contour step s; the first pass multiplies by b
  * on load, the last multiplies by b on store and writes slice s+1.
  *
+ * Lengths of 8 and more whose operator fits in shared memory are contracted on
+ * the tensor cores instead (scft_pass_tc.cu); this file serves the others, and the
+ * 64^3 FP32 grid where its cluster cannot be scheduled.
+ *
  * The kernels are written once over the value type P: double (plain form),
  * float (per-axis passes of the FP32 form) and dfloat (the FP32x2 form: slices,
  * Boltzmann factors and operator tables stored as FP32 pairs, every operation

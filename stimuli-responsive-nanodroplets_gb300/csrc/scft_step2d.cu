@@ -1543,8 +1543,7 @@ static cudaError_t launch_t(const Step2DArgs &a, int nblocks, cudaStream_t st, i
 
 /* Returns the shared-memory bytes of the fused step for (nx, nz) in this
  * precision, or 0 if the shape has no fused kernel. Only the FP32 form has
- * one: an FP64 or double-float row pair does not fit in registers, and those
- * forms are bound by arithmetic, so they keep the per-axis passes. */
+ * one: the others run the loops of scft_pass_tc.cu. */
 size_t scft_step2d_smem(int prec, int nx, int nz)
 {
 #define X(NX_, NZ_, A_, B_)                                                                                           \
