@@ -310,12 +310,13 @@ __device__ __forceinline__ void q_partial(const PostArgs &a, int b, int sp)
     if (last_cta(&a.table[b].q_arrived, (unsigned)(a.qparts * a.nq_species))) prepare_update(a, b);
 }
 
-/* CTAs of 64 threads: a small grid's FP64 sums spread over four times as many SMs.
- * Both contour loops run together, for more slices in flight per thread; the rows of
- * Q take no launch of their own. 256 films of 192x96 in FP32, bounded by the slices
- * read from HBM: densities and Q 1794 -> 1768 us (in launches for all 17 species, Q
- * took 275 of them); one 32x16 film, bounded by latency and launches: with the update
- * below, 341 -> 307 us an iteration. */
+/* CTAs of 64 threads: a small grid's FP64 sums spread over four times as many SMs;
+ * the rows of Q take no launch of their own. 256 films of 192x96 in FP32 are bounded
+ * by the slices read from HBM, 4 iterations in all: 38.4 ms with launches for Q of all
+ * 17 species, 38.3 with both contour loops of a block run together (more slices in
+ * flight a thread, but longer strides between a warp's loads), 37.3 like this. One
+ * 32x16 film, bounded by latency and launches: with the update below, 341 -> 307 us
+ * an iteration. */
 template <typename P>
 __global__ void __launch_bounds__(DENSITY_THREADS) k_density(PostArgs a)
 {
@@ -356,25 +357,19 @@ __global__ void __launch_bounds__(DENSITY_THREADS) k_density(PostArgs a)
             load_p<P, V>(qf + (long)top * a.sm + idx, y);
 #pragma unroll
             for (int v = 0; v < V; ++v) e2[v].add(x[v], y[v]);
-            int s = 1;
 #pragma unroll 4
-            for (; s + 1 < mid; s += 2) {
-                P x2[V], y2[V];
-                load_p<P, V>(qf + (long)s * a.sm + idx, x);
-                load_p<P, V>(qf + (long)(top - s) * a.sm + idx, y);
-                load_p<P, V>(qf + (long)(s + 1) * a.sm + idx, x2);
-                load_p<P, V>(qf + (long)(top - s - 1) * a.sm + idx, y2);
-#pragma unroll
-                for (int v = 0; v < V; ++v) {
-                    h4[v].add(x[v], y[v]);
-                    h2[v].add(x2[v], y2[v]);
-                }
-            }
-            if (s < mid) {
+            for (int s = 1; s < mid; s += 2) {
                 load_p<P, V>(qf + (long)s * a.sm + idx, x);
                 load_p<P, V>(qf + (long)(top - s) * a.sm + idx, y);
 #pragma unroll
                 for (int v = 0; v < V; ++v) h4[v].add(x[v], y[v]);
+            }
+#pragma unroll 4
+            for (int s = 2; s < mid; s += 2) {
+                load_p<P, V>(qf + (long)s * a.sm + idx, x);
+                load_p<P, V>(qf + (long)(top - s) * a.sm + idx, y);
+#pragma unroll
+                for (int v = 0; v < V; ++v) h2[v].add(x[v], y[v]);
             }
             if (mid > 0) {
                 load_p<P, V>(qf + (long)mid * a.sm + idx, x);
@@ -402,25 +397,19 @@ __global__ void __launch_bounds__(DENSITY_THREADS) k_density(PostArgs a)
             load_p<P, V>(qb + (long)(top - bd.stop) * a.sm + idx, y);
 #pragma unroll
             for (int v = 0; v < V; ++v) ends[v].add(x[v], y[v]);
-            int s = bd.start + 1;
 #pragma unroll 4
-            for (; s + 1 <= bd.stop - 2; s += 2) {
-                P x2[V], y2[V];
-                load_p<P, V>(qf + (long)s * a.sm + idx, x);
-                load_p<P, V>(qb + (long)(top - s) * a.sm + idx, y);
-                load_p<P, V>(qf + (long)(s + 1) * a.sm + idx, x2);
-                load_p<P, V>(qb + (long)(top - s - 1) * a.sm + idx, y2);
-#pragma unroll
-                for (int v = 0; v < V; ++v) {
-                    a4[v].add(x[v], y[v]);
-                    a2[v].add(x2[v], y2[v]);
-                }
-            }
-            if (s <= bd.stop - 1) {
+            for (int s = bd.start + 1; s <= bd.stop - 1; s += 2) {
                 load_p<P, V>(qf + (long)s * a.sm + idx, x);
                 load_p<P, V>(qb + (long)(top - s) * a.sm + idx, y);
 #pragma unroll
                 for (int v = 0; v < V; ++v) a4[v].add(x[v], y[v]);
+            }
+#pragma unroll 4
+            for (int s = bd.start + 2; s <= bd.stop - 2; s += 2) {
+                load_p<P, V>(qf + (long)s * a.sm + idx, x);
+                load_p<P, V>(qb + (long)(top - s) * a.sm + idx, y);
+#pragma unroll
+                for (int v = 0; v < V; ++v) a2[v].add(x[v], y[v]);
             }
 #pragma unroll
             for (int v = 0; v < V; ++v) out[idx + v] = ends[v].value() + 4.0 * a4[v].value() + 2.0 * a2[v].value();
