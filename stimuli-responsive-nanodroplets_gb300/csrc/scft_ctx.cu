@@ -1055,21 +1055,40 @@ static double tc_loop_plan(const scft_ctx *c, int cluster, int smem_limit, TcLoo
 }
 
 /* The 2D form with one tile per CTA and axis: nothing to choose but the cluster. */
-static double tc_exchange_plan(const scft_ctx *c, int cluster, int smem_limit, TcLoop &lp)
+static double tc_exchange_plan(int prec, const TcGeom &g0, const TcGeom &g1, int cluster, int smem_limit, TcLoop &lp)
 {
-    const int prec = c->opt.precision;
     memset(&lp, 0, sizeof(lp));
     lp.nax = 2;
     lp.cluster = cluster;
     lp.exchange = 1;
     double cost = 0.0;
     for (int ax = 0; ax < 2; ++ax) {
-        lp.g[ax] = c->axes[ax].t;
+        lp.g[ax] = ax ? g1 : g0;
         const int tile = (int)(((lp.g[ax].lines + cluster - 1) / cluster + 7) / 8 * 8);
         if (tile > 128 || !tc_apply(prec, lp.g[ax], tile, 1, smem_limit)) return -1.0;
         cost += tc_cta_cost(lp.g[ax], prec, 512, 1);
     }
     return scft_chain_tc_layout(prec, lp) <= (size_t)smem_limit ? cost : -1.0;
+}
+
+/* Test hook: the shared memory of a 2D loop with one tile per CTA and axis in clusters of
+ * `cluster`. at[ax][k], k = 0 .. 3: first byte and end of the axis' digits, then of its
+ * block sums; `*bytes`: in all. 1 where the loop does not fit. */
+extern "C" int scft_tc_exchange_layout(int prec, int nx, int nz, int wall, int cluster, long at[2][4], long *bytes)
+{
+    if (nx < 2 || nz < 2 || cluster < 1 || !at || !bytes) return SCFT_ERR_PARAM;
+    TcGeom g[2];
+    tc_shape(nx, 0, g[0]);
+    tc_shape(nz, wall, g[1]);
+    g[0].ls = g[0].inner = nz;
+    g[1].ls = g[1].inner = 1;
+    g[0].lines = nz;
+    g[1].lines = nx;
+    TcLoop lp;
+    if (tc_exchange_plan(prec, g[0], g[1], cluster, 232448, lp) < 0.0) return 1;
+    *bytes = (long)scft_chain_tc_layout(prec, lp);
+    for (int ax = 0; ax < 2; ++ax) scft_chain_tc_regions(prec, lp, ax, at[ax]);
+    return SCFT_OK;
 }
 
 struct LoopChoice {
@@ -1080,7 +1099,8 @@ struct LoopChoice {
 static bool tc_loop_make(const scft_ctx *c, int cluster, int exchange, int smem_limit, LoopChoice &ch)
 {
     if (exchange && c->axes.size() != 2) return false;
-    const double per = exchange ? tc_exchange_plan(c, cluster, smem_limit, ch.lp) : tc_loop_plan(c, cluster, smem_limit, ch.lp);
+    const double per = exchange ? tc_exchange_plan(c->opt.precision, c->axes[0].t, c->axes[1].t, cluster, smem_limit, ch.lp)
+                                : tc_loop_plan(c, cluster, smem_limit, ch.lp);
     ch.cost = per * (c->maxlen - 1);
     ch.resident = 0;
     return per >= 0.0;

@@ -158,6 +158,7 @@ struct TcLoop {
     int slots[3];      /* tiles taken side by side: cluster / parts */
     unsigned op_at[3]; /* shared-memory offsets of the axes' operator digits and of the tile region */
     unsigned tile_at, tile_bytes;
+    unsigned ex_at; /* exchange: block sums, behind the digits of either axis */
     /* exchange: the axes' lines in shared memory, values from line to line, ceil(2^32 / tile) */
     unsigned buf_at[2], mag_tile[2];
     int pitch[2];
@@ -169,6 +170,7 @@ cudaError_t scft_pass_tc_configure(int smem_bytes);
 cudaError_t scft_launch_pass_tc(int prec, const TcGeom &g, const PassArgs &a, cudaStream_t st);
 struct Step2DArgs;
 size_t scft_chain_tc_layout(int prec, TcLoop &lp);
+void scft_chain_tc_regions(int prec, const TcLoop &lp, int ax, long at[4]);
 cudaError_t scft_launch_chain_tc(int prec, const TcLoop &lp, const Step2DArgs &a, int nchains, cudaStream_t st,
                                  int *clusters);
 /* 1 if a tensor-core wait of a pass gave up since the last call (clears it) */

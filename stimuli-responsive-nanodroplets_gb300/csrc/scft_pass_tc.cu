@@ -450,7 +450,8 @@ constexpr int EBITS = 11; /* bits of an exponent */
  * shared memory to lines of the other axis in their CTAs' shared memory. */
 template <typename P, int NB, int NT>
 __device__ __forceinline__ void tc_tile2d(const TcGeom &g, const Exchange<P> &xc, bool last, int tile_i, unsigned char *smem,
-                                          uint32_t sm_op, uint32_t sm_a, uint32_t bar_op, bool wait_op, bool &ok)
+                                          uint32_t sm_op, uint32_t sm_a, uint32_t sm_ex, uint32_t bar_op, bool wait_op,
+                                          bool &ok)
 {
     constexpr int S = Dig<P>::S, L = Dig<P>::L, CELL = S * NB * 128;
     using Fix = typename FixT<P>::T;
@@ -495,7 +496,7 @@ __device__ __forceinline__ void tc_tile2d(const TcGeom &g, const Exchange<P> &xc
 
     /* ---- products, 16 outputs x 8 lines of one block at a time */
     using Acc = typename std::conditional<std::is_same<P, float>::value, float, long long>::type;
-    Acc *ex = reinterpret_cast<Acc *>(smem + sm_a + tile_bytes(g, S, 8));
+    Acc *ex = reinterpret_cast<Acc *>(smem + sm_ex);
     const int pitch = nc * W * NB + 4; /* values of a line: block by block, shifted by four from line to line */
     const int nr = (nlines + 7) / 8, np = (nc + 1) / 2, ks = g.hp / 16;
 #pragma unroll 1
@@ -1002,11 +1003,20 @@ __global__ void __launch_bounds__(512, 1) k_chain_tc(const __grid_constant__ TcL
  * other axis it belongs to (st.async), with the largest exponent of the 8 lines a
  * warp sends, and that CTA waits for its bytes on its own barrier. No CTA waits
  * for stores to reach L2, for a cluster barrier and for the loads after it, nor
- * looks for a line's largest value. A line of one axis has a point of every line
- * of the other, so a CTA can only be sent lines again once all CTAs, itself
- * included, have sent what they made of the last ones: one buffer per axis is
- * enough. Only q_{s+1} goes to global memory, for the densities; what is sent
+ * looks for a line's largest value. Only q_{s+1} goes to global memory, for the densities; what is sent
  * after the last axis is b q_{s+1} already.
+ *
+ * A CTA's lines of an axis are complete when every CTA has sent the points of them;
+ * warps whose outputs go elsewhere may still be at work, there and in the CTA
+ * itself. What orders each write to a buffer after the last read of what it held:
+ *   - lines of an axis are read into digits before the tile's first CTA barrier; a CTA
+ *     sends points of the next ones only after it has received its lines of the other
+ *     axis whole, a point of each of these lines among them, sent after that barrier;
+ *   - digits are read by the products, before the tile's second CTA barrier, and
+ *     written again for the next tile, after it;
+ *   - block sums are read by the outputs and written again by the next tile's products,
+ *     after its first CTA barrier; they lie behind the digits of either axis, which
+ *     warps that have already gone on may be writing.
  *
  * A step is two serial phases of digits, products and outputs, each bounded by
  * the latency of its own instructions on small grids (one item a thread) and on
@@ -1099,9 +1109,9 @@ __global__ void __launch_bounds__(512, 1) k_chain2d_tc(const __grid_constant__ T
                                     reinterpret_cast<const P *>(s + 1 < cd.seg_end ? cd.b0 : cd.b1),
                                     reinterpret_cast<P *>(cd.q) + (long)(s + 1) * a.sstride};
             if (g.nb == 4)
-                tc_tile2d<P, 4, 512>(g, xc, ax == 1, rank, smem, lp.op_at[ax], lp.tile_at, bars + 8 * ax, t == 0, ok);
+                tc_tile2d<P, 4, 512>(g, xc, ax == 1, rank, smem, lp.op_at[ax], lp.tile_at, lp.ex_at, bars + 8 * ax, t == 0, ok);
             else
-                tc_tile2d<P, 2, 512>(g, xc, ax == 1, rank, smem, lp.op_at[ax], lp.tile_at, bars + 8 * ax, t == 0, ok);
+                tc_tile2d<P, 2, 512>(g, xc, ax == 1, rank, smem, lp.op_at[ax], lp.tile_at, lp.ex_at, bars + 8 * ax, t == 0, ok);
         }
     }
     if (!ok && threadIdx.x == 0) atomicExch(&g_scft_pass_fault, 1);
@@ -1141,13 +1151,15 @@ cudaError_t scft_launch_pass_tc(int prec, const TcGeom &g, const PassArgs &a, cu
  * returns its bytes. */
 size_t scft_chain_tc_layout(int prec, TcLoop &lp)
 {
-    uint32_t at = SM_OP, tile = 0;
+    uint32_t at = SM_OP, tile = 0, digits = 0, sums = 0;
     for (int ax = 0; ax < lp.nax; ++ax) {
         lp.op_at[ax] = at;
         at += (lp.g[ax].op_part + 127) / 128 * 128;
         const int S = prec == SCFT_PREC_FP32 ? Dig<float>::S : Dig<double>::S, value = prec == SCFT_PREC_FP32 ? 4 : 8;
-        const uint32_t b = tile_bytes(lp.g[ax], S, 8) + exchange_bytes(lp.g[ax], value);
-        if (b > tile) tile = b;
+        const uint32_t d = (tile_bytes(lp.g[ax], S, 8) + 127) / 128 * 128, e = exchange_bytes(lp.g[ax], value);
+        if (d > digits) digits = d;
+        if (e > sums) sums = e;
+        if (d + e > tile) tile = d + e;
         lp.slots[ax] = lp.cluster / lp.g[ax].parts;
         if (lp.exchange) { /* lines, shifted by half the banks from one to the next */
             lp.pitch[ax] = (lp.g[ax].n + 15) / 16 * 16 + 8;
@@ -1157,8 +1169,18 @@ size_t scft_chain_tc_layout(int prec, TcLoop &lp)
         }
     }
     lp.tile_at = at;
-    lp.tile_bytes = (tile + 127) / 128 * 128;
+    lp.ex_at = at + digits;
+    lp.tile_bytes = ((lp.exchange ? digits + sums : tile) + 127) / 128 * 128;
     return (size_t)at + (lp.exchange ? 1 : GROUPS) * lp.tile_bytes;
+}
+
+/* First byte and end of an axis' digits and of its block sums in the exchange form. */
+void scft_chain_tc_regions(int prec, const TcLoop &lp, int ax, long at[4])
+{
+    at[0] = lp.tile_at;
+    at[1] = at[0] + tile_bytes(lp.g[ax], prec == SCFT_PREC_FP32 ? Dig<float>::S : Dig<double>::S, 8);
+    at[2] = lp.ex_at;
+    at[3] = at[2] + exchange_bytes(lp.g[ax], prec == SCFT_PREC_FP32 ? 4 : 8);
 }
 
 template <typename P>
