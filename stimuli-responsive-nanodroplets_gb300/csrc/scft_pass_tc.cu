@@ -337,9 +337,13 @@ __device__ __forceinline__ void set_nan(double &y) { y = __longlong_as_double(0x
 __device__ __forceinline__ void set_nan(dfloat &y) { y = dfloat(__int_as_float(0x7fc00000), __int_as_float(0x7fc00000)); }
 __device__ __forceinline__ void set_nan(float &y) { y = __int_as_float(0x7fc00000); }
 
-/* Shared memory (byte offsets): one barrier per axis, two sets of line exponents,
- * operator digits (one region per axis), then the digits of a tile's lines. */
+/* Shared memory (byte offsets): one barrier per axis, four sets of line
+ * exponents (two for each group of warps, see k_chain2d_tc for its own), operator
+ * digits (one region per axis), then the digits of a tile's lines. */
 constexpr uint32_t SM_BAR = 0, SM_FAIL = 32, SM_ELINE = 64, SM_OP = SM_ELINE + 4 * ROWS * 4;
+/* k_chain2d_tc: what peers send for an axis, and what the tile in hand keeps of it */
+__host__ __device__ constexpr uint32_t sm_received(int ax) { return SM_ELINE + ax * ROWS * 4; }
+__host__ __device__ constexpr uint32_t sm_kept(int set) { return SM_ELINE + (2 + set) * ROWS * 4; }
 
 /* bytes of a tile's digits (an MMA of a pass reads 16 lines, of the loops 8) */
 __host__ __device__ inline uint32_t tile_bytes(const TcGeom &g, int digits, int lines)
@@ -398,7 +402,8 @@ struct TcPhase {
 template <typename P>
 struct Exchange {
     const P *in;       /* the tile's lines, `pitch` values apart */
-    const int *eline;  /* their largest exponents, below the step's number */
+    const int *eline;  /* their largest exponents, below the step's number; peers write here */
+    int *kept;         /* the tile's copy of them, for its outputs */
     int pitch, tag;    /* tag: the number the receiver expects, in place */
     uint32_t out, out_eline, bar; /* offsets in every CTA's shared memory */
     int out_pitch, out_tile;
@@ -465,6 +470,8 @@ __device__ __forceinline__ void tc_tile2d(const TcGeom &g, const Exchange<P> &xc
         return p == 0 ? k : p == 1 ? m - 1 - k : p == 2 ? k + m : n - 1 - k;
     };
 
+    /* a CTA that has its points may send the next lines while other warps are at this tile's outputs */
+    if (tid < g.tile) xc.kept[tid] = xc.eline[tid] & ((1 << EBITS) - 1);
     /* ---- digits: an item is two neighbouring points and their images of one line */
 #pragma unroll 1
     for (int idx = tid; idx < g.tile * nk8 * 4; idx += NT) {
@@ -522,7 +529,7 @@ __device__ __forceinline__ void tc_tile2d(const TcGeom &g, const Exchange<P> &xc
         const int u = parts == 1 ? w : parts == NB ? w / NB : w / NH, part = parts == 1 ? 0 : w - u * parts;
         const int rg = nr == 1 ? 0 : (int)__umulhi((unsigned)u, g.mag_og), k = (u - rg * og) * 4 + (lane & 3), r = rg * 8 + (lane >> 2);
         const bool in = r < nlines && k < hb;
-        const int em = xc.eline[r] & ((1 << EBITS) - 1);
+        const int em = xc.kept[r];
         const bool bad = em == ExpoMax<P>::v || !ok;
         const int base = g.ls == 1 ? (L0 + r) * n : L0 + r;
         const int odd = (lane >> 2) & 1;
@@ -1016,7 +1023,10 @@ __global__ void __launch_bounds__(512, 1) k_chain_tc(const __grid_constant__ TcL
  *     written again for the next tile, after it;
  *   - block sums are read by the outputs and written again by the next tile's products,
  *     after its first CTA barrier; they lie behind the digits of either axis, which
- *     warps that have already gone on may be writing.
+ *     warps that have already gone on may be writing;
+ *   - the largest exponents sent with the lines are read before the tile's first CTA
+ *     barrier, like the lines; the outputs read a copy of them, of which there are two
+ *     in turn, so that one is written again two tiles on, after the CTA barriers between.
  *
  * A step is two serial phases of digits, products and outputs, each bounded by
  * the latency of its own instructions on small grids (one item a thread) and on
@@ -1038,6 +1048,7 @@ __global__ void __launch_bounds__(512, 1) k_chain2d_tc(const __grid_constant__ T
     const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(smem), bars = sbase + SM_BAR;
     bool mine[2], ok = true;
     uint32_t bytes[2];
+    int tiles = 0; /* tiles done */
 #pragma unroll
     for (int ax = 0; ax < 2; ++ax) {
         const TcGeom &g = lp.g[ax];
@@ -1065,7 +1076,7 @@ __global__ void __launch_bounds__(512, 1) k_chain2d_tc(const __grid_constant__ T
         const P *src = reinterpret_cast<const P *>(cd.q) + (long)run.s * a.sstride;
         const P *bz = reinterpret_cast<const P *>(run.s < cd.seg_end ? cd.b0 : cd.b1);
         P *in = reinterpret_cast<P *>(smem + lp.buf_at[0]);
-        int *eline = reinterpret_cast<int *>(smem + SM_ELINE);
+        int *eline = reinterpret_cast<int *>(smem + sm_received(0));
         const int L0 = rank * g.tile, nlines = (int)min((long)g.tile, g.lines - L0);
         for (int i = threadIdx.x; i < nlines * g.n; i += 512) {
             const int x = i / nlines, r = i - x * nlines; /* lines of the slowest axis: neighbours in memory */
@@ -1095,11 +1106,12 @@ __global__ void __launch_bounds__(512, 1) k_chain2d_tc(const __grid_constant__ T
                     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes[ax]) : "memory");
             }
             const Exchange<P> xc = {reinterpret_cast<const P *>(smem + lp.buf_at[ax]),
-                                    reinterpret_cast<const int *>(smem + SM_ELINE) + ax * ROWS,
+                                    reinterpret_cast<const int *>(smem + sm_received(ax)),
+                                    reinterpret_cast<int *>(smem + sm_kept(tiles++ & 1)),
                                     lp.pitch[ax],
                                     (t + 1 + ax) << EBITS, /* larger than all before: the maxima need no reset */
                                     lp.buf_at[1 - ax],
-                                    SM_ELINE + (1 - ax) * ROWS * 4,
+                                    sm_received(1 - ax),
                                     SM_BAR + 16 + 8 * (1 - ax),
                                     lp.pitch[1 - ax],
                                     o.tile,
@@ -1181,6 +1193,16 @@ void scft_chain_tc_regions(int prec, const TcLoop &lp, int ax, long at[4])
     at[1] = at[0] + tile_bytes(lp.g[ax], prec == SCFT_PREC_FP32 ? Dig<float>::S : Dig<double>::S, 8);
     at[2] = lp.ex_at;
     at[3] = at[2] + exchange_bytes(lp.g[ax], prec == SCFT_PREC_FP32 ? 4 : 8);
+}
+
+/* Test hook: first byte and end of the line exponents in k_chain2d_tc: sent by peers for
+ * either axis, then the two sets that the outputs read. */
+extern "C" void scft_tc_exchange_exponents(long at[4][2])
+{
+    for (int k = 0; k < 4; ++k) {
+        at[k][0] = k < 2 ? sm_received(k) : sm_kept(k - 2);
+        at[k][1] = at[k][0] + ROWS * 4;
+    }
 }
 
 template <typename P>

@@ -30,3 +30,15 @@ def test_sums_behind_the_digits_of_either_axis(srn, grid, wall, prec):
             for o in (x, z):
                 assert a[3] <= o[0] or o[1] <= a[2], (cluster, x, z)
     assert fits or grid[0] * grid[1] > 96 * 64
+
+
+def test_outputs_read_exponents_that_no_peer_writes(srn):
+    """A CTA whose lines of the other axis are complete sends the next exponents while
+    warps of the receiver may still be scaling outputs by the last ones."""
+    f = importlib.import_module(srn.__name__ + "._lib").lib().scft_tc_exchange_exponents
+    f.restype, f.argtypes = None, [C.POINTER(C.c_long)]
+    at = (C.c_long * 8)()
+    f(at)
+    sets = sorted(zip(at[0::2], at[1::2]))
+    assert all(b - a >= 128 * 4 for a, b in sets)
+    assert all(p[1] <= q[0] for p, q in zip(sets, sets[1:]))
