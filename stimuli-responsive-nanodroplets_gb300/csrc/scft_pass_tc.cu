@@ -239,12 +239,15 @@ __device__ __forceinline__ dfloat ld1(const dfloat *p)
     return dfloat(t.x, t.y);
 }
 
-/* factors that no one writes while the kernel runs: they may stay in L1 */
-__device__ __forceinline__ double ldc(const double *p) { return __ldg(p); }
-__device__ __forceinline__ float ldc(const float *p) { return __ldg(p); }
+/* factors that no one writes after pdl_wait(): they may stay in L1. Ordinary loads, as the
+ * kernel can have started while the one before it wrote them: the read-only path
+ * (ld.global.nc, __ldg) wants data that no one writes from a kernel's start on, and neither
+ * the wait nor the compiler orders it */
+__device__ __forceinline__ double ldc(const double *p) { return *p; }
+__device__ __forceinline__ float ldc(const float *p) { return *p; }
 __device__ __forceinline__ dfloat ldc(const dfloat *p)
 {
-    const float2 t = __ldg(reinterpret_cast<const float2 *>(p));
+    const float2 t = *reinterpret_cast<const float2 *>(p);
     return dfloat(t.x, t.y);
 }
 
@@ -601,7 +604,7 @@ __device__ __forceinline__ void tc_tile2d(const TcGeom &g, const Exchange<P> &xc
 /* One tile of lines and one part of its outputs: y = K x (times b before the
  * first axis, after the last). Ends with every thread of the CTA past the digits. */
 template <typename P, int NB, int NT, bool SPLIT>
-__device__ __forceinline__ void tc_tile(const TcGeom &g, const P *src, P *dst, const P *__restrict__ bz,
+__device__ __forceinline__ void tc_tile(const TcGeom &g, const P *src, P *dst, const P *bz,
                                         bool first, bool last, int tile_i, int part, unsigned char *smem,
                                         uint32_t sm_op, uint32_t sm_a, uint32_t bar_op, bool wait_op, TcPhase &ph)
 {

@@ -4,7 +4,8 @@
  * before has triggered or ended, and pdl_wait() returns when that kernel, and all
  * it waited for itself, is complete. Every CTA of such a kernel calls pdl_wait()
  * on every path, so that kernels complete in stream order, and touches nothing
- * that a kernel writes before it. The tensor-core passes load their operator
+ * that a kernel writes before it; nor does it read such data by the read-only path
+ * (__ldg), which takes them as constant from the kernel's start on. The tensor-core passes load their operator
  * digits meanwhile: a 48x32x40 film in FP32x2, three passes of ~10 us a step, 31 ->
  * 24 us; a 64^3 blend in FP64 15.4 -> 14.1 ms an iteration; the launches around
  * the contour loop of a 32x16 film 307 -> 296 us.
