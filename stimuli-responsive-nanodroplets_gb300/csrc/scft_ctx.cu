@@ -119,6 +119,7 @@ struct scft_ctx {
      * them per launch (plan_rounds); empty: one launch */
     std::vector<std::pair<int, int>> rounds; /* first unit, units */
     StepUnit *units = nullptr;
+    int tc_carry = 0; /* tensor-core passes carry between levels: some operator's digits call for it (tc_table) */
     int loop_tc = 0; /* the cluster contour loop on the tensor-core tiles (k_chain_tc) */
     TcLoop loop;
     int *order = nullptr; /* chain indices, longest first */
@@ -682,15 +683,23 @@ static uint16_t half_of_int(int d)
 /* The operator digits of one axis in the layout of k_pass_tc: chunk, block,
  * 16-point step, then rows (digit, output) as K-major 8 x 16-byte core
  * matrices. Entries are integers M 2^kq below 2^(10 sk - 1) in balanced digits
- * of 10 bits, kq = 10 sk - 1 for nb = 2 and 10 sk for nb = 4. */
-static std::vector<uint16_t> tc_table(const std::vector<long double> &K, const TcGeom &g, int sk)
+ * of 10 bits, kq = 10 sk - 1 for nb = 2 and 10 sk for nb = 4.
+ * sums[l], if asked for: the largest sum of level l, over whole rows and over 16 points
+ * of a row, that data digits of up to 512 can make. */
+struct TcSums {
+    double row[6], step[6];
+};
+static std::vector<uint16_t> tc_table(const std::vector<long double> &K, const TcGeom &g, int sk, TcSums *sums = nullptr)
 {
     const std::vector<long double> M = tc_blocks(K, g.n, g.nb, g.hb);
     const int kq = 10 * sk - (g.nb == 4 ? 0 : 1);
     std::vector<uint16_t> T((size_t)g.nb * g.hp * g.nchunks * g.w * sk, 0);
+    if (sums) memset(sums, 0, sizeof(*sums));
     for (int b = 0; b < g.nb; ++b)
-        for (int i = 0; i < g.hb; ++i)
+        for (int i = 0; i < g.hb; ++i) {
+            double row[6] = {0.0}, step16[6];
             for (int j = 0; j < g.hb; ++j) {
+                if (j % 16 == 0) memset(step16, 0, sizeof(step16));
                 long long v = llroundl(ldexpl(M[((size_t)b * g.hb + i) * g.hb + j], kq));
                 const int c = i / g.w, o = i - c * g.w, wc = g.w;
                 const size_t chunk = (size_t)g.nb * g.hp * sk * ((size_t)c * g.w);
@@ -698,11 +707,42 @@ static std::vector<uint16_t> tc_table(const std::vector<long double> &K, const T
                 for (int d = sk - 1; d >= 0; --d) { /* lowest digit first */
                     long long q = d > 0 ? ((v + 512) & 1023) - 512 : v;
                     v = (v - q) >> 10;
-                    const int row = d * wc + o, k = j & 15;
-                    T[step + (size_t)(row / 8) * 128 + (k / 8) * 64 + (row % 8) * 8 + k % 8] = half_of_int((int)q);
+                    const int r = d * wc + o, k = j & 15;
+                    T[step + (size_t)(r / 8) * 128 + (k / 8) * 64 + (r % 8) * 8 + k % 8] = half_of_int((int)q);
+                    row[d] += 512.0 * std::abs((int)q);
+                    step16[d] += 512.0 * std::abs((int)q);
+                }
+                if (sums && (j % 16 == 15 || j + 1 == g.hb)) {
+                    double s = 0.0;
+                    for (int d = 0; d < sk; ++d) sums->step[d] = std::max(sums->step[d], s += step16[d]);
                 }
             }
+            if (sums) {
+                double s = 0.0;
+                for (int d = 0; d < sk; ++d) sums->row[d] = std::max(sums->row[d], s += row[d]);
+            }
+        }
     return T;
+}
+
+/* Levels 0 to 3 of FP64 and FP32x2 must be exact: a unit lost on level 3 is 2^-47 of the
+ * line's largest value. FP32 rounds to 2^-24, sixteen units of its level 1. */
+static bool tc_needs_carry(int prec, const TcSums &s) { return prec != SCFT_PREC_FP32 && s.row[3] > 16777216.0; }
+
+/* Test hook: the bounds of an operator's level sums (TcSums), and whether its passes
+ * carry between levels. */
+extern "C" int scft_tc_level_sums(int n, double alpha, int dirichlet, int prec, double row[6], double step[6])
+{
+    if (n < 2 || !row || !step) return SCFT_ERR_PARAM;
+    TcGeom g;
+    tc_shape(n, dirichlet, g);
+    std::vector<long double> K;
+    dense_operator(n, alpha, dirichlet, K);
+    TcSums s;
+    tc_table(K, g, tc_sk(prec), &s);
+    memcpy(row, s.row, sizeof(s.row));
+    memcpy(step, s.step, sizeof(s.step));
+    return tc_needs_carry(prec, s);
 }
 
 /* Test hook: the operator a tensor-core pass applies, decoded from its digits
@@ -823,7 +863,9 @@ static int axis_tables(scft_ctx *c, const Axis &A, double alpha, InstOps &o, int
         std::vector<long double> K;
         dense_operator(n, alpha, A.dirichlet, K);
         void *td = nullptr;
-        int rc = upload(c, &td, tc_table(K, A.t, tc_sk(c->opt.precision)));
+        TcSums sums;
+        int rc = upload(c, &td, tc_table(K, A.t, tc_sk(c->opt.precision), &sums));
+        if (tc_needs_carry(c->opt.precision, sums)) c->tc_carry = 1;
         if (rc) return rc;
         o.tc[ai] = td;
         return SCFT_OK;
@@ -1119,7 +1161,7 @@ static std::vector<LoopChoice> tc_loops(const scft_ctx *c, int smem_limit)
         if ((!exchange && (cluster & (cluster - 1)) != 0) || !tc_loop_make(c, cluster, exchange, smem_limit, ch)) continue;
         Step2DArgs a;
         memset(&a, 0, sizeof(a));
-        if (scft_launch_chain_tc(c->opt.precision, ch.lp, a, 1, c->stream, &ch.resident) != cudaSuccess || ch.resident < 1) {
+        if (scft_launch_chain_tc(c->opt.precision, c->tc_carry, ch.lp, a, 1, c->stream, &ch.resident) != cudaSuccess || ch.resident < 1) {
             cudaGetLastError();
             continue;
         }
@@ -1144,6 +1186,7 @@ static std::map<std::string, int> g_tune_cache;
 static int launch_steps(scft_ctx *c, const ChainDesc *chains, int nchains_total, int maxlen);
 static int plan_rounds(scft_ctx *c);
 static void drop_rounds(scft_ctx *c);
+static void drop_graph(scft_ctx *c);
 
 static int autotune_axes(scft_ctx *c)
 {
@@ -1258,7 +1301,7 @@ static int tc_resident(const scft_ctx *c)
     Step2DArgs a;
     memset(&a, 0, sizeof(a));
     int n = 0;
-    if (scft_launch_chain_tc(c->opt.precision, c->loop, a, 1, c->stream, &n) == cudaSuccess) return n;
+    if (scft_launch_chain_tc(c->opt.precision, c->tc_carry, c->loop, a, 1, c->stream, &n) == cudaSuccess) return n;
     cudaGetLastError();
     return 0;
 }
@@ -1895,7 +1938,9 @@ extern "C" int scft_set_surface(scft_ctx *c, int b, const scft_surface *s)
             return SCFT_ERR_PARAM;
         }
         InstOps o;
+        const int carry = c->tc_carry;
         rc = build_opset(c, d, o);
+        if (c->tc_carry != carry) drop_graph(c);
         if (rc) return rc;
         c->ops_h.push_back(o);
         c->ops_alpha.insert(c->ops_alpha.end(), {d.alphax, d.alphay, d.alphaz});
@@ -2081,18 +2126,24 @@ static int plan_rounds(scft_ctx *c)
     return upload(c, (void **)&c->units, units);
 }
 
-/* Back to one launch, before something changes that the parts were cut for. */
-static void drop_rounds(scft_ctx *c)
+/* An iteration is captured again when its launches change. */
+static void drop_graph(scft_ctx *c)
 {
-    if (c->rounds.empty()) return;
     cudaStreamSynchronize(c->stream);
-    c->launches_per_iter -= (long)c->rounds.size() - 1;
-    c->prop_launches_per_iter = 1;
-    c->rounds.clear();
     if (c->graph_exec) cudaGraphExecDestroy(c->graph_exec);
     if (c->graph) cudaGraphDestroy(c->graph);
     c->graph_exec = nullptr;
     c->graph = nullptr;
+}
+
+/* Back to one launch, before something changes that the parts were cut for. */
+static void drop_rounds(scft_ctx *c)
+{
+    if (c->rounds.empty()) return;
+    c->launches_per_iter -= (long)c->rounds.size() - 1;
+    c->prop_launches_per_iter = 1;
+    c->rounds.clear();
+    drop_graph(c);
 }
 
 /* All contour steps of every chain: one launch per axis per step. */
@@ -2109,7 +2160,7 @@ static int launch_steps(scft_ctx *c, const ChainDesc *chains, int nchains_total,
             if (c->fused3d)
                 CK(scft_launch_step3d(a, r.second, c->stream, 0));
             else
-                CK(scft_launch_chain_tc(c->opt.precision, c->loop, a, r.second, c->stream, nullptr));
+                CK(scft_launch_chain_tc(c->opt.precision, c->tc_carry, c->loop, a, r.second, c->stream, nullptr));
         }
         return SCFT_OK;
     }
@@ -2138,7 +2189,7 @@ static int launch_steps(scft_ctx *c, const ChainDesc *chains, int nchains_total,
         a.s = 0;
         a.s_end = maxlen - 1;
         a.sstride = c->sm;
-        CK(scft_launch_chain_tc(c->opt.precision, c->loop, a, nchains_total, c->stream, nullptr));
+        CK(scft_launch_chain_tc(c->opt.precision, c->tc_carry, c->loop, a, nchains_total, c->stream, nullptr));
         return SCFT_OK;
     }
     const int npass = (int)c->axes.size();
@@ -2159,7 +2210,7 @@ static int launch_steps(scft_ctx *c, const ChainDesc *chains, int nchains_total,
             pa.h = A.h;
             pa.even = A.even;
             if (A.tc)
-                CK(scft_launch_pass_tc(c->opt.precision, A.t, pa, c->stream));
+                CK(scft_launch_pass_tc(c->opt.precision, c->tc_carry, A.t, pa, c->stream));
             else
                 CK(scft_launch_pass(c->opt.precision, A.g, pa, A.ntiles, c->stream));
         }

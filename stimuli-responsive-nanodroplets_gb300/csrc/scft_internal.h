@@ -167,11 +167,11 @@ struct TcLoop {
 size_t scft_pass_tc_smem(int prec, const TcGeom &g);
 int scft_pass_tc_fits(int prec, const TcGeom &g, int smem_limit);
 cudaError_t scft_pass_tc_configure(int smem_bytes);
-cudaError_t scft_launch_pass_tc(int prec, const TcGeom &g, const PassArgs &a, cudaStream_t st);
+cudaError_t scft_launch_pass_tc(int prec, int carry, const TcGeom &g, const PassArgs &a, cudaStream_t st);
 struct Step2DArgs;
 size_t scft_chain_tc_layout(int prec, TcLoop &lp);
 void scft_chain_tc_regions(int prec, const TcLoop &lp, int ax, long at[4]);
-cudaError_t scft_launch_chain_tc(int prec, const TcLoop &lp, const Step2DArgs &a, int nchains, cudaStream_t st,
+cudaError_t scft_launch_chain_tc(int prec, int carry, const TcLoop &lp, const Step2DArgs &a, int nchains, cudaStream_t st,
                                  int *clusters);
 /* 1 if a tensor-core wait of a pass gave up since the last call (clears it) */
 int scft_pass_tc_take_fault(void);

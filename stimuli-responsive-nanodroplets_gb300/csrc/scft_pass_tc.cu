@@ -18,15 +18,23 @@
  *     axis of length 4k, with the shift by half its length: integer sums and
  *     differences split it into NB = 2 or 4 blocks of size n/NB, exactly;
  *   - block operands and operators are cut into balanced digits of 10 bits,
- *     which fp16 holds exactly; a product of two digit matrices with
- *     |digit| <= 512 sums to an integer below 2^24 that the FP32 accumulators
- *     hold exactly. Digit pairs (i, j) with i + j = l share the accumulator of
- *     level l; the levels kept (6 of FP64's, 4 of FP32's) leave out terms of
- *     2^-56 (2^-27) of the line's largest value;
+ *     which fp16 holds exactly, |digit| <= 512. Digit pairs (i, j) with i + j = l
+ *     share the FP32 accumulator of level l; the levels kept (6 of FP64's, 4 of
+ *     FP32's) leave out terms of 2^-56 (2^-27) of the line's largest value;
+ *   - a level's sum is an integer, which the accumulator holds exactly up to 2^24.
+ *     Its bound, 512 times the sum of the operator's digits up to that level over a
+ *     row, is taken from the digits when the table is made (tc_table): where levels 0
+ *     to 3 of FP64 or FP32x2 stay below 2^24 over whole rows, they are summed as they
+ *     are, otherwise (long lines, and operators wider than the line, whose digits and
+ *     those of a flat line add up with one sign) what is above 2^9 is carried to the
+ *     level above after every 16 points. The last two levels, and FP32's, may pass 2^24
+ *     by their bound (1.8 times on 192 points); a unit that is then lost is below
+ *     2^-56 (FP32: 2^-27 per unit of its level 1), and on random digits their sums are
+ *     at twelve standard deviations from it;
  *   - the levels are joined in 64-bit integers (FP32: three multiply-adds), and
  *     each output is rounded once to the value type.
- * Results do not depend on the tile, the number of output parts or what shares
- * the launch: every line is computed by the same integer arithmetic.
+ * Results do not depend on the tile, the number of output parts, the carries or what
+ * shares the launch: every line is computed by the same integer arithmetic.
  *
  * A CTA takes `tile` lines and a range of output chunks. Data digits and
  * operator digits sit in shared memory as 8 x 16-byte cells, which ldmatrix
@@ -267,6 +275,29 @@ __device__ __forceinline__ void mma16816(float (&c)[4], const uint32_t (&a)[4], 
                  : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
+/* What is above 2^9 in the sums of levels 1 to 3, an integer, moved to the level above,
+ * so that the next 16 points add to sums of at most 2^15: exact, two sums at a time.
+ * Upwards from level 1, so that no step waits for the one before it. Always done it
+ * costs 2-6 % of a whole solve (192x96, FP64 6.83 -> 6.97-7.12 ms, 150x75 FP32 4.84 ->
+ * 5.16), hence only where an operator needs it. */
+template <int L>
+__device__ __forceinline__ void carry_sums(float (&d)[L][4])
+{
+#pragma unroll
+    for (int l = 1; l <= 3; ++l)
+#pragma unroll
+        for (int v = 0; v < 4; v += 2)
+            asm("{\n\t.reg .b64 x, u, t, c;\n\t"
+                "mov.b64 x, {%0, %1};\n\tmov.b64 u, {%2, %3};\n\t"
+                "mov.b64 t, {0f4B400000, 0f4B400000};\n\tmov.b64 c, {0f3A800000, 0f3A800000};\n\t"
+                "fma.rn.f32x2 t, x, c, t;\n\t" /* 1.5 2^23 + x / 1024: its unit is 1 */
+                "mov.b64 c, {0fCB400000, 0fCB400000};\n\tadd.rn.f32x2 t, t, c;\n\t"
+                "add.rn.f32x2 u, u, t;\n\t"
+                "mov.b64 c, {0fC4800000, 0fC4800000};\n\tfma.rn.f32x2 x, t, c, x;\n\t"
+                "mov.b64 {%0, %1}, x;\n\tmov.b64 {%2, %3}, u;\n\t}"
+                : "+f"(d[l][v]), "+f"(d[l][v + 1]), "+f"(d[l - 1][v]), "+f"(d[l - 1][v + 1]));
+}
+
 __device__ __forceinline__ long long mad_wide(int a, int b, long long c)
 {
     long long d;
@@ -364,7 +395,7 @@ __host__ __device__ inline uint32_t exchange_bytes(const TcGeom &g, int value)
  * lines fill the MMA. ldmatrix rows: operator (8 outputs, 8 points) cells at (output half, point
  * half) = (lane >> 3 & 1, lane >> 4), line cells at (digit, point half) = (lane >> 4, lane >> 3 & 1).
  * d[.][v]: output (lane >> 2) + 8 (v >> 1), line 2 (lane & 3) + (v & 1). */
-template <typename P, int NB>
+template <typename P, int NB, bool CARRY>
 __device__ __forceinline__ void products16x8(float (&d)[Dig<P>::L][4], uint32_t op, uint32_t lines, int nk8, int ks, int nc, int rg, int cp, int b)
 {
     constexpr int S = Dig<P>::S, SK = Dig<P>::SK, L = Dig<P>::L, CELL = S * NB * 128;
@@ -378,6 +409,7 @@ __device__ __forceinline__ void products16x8(float (&d)[Dig<P>::L][4], uint32_t 
         for (int v = 0; v < 4; ++v) d[l][v] = 0.0f;
 #pragma unroll 1
     for (int k = 0; k < ks; ++k) {
+        if (CARRY && k > 0) carry_sums(d);
         uint32_t bf[(S + 1) / 2][4]; /* line digits 2i, 2i + 1 */
 #pragma unroll
         for (int i = 0; i < (S + 1) / 2; ++i)
@@ -456,7 +488,7 @@ constexpr int EBITS = 11; /* bits of an exponent */
 
 /* The tile of k_chain2d_tc: like tc_tile, from lines with their exponents in
  * shared memory to lines of the other axis in their CTAs' shared memory. */
-template <typename P, int NB, int NT>
+template <typename P, int NB, int NT, bool CARRY>
 __device__ __forceinline__ void tc_tile2d(const TcGeom &g, const Exchange<P> &xc, bool last, int tile_i, unsigned char *smem,
                                           uint32_t sm_op, uint32_t sm_a, uint32_t sm_ex, uint32_t bar_op, bool wait_op,
                                           bool &ok)
@@ -513,7 +545,7 @@ __device__ __forceinline__ void tc_tile2d(const TcGeom &g, const Exchange<P> &xc
     for (int u = warp; u < nr * np * NB; u += NT / 32) {
         const int b = u % NB, v = u / NB, rg = nr == 1 ? 0 : v / np, cp = v - rg * np;
         float d[L][4];
-        products16x8<P, NB>(d, sbase + sm_op, sbase + sm_a, nk8, ks, nc, rg, cp, b);
+        products16x8<P, NB, CARRY>(d, sbase + sm_op, sbase + sm_a, nk8, ks, nc, rg, cp, b);
         Acc *at = ex + (rg * 8 + 2 * (lane & 3)) * pitch + (b * nc + 2 * cp) * W + (lane >> 2);
 #pragma unroll
         for (int i = 0; i < 4; ++i)
@@ -603,7 +635,7 @@ __device__ __forceinline__ void tc_tile2d(const TcGeom &g, const Exchange<P> &xc
 
 /* One tile of lines and one part of its outputs: y = K x (times b before the
  * first axis, after the last). Ends with every thread of the CTA past the digits. */
-template <typename P, int NB, int NT, bool SPLIT>
+template <typename P, int NB, int NT, bool SPLIT, bool CARRY>
 __device__ __forceinline__ void tc_tile(const TcGeom &g, const P *src, P *dst, const P *bz,
                                         bool first, bool last, int tile_i, int part, unsigned char *smem,
                                         uint32_t sm_op, uint32_t sm_a, uint32_t bar_op, bool wait_op, TcPhase &ph)
@@ -765,7 +797,7 @@ __device__ __forceinline__ void tc_tile(const TcGeom &g, const P *src, P *dst, c
         for (int u = warp; u < nr * np * NB; u += NT / 32) {
             const int b = u % NB, v = u / NB, rg = nr == 1 ? 0 : v / np, cp = v - rg * np;
             float d[L][4];
-            products16x8<P, NB>(d, sbase + sm_op, sbase + sm_a, nk8, ks, nc, rg, cp, b);
+            products16x8<P, NB, CARRY>(d, sbase + sm_op, sbase + sm_a, nk8, ks, nc, rg, cp, b);
             Acc *at = ex + (rg * 8 + 2 * (lane & 3)) * pitch + (b * nc + 2 * cp) * W + (lane >> 2);
 #pragma unroll
             for (int i = 0; i < 4; ++i)
@@ -810,6 +842,7 @@ __device__ __forceinline__ void tc_tile(const TcGeom &g, const P *src, P *dst, c
                 for (int v = 0; v < 4; ++v) d[l][v] = 0.0f;
 #pragma unroll 1
             for (int k = 0; k < ks; ++k) {
+                if (CARRY && k > 0) carry_sums(d);
                 uint32_t bf[SK / 2][4]; /* digits 2j, 2j + 1 */
 #pragma unroll
                 for (int j = 0; j < SK / 2; ++j) ldsm4(bf[j], b0 + (uint32_t)(k * SK * 256 + j * 512));
@@ -907,7 +940,7 @@ __device__ __forceinline__ void tc_begin(unsigned char *smem, int nax)
 } // namespace
 
 /* One pass: a CTA per (tile, part) and chain. */
-template <typename P, int NB>
+template <typename P, int NB, bool CARRY>
 __global__ void __launch_bounds__(256, 2) k_pass_tc(TcGeom g, PassArgs a)
 {
     const ChainDesc cd = a.chains[blockIdx.y];
@@ -932,7 +965,7 @@ __global__ void __launch_bounds__(256, 2) k_pass_tc(TcGeom g, PassArgs a)
     P *dst = a.last ? reinterpret_cast<P *>(cd.q) + (long)(a.s + 1) * a.sstride : reinterpret_cast<P *>(cd.tmp);
     const P *bz = reinterpret_cast<const P *>(a.s < cd.seg_end ? cd.b0 : cd.b1);
     TcPhase ph = {0, true};
-    tc_tile<P, NB, 256, false>(g, src, dst, bz, a.first, a.last, tile_i, part, smem, SM_OP, SM_OP + g.op_part, bar_op, true, ph);
+    tc_tile<P, NB, 256, false, CARRY>(g, src, dst, bz, a.first, a.last, tile_i, part, smem, SM_OP, SM_OP + g.op_part, bar_op, true, ph);
     if (!ph.ok && threadIdx.x == 0) atomicExch(&g_scft_pass_fault, 1);
 }
 
@@ -948,7 +981,7 @@ __global__ void __launch_bounds__(256, 2) k_pass_tc(TcGeom g, PassArgs a)
  * 512 threads at a time (three groups, or groups of 384 threads, do not fit or
  * gain nothing: issue slots are ~45 % busy, shared memory 50 %, and neither more
  * warps nor more overlap moves that). Control flow is uniform over the cluster. */
-template <typename P>
+template <typename P, bool CARRY>
 __global__ void __launch_bounds__(512, 1) k_chain_tc(const __grid_constant__ TcLoop lp, Step2DArgs a)
 {
     const int rank = blockIdx.x % lp.cluster, slot = blockIdx.x / lp.cluster; /* clusters are consecutive blocks */
@@ -995,10 +1028,10 @@ __global__ void __launch_bounds__(512, 1) k_chain_tc(const __grid_constant__ TcL
 #pragma unroll 1
                 for (int t = t0; (long)t * g.tile < g.lines; t += GROUPS * lp.slots[ax]) {
                     if (g.nb == 4)
-                        tc_tile<P, 4, 512 / GROUPS, true>(g, src, dst, bz, first, last, t, part, smem, lp.op_at[ax], tile_at,
+                        tc_tile<P, 4, 512 / GROUPS, true, CARRY>(g, src, dst, bz, first, last, t, part, smem, lp.op_at[ax], tile_at,
                                                  sbase + SM_BAR + 8 * ax, s == run.s && t == t0, ph);
                     else
-                        tc_tile<P, 2, 512 / GROUPS, true>(g, src, dst, bz, first, last, t, part, smem, lp.op_at[ax], tile_at,
+                        tc_tile<P, 2, 512 / GROUPS, true, CARRY>(g, src, dst, bz, first, last, t, part, smem, lp.op_at[ax], tile_at,
                                                  sbase + SM_BAR + 8 * ax, s == run.s && t == t0, ph);
                 }
             /* this axis' slice is complete before the next one reads it */
@@ -1037,7 +1070,7 @@ __global__ void __launch_bounds__(512, 1) k_chain_tc(const __grid_constant__ TcL
  * and the rate of mma.sync (2500 + 2500), with ~600 between them. FP64, a step:
  * 32x16 7.0 -> 4.0 us, 64x64 6.9 -> 5.2, 192x96 10.8 -> 8.4 against the loop
  * above, which stays for 3D grids and for slices that do not fit one tile a CTA. */
-template <typename P>
+template <typename P, bool CARRY>
 __global__ void __launch_bounds__(512, 1) k_chain2d_tc(const __grid_constant__ TcLoop lp, Step2DArgs a)
 {
     const int rank = blockIdx.x % lp.cluster, slot = blockIdx.x / lp.cluster; /* clusters are consecutive blocks */
@@ -1124,9 +1157,9 @@ __global__ void __launch_bounds__(512, 1) k_chain2d_tc(const __grid_constant__ T
                                     reinterpret_cast<const P *>(s + 1 < cd.seg_end ? cd.b0 : cd.b1),
                                     reinterpret_cast<P *>(cd.q) + (long)(s + 1) * a.sstride};
             if (g.nb == 4)
-                tc_tile2d<P, 4, 512>(g, xc, ax == 1, rank, smem, lp.op_at[ax], lp.tile_at, lp.ex_at, bars + 8 * ax, t == 0, ok);
+                tc_tile2d<P, 4, 512, CARRY>(g, xc, ax == 1, rank, smem, lp.op_at[ax], lp.tile_at, lp.ex_at, bars + 8 * ax, t == 0, ok);
             else
-                tc_tile2d<P, 2, 512>(g, xc, ax == 1, rank, smem, lp.op_at[ax], lp.tile_at, lp.ex_at, bars + 8 * ax, t == 0, ok);
+                tc_tile2d<P, 2, 512, CARRY>(g, xc, ax == 1, rank, smem, lp.op_at[ax], lp.tile_at, lp.ex_at, bars + 8 * ax, t == 0, ok);
         }
     }
     if (!ok && threadIdx.x == 0) atomicExch(&g_scft_pass_fault, 1);
@@ -1141,13 +1174,14 @@ size_t scft_pass_tc_smem(int prec, const TcGeom &g)
                                                       : tile_bytes(g, Dig<double>::S, 16));
 }
 
-template <typename P>
+template <typename P, bool CARRY>
 static cudaError_t launch_tc(const TcGeom &g, const PassArgs &a, cudaStream_t st)
 {
     const size_t smem = SM_OP + g.op_part + tile_bytes(g, Dig<P>::S, 16);
     const dim3 grid((unsigned)((g.lines + g.tile - 1) / g.tile * g.parts), a.nchains);
     if (g.tile < 8 || g.tile % 8 || g.tile > ROWS) return cudaErrorInvalidValue;
-    return g.nb == 4 ? pdl_launch(k_pass_tc<P, 4>, grid, 256, smem, st, g, a) : pdl_launch(k_pass_tc<P, 2>, grid, 256, smem, st, g, a);
+    return g.nb == 4 ? pdl_launch(k_pass_tc<P, 4, CARRY>, grid, 256, smem, st, g, a)
+                     : pdl_launch(k_pass_tc<P, 2, CARRY>, grid, 256, smem, st, g, a);
 }
 
 int scft_pass_tc_fits(int prec, const TcGeom &g, int smem_limit)
@@ -1155,11 +1189,12 @@ int scft_pass_tc_fits(int prec, const TcGeom &g, int smem_limit)
     return scft_pass_tc_smem(prec, g) <= (size_t)smem_limit;
 }
 
-cudaError_t scft_launch_pass_tc(int prec, const TcGeom &g, const PassArgs &a, cudaStream_t st)
+/* carry: an operator of the context needs the carries of carry_sums (FP32 never does). */
+cudaError_t scft_launch_pass_tc(int prec, int carry, const TcGeom &g, const PassArgs &a, cudaStream_t st)
 {
-    if (prec == SCFT_PREC_FP64) return launch_tc<double>(g, a, st);
-    if (prec == SCFT_PREC_FP32X2) return launch_tc<dfloat>(g, a, st);
-    return launch_tc<float>(g, a, st);
+    if (prec == SCFT_PREC_FP64) return carry ? launch_tc<double, true>(g, a, st) : launch_tc<double, false>(g, a, st);
+    if (prec == SCFT_PREC_FP32X2) return carry ? launch_tc<dfloat, true>(g, a, st) : launch_tc<dfloat, false>(g, a, st);
+    return launch_tc<float, false>(g, a, st);
 }
 
 /* Shared-memory layout of the cluster loop, from the axes' tiles and parts;
@@ -1208,7 +1243,7 @@ extern "C" void scft_tc_exchange_exponents(long at[4][2])
     }
 }
 
-template <typename P>
+template <typename P, bool CARRY>
 static cudaError_t launch_chain(const TcLoop &lp, const Step2DArgs &a, int nchains, cudaStream_t st, int *clusters)
 {
     TcLoop l = lp;
@@ -1228,45 +1263,49 @@ static cudaError_t launch_chain(const TcLoop &lp, const Step2DArgs &a, int nchai
     cfg.attrs = attr;
     cfg.numAttrs = 2;
     if (lp.exchange) {
-        if (clusters) return cudaOccupancyMaxActiveClusters(clusters, k_chain2d_tc<P>, &cfg);
-        return cudaLaunchKernelEx(&cfg, k_chain2d_tc<P>, l, a);
+        if (clusters) return cudaOccupancyMaxActiveClusters(clusters, k_chain2d_tc<P, CARRY>, &cfg);
+        return cudaLaunchKernelEx(&cfg, k_chain2d_tc<P, CARRY>, l, a);
     }
-    if (clusters) return cudaOccupancyMaxActiveClusters(clusters, k_chain_tc<P>, &cfg);
-    return cudaLaunchKernelEx(&cfg, k_chain_tc<P>, l, a);
+    if (clusters) return cudaOccupancyMaxActiveClusters(clusters, k_chain_tc<P, CARRY>, &cfg);
+    return cudaLaunchKernelEx(&cfg, k_chain_tc<P, CARRY>, l, a);
 }
 
 /* Launches the contour loops of nchains chains; with clusters != NULL only asks
  * how many clusters can be resident. */
-cudaError_t scft_launch_chain_tc(int prec, const TcLoop &lp, const Step2DArgs &a, int nchains, cudaStream_t st,
+cudaError_t scft_launch_chain_tc(int prec, int carry, const TcLoop &lp, const Step2DArgs &a, int nchains, cudaStream_t st,
                                  int *clusters)
 {
-    if (prec == SCFT_PREC_FP64) return launch_chain<double>(lp, a, nchains, st, clusters);
-    if (prec == SCFT_PREC_FP32X2) return launch_chain<dfloat>(lp, a, nchains, st, clusters);
-    return launch_chain<float>(lp, a, nchains, st, clusters);
+    if (prec == SCFT_PREC_FP64)
+        return carry ? launch_chain<double, true>(lp, a, nchains, st, clusters) : launch_chain<double, false>(lp, a, nchains, st, clusters);
+    if (prec == SCFT_PREC_FP32X2)
+        return carry ? launch_chain<dfloat, true>(lp, a, nchains, st, clusters) : launch_chain<dfloat, false>(lp, a, nchains, st, clusters);
+    return launch_chain<float, false>(lp, a, nchains, st, clusters);
 }
 
-template <typename P>
+template <typename P, bool CARRY>
 static cudaError_t configure_tc(int smem_bytes)
 {
     /* one carve-out for every pass, so the SMs keep their split between launches */
-    const void *k[] = {(const void *)k_pass_tc<P, 4>, (const void *)k_pass_tc<P, 2>, (const void *)k_chain_tc<P>,
-                       (const void *)k_chain2d_tc<P>};
+    const void *k[] = {(const void *)k_pass_tc<P, 4, CARRY>, (const void *)k_pass_tc<P, 2, CARRY>, (const void *)k_chain_tc<P, CARRY>,
+                       (const void *)k_chain2d_tc<P, CARRY>};
     cudaError_t e = cudaSuccess;
     for (const void *f : k) {
         if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
         if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
     }
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_chain_tc<P>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_chain2d_tc<P>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_chain_tc<P, CARRY>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_chain2d_tc<P, CARRY>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     return e;
 }
 
 /* Raise the dynamic shared-memory limit once, outside any stream capture. */
 cudaError_t scft_pass_tc_configure(int smem_bytes)
 {
-    cudaError_t e = configure_tc<double>(smem_bytes);
-    if (e == cudaSuccess) e = configure_tc<dfloat>(smem_bytes);
-    if (e == cudaSuccess) e = configure_tc<float>(smem_bytes);
+    cudaError_t e = configure_tc<double, false>(smem_bytes);
+    if (e == cudaSuccess) e = configure_tc<double, true>(smem_bytes);
+    if (e == cudaSuccess) e = configure_tc<dfloat, false>(smem_bytes);
+    if (e == cudaSuccess) e = configure_tc<dfloat, true>(smem_bytes);
+    if (e == cudaSuccess) e = configure_tc<float, false>(smem_bytes);
     return e;
 }
 
