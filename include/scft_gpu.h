@@ -99,6 +99,13 @@ typedef struct scft_ctx scft_ctx;
 #define SCFT_PREC_FP32X2 2 /* propagators in double-float arithmetic (pairs of FP32, ~48-bit
                               significand, FP32 exponent range) on double-float slices,
                               reductions FP64: the finishing form below the FP32 form's floor */
+/* The contour steps of FP64 and FP32X2, and those of FP32 on grids without a fused loop of
+ * their own, hold each grid line in fixed point under its largest value (58 bits, FP32: 28):
+ * the error of a propagator value is 2^-56 (2^-27) of its line's largest value a step,
+ * however small the value, as it is with the FFTs of SCFT.c:2474-2631. At 1e-9 of that
+ * largest value, a grafted chain far from its wall say, FP64 keeps about 8 digits and FP32
+ * none, where it may come out negative. Values below the type's smallest normal number
+ * count as zero. */
 
 #define SCFT_NOISE_HOST 0    /* caller passes noise arrays to scft_iterate */
 #define SCFT_NOISE_DRAND48 1 /* device replays the drand48 stream (funGaussDev) */
