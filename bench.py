@@ -201,6 +201,7 @@ def measure_form(srn, surfaces, precision: str, steps: int, warmup: int, device:
         "contour_steps_per_instance_iteration": steps_iter,
         "device_bytes": sv.device_bytes,
         "threads_per_line": int(t["threads_per_line"]),
+        "ctas_per_chain": int(t["ctas_per_chain"]),
         "kernel": {1: f"k_chain2d<float,{sv.grid[0]},{sv.grid[2]}> (persistent fused contour loop)",
                    2: "k_chain3d (64^3 contour loop, one 8-CTA cluster per chain)"}.get(
                        t["fused_chain"], "k_pass_tc / k_chain_tc / k_chain2d_tc (axis contractions on the tensor cores)"),

@@ -312,10 +312,15 @@ typedef struct scft_timing {
                           2 the 64^3 cluster kernel; 0 per-axis passes (prop_launches tells whether
                           each is a launch or a chain's passes run in one) */
     int threads_per_line; /* fused 2D kernel: 2 when a batch of at most one chain per SM gives each
-                             line two threads, or each chain several CTAs (bit-identical results), else 1 */
+                             line two threads, or each chain several CTAs (bit-identical results;
+                             scft_chain_ctas tells them apart), else 1 */
 } scft_timing;
 int scft_enable_timing(scft_ctx *ctx, int on);
 int scft_get_timing(const scft_ctx *ctx, scft_timing *t);
+/* CTAs that share one chain in the contour loop: 0 where the axis passes are launches of their
+ * own, 1 for the fused 2D loop with one or two threads per line, else the size of the chain's
+ * cluster. Negative on a NULL context. */
+int scft_chain_ctas(const scft_ctx *ctx);
 
 const char *scft_last_error(void);
 

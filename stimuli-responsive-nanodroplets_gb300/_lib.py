@@ -176,6 +176,7 @@ def lib() -> C.CDLL:
         "scft_static_scratch_bytes": (C.c_size_t, []),
         "scft_enable_timing": (I, [VP, I]),
         "scft_get_timing": (I, [VP, P(CTiming)]),
+        "scft_chain_ctas": (I, [VP]),
         "scft_last_error": (C.c_char_p, []),
         "scft_device_memory": (I, [I, P(C.c_size_t), P(C.c_size_t)]),
         "scft_noise_fill": (I, [us3, P(CDerived), dp]),

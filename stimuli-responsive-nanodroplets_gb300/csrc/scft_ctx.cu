@@ -2675,6 +2675,14 @@ extern "C" int scft_get_timing(const scft_ctx *c, scft_timing *t)
     return SCFT_OK;
 }
 
+extern "C" int scft_chain_ctas(const scft_ctx *c)
+{
+    if (!c) return SCFT_ERR_PARAM;
+    if (c->fused2d) return c->wide2d > 1 ? c->wide2d : 1;
+    if (c->fused3d) return scft_step3d_ctas();
+    return c->loop_tc ? c->loop.cluster : 0;
+}
+
 /* ------------------------------------------------- internal hooks */
 /* Used by scft_noalloc.cu: context facts and the contour-step launcher on a
  * caller-provided chain descriptor. */

@@ -252,6 +252,7 @@ size_t scft_step2d_smem(int prec, int nx, int nz);
 /* 64^3 periodic FP32 grids: one 8-CTA cluster per chain (scft_step3d.cu) */
 size_t scft_step3d_smem(int prec, int nx, int ny, int nz);
 cudaError_t scft_launch_step3d(const Step2DArgs &a, int nchains, cudaStream_t st, int configure);
+int scft_step3d_ctas(void);     /* CTAs of a chain's cluster */
 int scft_step3d_resident(void); /* clusters that fit on the GPU */
 /* What cluster `slot` of a launch runs: chain and contour steps. */
 struct StepRange {

@@ -366,6 +366,8 @@ static cudaError_t resident_clusters(int *nclusters)
     return cudaOccupancyMaxActiveClusters(nclusters, k_chain3d, &cfg);
 }
 
+int scft_step3d_ctas(void) { return CL; }
+
 int scft_step3d_resident(void)
 {
     int n = 0;

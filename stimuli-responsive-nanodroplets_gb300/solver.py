@@ -259,7 +259,7 @@ class Solver:
         L.check(L.lib().scft_get_timing(self._h, C.byref(t)), "scft_get_timing")
         return {"total_ms": t.total_ms, "prop_ms": t.prop_ms, "prop_launches": t.prop_launches,
                 "kernel_launches": t.kernel_launches, "fused_chain": int(t.fused_chain),
-                "threads_per_line": int(t.threads_per_line)}
+                "threads_per_line": int(t.threads_per_line), "ctas_per_chain": int(L.lib().scft_chain_ctas(self._h))}
 
 
 # ----------------------------------------------------------------- host side
