@@ -637,34 +637,85 @@ static void tc_shape(int n, int dirichlet, TcGeom &g)
     g.cpp = g.nchunks;
 }
 
+/* A number in [-1, 1] as hi 2^-62 + lo 2^-124: what the operator's cosine sums are taken in,
+ * as the host's long double is 113 bits in software (a context of a 64x64 bulk: 0.3 of its
+ * 0.9 ms went into two tables). */
+struct Fixed {
+    long long hi, lo;
+};
+static Fixed fixed(long double x)
+{
+    const long double y = ldexpl(x, 62), hi = floorl(y);
+    return {(long long)hi, (long long)ldexpl(y - hi, 62)};
+}
+/* x y in units of 2^-108 */
+static __int128 product(const Fixed &x, const Fixed &y)
+{
+    return (((__int128)x.hi * y.hi) >> 16) + (((__int128)x.hi * y.lo + (__int128)x.lo * y.hi) >> 78);
+}
+
+/* The values of an axis' operator that dense_operator lays out, in units of 2^-90: the
+ * circulant's c[d], or f[d] of K[a][b] = f[a - b] - f[a + b + 2] between walls. */
+struct AxisOp {
+    int n, dirichlet;
+    std::vector<__int128> v;
+    __int128 at(int i, int j) const
+    {
+        const int d = i < j ? j - i : i - j;
+        return dirichlet ? v[d] - v[i + j + 2] : v[d];
+    }
+};
+static AxisOp axis_operator(int n, double alpha, int dirichlet)
+{
+    const long double pi = 3.141592653589793238462643383279502884L;
+    /* periods N: the axis, or the odd extension of one between walls; modes m and N - m are one */
+    const int N = dirichlet ? 2 * (n + 1) : n, top = dirichlet ? n : n / 2, scale = dirichlet ? n + 1 : n;
+    AxisOp op{n, dirichlet, std::vector<__int128>(N)};
+    std::vector<Fixed> E(top + 1), cs(N);
+    for (int m = 0; m <= top; ++m) {
+        const double k = kval(m, N);
+        E[m] = fixed(dirichlet && m == 0 ? 0.0L : expl(-(long double)alpha * (long double)k * (long double)k));
+    }
+    for (int d = 0; d <= N / 2; ++d) {
+        if (N % 2 == 0 && 4 * d > N) { /* the other way up */
+            const __int128 c = -(((__int128)cs[N / 2 - d].hi << 62) + cs[N / 2 - d].lo);
+            cs[d] = {(long long)(c >> 62), (long long)(c & ((1LL << 62) - 1))};
+        } else {
+            cs[d] = fixed(cosl(2.0L * pi * d / N));
+        }
+        cs[(N - d) % N] = cs[d];
+    }
+    for (int d = 0; d <= N / 2; ++d) {
+        __int128 s = 0;
+        for (int m = 0, at = 0; m <= top; ++m, at = at + d < N ? at + d : at + d - N) {
+            const __int128 p = product(E[m], cs[at]);
+            s += dirichlet || m == 0 || 2 * m == n ? p : 2 * p;
+        }
+        op.v[d] = op.v[(N - d) % N] = (s >> 18) / scale;
+    }
+    return op;
+}
+
 /* Block operators of the tensor-core passes (scft_pass_tc.cu): with u_b the sums
  * and differences of a line's points (block 0 all sums, then the mirror
  * difference; on a periodic axis of length 4k the half-axis difference's pair
- * after them), y is built from M_b u_b by the same sums and differences. Points
- * of block row and column i < hb; the middle point of an odd axis counts
+ * after them), y is built from M_b u_b by the same sums and differences. M[b] of
+ * one entry, times nb, in units of 2^-90; the middle point of an odd axis counts
  * itself twice in its sum, which the operator's column halves. */
-static std::vector<long double> tc_blocks(const std::vector<long double> &K, int n, int nb, int hb)
+static void tc_block_entries(const AxisOp &K, int nb, int i, int j, __int128 M[4])
 {
-    std::vector<long double> M((size_t)nb * hb * hb, 0.0L);
-    const int m = n / 2;
-    for (int i = 0; i < hb; ++i)
-        for (int j = 0; j < hb; ++j) {
-            const auto k = [&](int col) { return K[(size_t)i * n + col]; };
-            const size_t at = (size_t)i * hb + j, sz = (size_t)hb * hb;
-            if (nb == 2) {
-                const bool mid = 2 * j + 1 == n;
-                M[at] = mid ? k(j) / 2.0L : (k(j) + k(n - 1 - j)) / 2.0L;
-                M[sz + at] = mid ? 0.0L : (k(j) - k(n - 1 - j)) / 2.0L;
-            } else {
-                const long double a0 = k(j) + k(j + m), a1 = k(m - 1 - j) + k(n - 1 - j);
-                const long double b0 = k(j) - k(j + m), b1 = k(m - 1 - j) - k(n - 1 - j);
-                M[at] = (a0 + a1) / 4.0L;
-                M[sz + at] = (a0 - a1) / 4.0L;
-                M[2 * sz + at] = (b0 + b1) / 4.0L;
-                M[3 * sz + at] = (b0 - b1) / 4.0L;
-            }
-        }
-    return M;
+    const int n = K.n, m = n / 2;
+    if (nb == 2) {
+        const bool mid = 2 * j + 1 == n;
+        M[0] = mid ? K.at(i, j) : K.at(i, j) + K.at(i, n - 1 - j);
+        M[1] = mid ? 0 : K.at(i, j) - K.at(i, n - 1 - j);
+        return;
+    }
+    const __int128 k0 = K.at(i, j), k1 = K.at(i, m - 1 - j), k2 = K.at(i, j + m), k3 = K.at(i, n - 1 - j);
+    M[0] = k0 + k2 + (k1 + k3);
+    M[1] = k0 + k2 - (k1 + k3);
+    M[2] = k0 - k2 + (k1 - k3);
+    M[3] = k0 - k2 - (k1 - k3);
 }
 
 static int tc_sk(int prec) { return prec == SCFT_PREC_FP32 ? 4 : 6; }
@@ -674,9 +725,8 @@ static uint16_t half_of_int(int d)
 {
     if (d == 0) return 0;
     const uint16_t sign = d < 0 ? 0x8000 : 0;
-    unsigned u = (unsigned)(d < 0 ? -d : d);
-    int e = 0;
-    while ((u >> e) > 1) ++e;
+    const unsigned u = (unsigned)(d < 0 ? -d : d);
+    const int e = 31 - __builtin_clz(u);
     return (uint16_t)(sign | ((15 + e) << 10) | ((u << (10 - e)) & 0x3ff));
 }
 
@@ -689,39 +739,39 @@ static uint16_t half_of_int(int d)
 struct TcSums {
     double row[6], step[6];
 };
-static std::vector<uint16_t> tc_table(const std::vector<long double> &K, const TcGeom &g, int sk, TcSums *sums = nullptr)
+static std::vector<uint16_t> tc_table(const AxisOp &K, const TcGeom &g, int sk, TcSums *sums = nullptr)
 {
-    const std::vector<long double> M = tc_blocks(K, g.n, g.nb, g.hb);
-    const int kq = 10 * sk - (g.nb == 4 ? 0 : 1);
+    const int sh = 92 - 10 * sk; /* from nb M in units of 2^-90 to M 2^kq */
     std::vector<uint16_t> T((size_t)g.nb * g.hp * g.nchunks * g.w * sk, 0);
     if (sums) memset(sums, 0, sizeof(*sums));
-    for (int b = 0; b < g.nb; ++b)
-        for (int i = 0; i < g.hb; ++i) {
-            double row[6] = {0.0}, step16[6];
-            for (int j = 0; j < g.hb; ++j) {
-                if (j % 16 == 0) memset(step16, 0, sizeof(step16));
-                long long v = llroundl(ldexpl(M[((size_t)b * g.hb + i) * g.hb + j], kq));
-                const int c = i / g.w, o = i - c * g.w, wc = g.w;
-                const size_t chunk = (size_t)g.nb * g.hp * sk * ((size_t)c * g.w);
+    for (int i = 0; i < g.hb; ++i) {
+        const int c = i / g.w, o = i - c * g.w, wc = g.w;
+        const size_t chunk = (size_t)g.nb * g.hp * sk * ((size_t)c * g.w);
+        int row[4][6] = {}, step16[4][6]; /* sums of the digits' sizes */
+        for (int j = 0; j < g.hb; ++j) {
+            if (j % 16 == 0) memset(step16, 0, sizeof(step16));
+            __int128 M[4];
+            tc_block_entries(K, g.nb, i, j, M);
+            for (int b = 0; b < g.nb; ++b) {
+                long long v = (long long)((M[b] + ((__int128)1 << (sh - 1))) >> sh);
                 const size_t step = chunk + ((size_t)b * (g.hp / 16) + j / 16) * ((size_t)sk * wc * 16);
                 for (int d = sk - 1; d >= 0; --d) { /* lowest digit first */
-                    long long q = d > 0 ? ((v + 512) & 1023) - 512 : v;
+                    const int q = d > 0 ? (int)((v + 512) & 1023) - 512 : (int)v;
                     v = (v - q) >> 10;
                     const int r = d * wc + o, k = j & 15;
-                    T[step + (size_t)(r / 8) * 128 + (k / 8) * 64 + (r % 8) * 8 + k % 8] = half_of_int((int)q);
-                    row[d] += 512.0 * std::abs((int)q);
-                    step16[d] += 512.0 * std::abs((int)q);
-                }
-                if (sums && (j % 16 == 15 || j + 1 == g.hb)) {
-                    double s = 0.0;
-                    for (int d = 0; d < sk; ++d) sums->step[d] = std::max(sums->step[d], s += step16[d]);
+                    T[step + (size_t)(r / 8) * 128 + (k / 8) * 64 + (r % 8) * 8 + k % 8] = half_of_int(q);
+                    row[b][d] += std::abs(q);
+                    step16[b][d] += std::abs(q);
                 }
             }
-            if (sums) {
-                double s = 0.0;
-                for (int d = 0; d < sk; ++d) sums->row[d] = std::max(sums->row[d], s += row[d]);
-            }
+            if (sums && (j % 16 == 15 || j + 1 == g.hb))
+                for (int b = 0; b < g.nb; ++b)
+                    for (int d = 0, s = 0; d < sk; ++d) sums->step[d] = std::max(sums->step[d], 512.0 * (s += step16[b][d]));
         }
+        if (sums)
+            for (int b = 0; b < g.nb; ++b)
+                for (int d = 0, s = 0; d < sk; ++d) sums->row[d] = std::max(sums->row[d], 512.0 * (s += row[b][d]));
+    }
     return T;
 }
 
@@ -736,10 +786,8 @@ extern "C" int scft_tc_level_sums(int n, double alpha, int dirichlet, int prec, 
     if (n < 2 || !row || !step) return SCFT_ERR_PARAM;
     TcGeom g;
     tc_shape(n, dirichlet, g);
-    std::vector<long double> K;
-    dense_operator(n, alpha, dirichlet, K);
     TcSums s;
-    tc_table(K, g, tc_sk(prec), &s);
+    tc_table(axis_operator(n, alpha, dirichlet), g, tc_sk(prec), &s);
     memcpy(row, s.row, sizeof(s.row));
     memcpy(step, s.step, sizeof(s.step));
     return tc_needs_carry(prec, s);
@@ -756,7 +804,7 @@ extern "C" int scft_tc_operator(int n, double alpha, int dirichlet, int prec, do
     std::vector<long double> K;
     dense_operator(n, alpha, dirichlet, K);
     const int sk = tc_sk(prec), m = n / 2;
-    const std::vector<uint16_t> T = tc_table(K, g, sk);
+    const std::vector<uint16_t> T = tc_table(axis_operator(n, alpha, dirichlet), g, sk);
     auto digit = [](uint16_t h) {
         const int e = (h >> 10) & 31;
         const long double v = e ? ldexpl(1024 + (h & 0x3ff), e - 25) : ldexpl(h & 0x3ff, -24);
@@ -856,15 +904,20 @@ static std::vector<TcChoice> tc_choices(const scft_ctx *c, const TcGeom &g0, int
 
 
 /* Operator tables of one grid axis (pass slot ai) for one operator set. */
-static int axis_tables(scft_ctx *c, const Axis &A, double alpha, InstOps &o, int ai)
+static int axis_tables(scft_ctx *c, const Axis &A, const scft_derived &dv, InstOps &o, int ai)
 {
     const int n = A.g.n;
+    const double alphas[3] = {dv.alphax, dv.alphay, dv.alphaz}, alpha = alphas[A.src];
     if (A.tc) {
-        std::vector<long double> K;
-        dense_operator(n, alpha, A.dirichlet, K);
+        /* axes alike share a table */
+        for (int k = 0; k < ai; ++k)
+            if (c->axes[k].tc && c->axes[k].g.n == n && c->axes[k].dirichlet == A.dirichlet && alphas[c->axes[k].src] == alpha) {
+                o.tc[ai] = o.tc[k];
+                return SCFT_OK;
+            }
         void *td = nullptr;
         TcSums sums;
-        int rc = upload(c, &td, tc_table(K, A.t, tc_sk(c->opt.precision), &sums));
+        int rc = upload(c, &td, tc_table(axis_operator(n, alpha, A.dirichlet), A.t, tc_sk(c->opt.precision), &sums));
         if (tc_needs_carry(c->opt.precision, sums)) c->tc_carry = 1;
         if (rc) return rc;
         o.tc[ai] = td;
@@ -1038,16 +1091,14 @@ static int build_axes(scft_ctx *c)
             }
         }
         for (size_t u = 0; u < rep.size(); ++u) {
-            const scft_derived &dr = c->der[rep[u]];
-            const double alpha = ax == 0 ? dr.alphax : (ax == 1 ? dr.alphay : dr.alphaz);
-            int rc = axis_tables(c, A, alpha, c->ops_h[u], ai);
+            int rc = axis_tables(c, A, c->der[rep[u]], c->ops_h[u], ai);
             if (rc) return rc;
         }
         c->axes.push_back(A);
     }
     /* the limit is a cap, not a reservation: set the device maximum once */
     CK(scft_pass_configure(optin_limit));
-    CK(scft_pass_tc_configure(optin_limit));
+    CK(scft_pass_tc_configure(c->opt.precision, optin_limit));
     return SCFT_OK;
 }
 
@@ -1877,9 +1928,7 @@ static int build_opset(scft_ctx *c, const scft_derived &d, InstOps &o)
 {
     memset(&o, 0, sizeof(o));
     for (size_t ai = 0; ai < c->axes.size(); ++ai) {
-        const Axis &A = c->axes[ai];
-        const double alpha = A.src == 0 ? d.alphax : (A.src == 1 ? d.alphay : d.alphaz);
-        int rc = axis_tables(c, A, alpha, o, (int)ai);
+        int rc = axis_tables(c, c->axes[ai], d, o, (int)ai);
         if (rc) return rc;
     }
     if (c->fused2d) {

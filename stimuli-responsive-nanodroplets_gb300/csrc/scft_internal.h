@@ -166,7 +166,7 @@ struct TcLoop {
 
 size_t scft_pass_tc_smem(int prec, const TcGeom &g);
 int scft_pass_tc_fits(int prec, const TcGeom &g, int smem_limit);
-cudaError_t scft_pass_tc_configure(int smem_bytes);
+cudaError_t scft_pass_tc_configure(int prec, int smem_bytes);
 cudaError_t scft_launch_pass_tc(int prec, int carry, const TcGeom &g, const PassArgs &a, cudaStream_t st);
 struct Step2DArgs;
 size_t scft_chain_tc_layout(int prec, TcLoop &lp);

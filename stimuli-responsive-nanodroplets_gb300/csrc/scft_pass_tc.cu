@@ -1301,14 +1301,12 @@ static cudaError_t configure_tc(int smem_bytes)
     return e;
 }
 
-/* Raise the dynamic shared-memory limit once, outside any stream capture. */
-cudaError_t scft_pass_tc_configure(int smem_bytes)
+/* Raise the dynamic shared-memory limit of a form's kernels once, outside any stream capture. */
+cudaError_t scft_pass_tc_configure(int prec, int smem_bytes)
 {
-    cudaError_t e = configure_tc<double, false>(smem_bytes);
-    if (e == cudaSuccess) e = configure_tc<double, true>(smem_bytes);
-    if (e == cudaSuccess) e = configure_tc<dfloat, false>(smem_bytes);
-    if (e == cudaSuccess) e = configure_tc<dfloat, true>(smem_bytes);
-    if (e == cudaSuccess) e = configure_tc<float, false>(smem_bytes);
+    if (prec == SCFT_PREC_FP32) return configure_tc<float, false>(smem_bytes);
+    cudaError_t e = prec == SCFT_PREC_FP64 ? configure_tc<double, false>(smem_bytes) : configure_tc<dfloat, false>(smem_bytes);
+    if (e == cudaSuccess) e = prec == SCFT_PREC_FP64 ? configure_tc<double, true>(smem_bytes) : configure_tc<dfloat, true>(smem_bytes);
     return e;
 }
 
