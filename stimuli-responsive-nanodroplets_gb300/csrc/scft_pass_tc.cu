@@ -329,11 +329,12 @@ __device__ __noinline__ double from_fix_slow(long long acc, int emax)
 {
     const unsigned long long u = acc < 0 ? (unsigned long long)-acc : (unsigned long long)acc;
     if (emax == 0 || u == 0) return 0.0;
-    if (emax < 64) return ((double)acc * 0x1p-60) * __hiloint2double((emax + 4) << 20, 0); /* acc 2^(emax - 1079), subnormal or not */
     const int lz = __clzll((long long)u), eb = emax + 7 - lz; /* biased exponent */
     const unsigned long long m = u << lz;
-    unsigned long long r = ((unsigned long long)(eb - 1) << 52) + (m >> 11) + ((m >> 10) & 1);
-    if (eb <= 0) r = 0;
+    if (eb < -51) return 0.0;
+    const int sh = eb > 0 ? 11 : 12 - eb; /* a subnormal's units are 2^-1074 */
+    unsigned long long r = (m >> sh) + ((m >> (sh - 1)) & 1);
+    if (eb > 0) r += (unsigned long long)(eb - 1) << 52;
     if (eb >= 2047) r = 0x7ff0000000000000ull;
     return __longlong_as_double((long long)(r | ((unsigned long long)acc & 0x8000000000000000ull)));
 }
