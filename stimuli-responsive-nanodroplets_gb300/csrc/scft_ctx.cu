@@ -1338,14 +1338,6 @@ static int autotune_axes(scft_ctx *c)
     return rc;
 }
 
-/* Contour steps by the cluster loop or by a launch per pass, the same arithmetic
- * either way: the loop saves launches and set-up, the passes spread every step
- * over all SMs. With the autotuner a few steps of each are timed on the context's
- * chains (every chain runs them); the time of an iteration follows from the
- * clusters that are resident together, or for the passes from the number of
- * chains still running if they fill the GPU. Without it the estimates decide,
- * the loop's doubled: with more clusters than the GPU holds it measured twice
- * its estimate (192x96, 160 chains). */
 /* Clusters of the chosen loop that fit on the GPU. */
 static int tc_resident(const scft_ctx *c)
 {
@@ -1357,6 +1349,14 @@ static int tc_resident(const scft_ctx *c)
     return 0;
 }
 
+/* Contour steps by the cluster loop or by a launch per pass, the same arithmetic
+ * either way: the loop saves launches and set-up, the passes spread every step
+ * over all SMs. With the autotuner a few steps of each are timed on the context's
+ * chains (every chain runs them); the time of an iteration follows from the
+ * clusters that are resident together, or for the passes from the number of
+ * chains still running if they fill the GPU. Without it the estimates decide, the
+ * loop's times 1.3, or 2 with more clusters than the GPU holds, where it measured
+ * twice its estimate (192x96, 160 chains). */
 static int choose_loop_tc(scft_ctx *c)
 {
     int optin = 0;
@@ -2120,8 +2120,10 @@ static PostArgs post_args(scft_ctx *c, const double *noise_dev)
  * anyway. Parts are of even length: the 3D loop alternates between two distributions of
  * the slice, and a part begins with the first, so that every bit is the same. Taken where
  * the steps it saves are worth more than a launch per round (~1.5 steps' time) and 5 %.
- * Contexts whose instances stop or change by themselves keep the one launch: the GPU deals
- * out what is left there, which the host cannot know. */
+ * Contexts whose instances stop or change by themselves keep the one launch, as the GPU deals
+ * out what is left there, which the host cannot know: the first stop rule, freeze or new
+ * surface drops the parts for good (drop_rounds), so that they serve runs of a fixed number
+ * of iterations and not sweeps or serving pools. */
 static int plan_rounds(scft_ctx *c)
 {
     const int resident = c->fused3d ? scft_step3d_resident() : c->loop_tc ? tc_resident(c) : 0, n = (int)c->chains_h.size();
