@@ -748,7 +748,8 @@ def main():
         "detail": {"fp32_prop_ms_per_step": f32["prop_ms_per_step"], "fp32_wall_ms_per_step": f32["wall_ms_per_step"],
                    "contour_steps_per_instance_iteration": f32["contour_steps_per_instance_iteration"],
                    "device_bytes_fp32": f32["device_bytes"],
-                   "fp32_threads_per_line": f32["threads_per_line"]},
+                   "fp32_threads_per_line": f32["threads_per_line"],
+                   "fp32_ctas_per_chain": f32["ctas_per_chain"]},
     }
     # the sweep and the serving stream are single-GPU measurements (replicas add nothing to them)
     if world > 1:
