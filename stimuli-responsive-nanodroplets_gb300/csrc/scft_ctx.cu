@@ -119,7 +119,7 @@ struct scft_ctx {
      * them per launch (plan_rounds); empty: one launch */
     std::vector<std::pair<int, int>> rounds; /* first unit, units */
     StepUnit *units = nullptr;
-    int tc_carry = 0; /* tensor-core passes carry between levels: some operator's digits call for it (tc_table) */
+    int tc_carry = 0; /* kernels that carry between levels: some operator's digits call for it (tc_carry_of) */
     int loop_tc = 0; /* the cluster contour loop on the tensor-core tiles (k_chain_tc) */
     TcLoop loop;
     int *order = nullptr; /* chain indices, longest first */
@@ -775,12 +775,22 @@ static std::vector<uint16_t> tc_table(const AxisOp &K, const TcGeom &g, int sk, 
     return T;
 }
 
-/* Levels 0 to 3 of FP64 and FP32x2 must be exact: a unit lost on level 3 is 2^-47 of the
- * line's largest value. FP32 rounds to 2^-24, sixteen units of its level 1. */
-static bool tc_needs_carry(int prec, const TcSums &s) { return prec != SCFT_PREC_FP32 && s.row[3] > 16777216.0; }
+/* Which levels an axis' passes carry: 0 none, 1 levels 1 to 3, 2 all. Sums within 2^24 are
+ * exact as they are. Operators whose first two digits alone make a level 1 of 2^22 (sixteen
+ * columns of full digits, 7 points wide and more) meet flat lines with digits of one sign: at
+ * DR_TARGET 0.002 and NS 48 FP64 was 1e-11 off without carries, and with levels 1 to 3 carried
+ * its last bits still differed between a loop and passes. For the others a unit lost on level 3
+ * would be 2^-47 of the line's largest value; FP32 rounds to 2^-24, eight units of its level 1. */
+static int tc_carry_of(int prec, const TcSums &s)
+{
+    const double most = 16777216.0;
+    if (s.row[prec == SCFT_PREC_FP32 ? 3 : 5] <= most) return 0;
+    if (s.row[1] > most / 4) return 2;
+    return prec != SCFT_PREC_FP32 && s.row[3] > most;
+}
 
 /* Test hook: the bounds of an operator's level sums (TcSums), and whether its passes
- * carry between levels. */
+ * carry between levels; scft_tc_carry: which. */
 extern "C" int scft_tc_level_sums(int n, double alpha, int dirichlet, int prec, double row[6], double step[6])
 {
     if (n < 2 || !row || !step) return SCFT_ERR_PARAM;
@@ -790,7 +800,16 @@ extern "C" int scft_tc_level_sums(int n, double alpha, int dirichlet, int prec, 
     tc_table(axis_operator(n, alpha, dirichlet), g, tc_sk(prec), &s);
     memcpy(row, s.row, sizeof(s.row));
     memcpy(step, s.step, sizeof(s.step));
-    return tc_needs_carry(prec, s);
+    return tc_carry_of(prec, s) != 0;
+}
+extern "C" int scft_tc_carry(int n, double alpha, int dirichlet, int prec)
+{
+    if (n < 2) return SCFT_ERR_PARAM;
+    TcGeom g;
+    tc_shape(n, dirichlet, g);
+    TcSums s;
+    tc_table(axis_operator(n, alpha, dirichlet), g, tc_sk(prec), &s);
+    return tc_carry_of(prec, s);
 }
 
 /* Test hook: the operator a tensor-core pass applies, decoded from its digits
@@ -913,12 +932,15 @@ static int axis_tables(scft_ctx *c, const Axis &A, const scft_derived &dv, InstO
         for (int k = 0; k < ai; ++k)
             if (c->axes[k].tc && c->axes[k].g.n == n && c->axes[k].dirichlet == A.dirichlet && alphas[c->axes[k].src] == alpha) {
                 o.tc[ai] = o.tc[k];
+                o.tc_carry |= (o.tc_carry >> 2 * k & 3) << 2 * ai;
                 return SCFT_OK;
             }
         void *td = nullptr;
         TcSums sums;
         int rc = upload(c, &td, tc_table(axis_operator(n, alpha, A.dirichlet), A.t, tc_sk(c->opt.precision), &sums));
-        if (tc_needs_carry(c->opt.precision, sums)) c->tc_carry = 1;
+        const int carry = tc_carry_of(c->opt.precision, sums);
+        o.tc_carry |= carry << 2 * ai;
+        if (carry) c->tc_carry = 1;
         if (rc) return rc;
         o.tc[ai] = td;
         return SCFT_OK;

@@ -34,6 +34,7 @@ struct InstOps {
     const void *kz, *twx, *ex;
     const void *spec[3], *tw[3], *kA[3], *kB[3];
     const void *tc[3]; /* operator digits of the tensor-core passes */
+    int tc_carry;      /* two bits an axis: 1 carry levels 1 to 3 of the sums, 2 all (tc_carry_of) */
 };
 
 /* One propagator chain of one instance: q[0] from init, then len-1 contour

@@ -23,14 +23,14 @@
  *     FP32's) leave out terms of 2^-56 (2^-27) of the line's largest value;
  *   - a level's sum is an integer, which the accumulator holds exactly up to 2^24.
  *     Its bound, 512 times the sum of the operator's digits up to that level over a
- *     row, is taken from the digits when the table is made (tc_table): where levels 0
- *     to 3 of FP64 or FP32x2 stay below 2^24 over whole rows, they are summed as they
- *     are, otherwise (long lines, and operators wider than the line, whose digits and
- *     those of a flat line add up with one sign) what is above 2^9 is carried to the
- *     level above after every 16 points. The last two levels, and FP32's, may pass 2^24
- *     by their bound (1.8 times on 192 points); a unit that is then lost is below
- *     2^-56 (FP32: 2^-27 per unit of its level 1), and on random digits their sums are
- *     at twelve standard deviations from it;
+ *     row, is taken from the digits when the table is made (tc_table). Where it stays
+ *     below, the sums are taken as they are; where it does not, what is above 2^9 is
+ *     carried to the level above after every 16 points: on every level for operators
+ *     that reach over many points, whose digits and those of a flat line add up with
+ *     one sign, so that all levels are exact; on levels 1 to 3 of FP64 and FP32x2 for
+ *     the others (long axes, 1.05 times 2^24 on level 3 of 192 points). Their last two
+ *     levels, and FP32's, then rest on the digits' mixed signs: twelve standard
+ *     deviations away, and a unit that is lost is below 2^-56 (FP32: 2^-27);
  *   - the levels are joined in 64-bit integers (FP32: three multiply-adds), and
  *     each output is rounded once to the value type.
  * Results do not depend on the tile, the number of output parts, the carries or what
@@ -277,16 +277,16 @@ __device__ __forceinline__ void mma16816(float (&c)[4], const uint32_t (&a)[4], 
                  : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
-/* What is above 2^9 in the sums of levels 1 to 3, an integer, moved to the level above,
+/* What is above 2^9 in the sums of levels FROM to TO, an integer, moved to the level above,
  * so that the next 16 points add to sums of at most 2^15: exact, two sums at a time.
- * Upwards from level 1, so that no step waits for the one before it. Always done it
- * costs 2-6 % of a whole solve (192x96, FP64 6.83 -> 6.97-7.12 ms, 150x75 FP32 4.84 ->
- * 5.16), hence only where an operator needs it. */
-template <int L>
+ * Upwards, so that no step waits for the one before it. Always done it costs 2-6 % of a whole
+ * solve (192x96, FP64 6.83 -> 6.97-7.12 ms, 150x75 FP32 4.84 -> 5.16), hence only where an
+ * operator needs it, in kernels of their own, as the test for it alone costs 2 %. */
+template <int FROM, int TO, int L>
 __device__ __forceinline__ void carry_sums(float (&d)[L][4])
 {
 #pragma unroll
-    for (int l = 1; l <= 3; ++l)
+    for (int l = FROM; l <= TO; ++l)
 #pragma unroll
         for (int v = 0; v < 4; v += 2)
             asm("{\n\t.reg .b64 x, u, t, c;\n\t"
@@ -298,6 +298,28 @@ __device__ __forceinline__ void carry_sums(float (&d)[L][4])
                 "mov.b64 c, {0fC4800000, 0fC4800000};\n\tfma.rn.f32x2 x, t, c, x;\n\t"
                 "mov.b64 {%0, %1}, x;\n\tmov.b64 {%2, %3}, u;\n\t}"
                 : "+f"(d[l][v]), "+f"(d[l][v + 1]), "+f"(d[l - 1][v]), "+f"(d[l - 1][v + 1]));
+}
+/* Before the next 16 points, and after half of the digit pairs of 16 points, where five or six
+ * of them alone could pass 2^24. how: InstOps::tc_carry of the axis. */
+template <int L>
+__device__ __forceinline__ void carry_step(float (&d)[L][4], int how)
+{
+    if (how) carry_sums<1, 3>(d);
+    if (L > 4 && how > 1) carry_sums<4, L - 1>(d);
+}
+template <int L>
+__device__ __forceinline__ void carry_half(float (&d)[L][4], int how)
+{
+    if (L > 4 && how > 1) carry_sums<4, L - 1>(d);
+}
+/* In the end, so that the last level rounds into the one above alike whichever pairs came first. */
+template <int L>
+__device__ __forceinline__ void carry_end(float (&d)[L][4], int how)
+{
+    if (L > 4 && how > 1) {
+        carry_sums<L - 1, L - 1>(d);
+        carry_sums<L - 2, L - 2>(d);
+    }
 }
 
 __device__ __forceinline__ long long mad_wide(int a, int b, long long c)
@@ -400,7 +422,7 @@ __host__ __device__ inline uint32_t exchange_bytes(const TcGeom &g, int value)
  * half) = (lane >> 3 & 1, lane >> 4), line cells at (digit, point half) = (lane >> 4, lane >> 3 & 1).
  * d[.][v]: output (lane >> 2) + 8 (v >> 1), line 2 (lane & 3) + (v & 1). */
 template <typename P, int NB, bool CARRY>
-__device__ __forceinline__ void products16x8(float (&d)[Dig<P>::L][4], uint32_t op, uint32_t lines, int nk8, int ks, int nc, int rg, int cp, int b)
+__device__ __forceinline__ void products16x8(float (&d)[Dig<P>::L][4], uint32_t op, uint32_t lines, int nk8, int ks, int nc, int rg, int cp, int b, int carry)
 {
     constexpr int S = Dig<P>::S, SK = Dig<P>::SK, L = Dig<P>::L, CELL = S * NB * 128;
     const int lane = threadIdx.x & 31;
@@ -413,13 +435,14 @@ __device__ __forceinline__ void products16x8(float (&d)[Dig<P>::L][4], uint32_t 
         for (int v = 0; v < 4; ++v) d[l][v] = 0.0f;
 #pragma unroll 1
     for (int k = 0; k < ks; ++k) {
-        if (CARRY && k > 0) carry_sums(d);
+        if (CARRY && k > 0) carry_step(d, carry);
         uint32_t bf[(S + 1) / 2][4]; /* line digits 2i, 2i + 1 */
 #pragma unroll
         for (int i = 0; i < (S + 1) / 2; ++i)
             ldsm4(bf[i], b0 + (uint32_t)(2 * k * CELL + min(2 * i + (lane >> 4), S - 1) * NB * 128));
 #pragma unroll
         for (int j = 0; j < SK; ++j) {
+            if (CARRY && j == SK / 2) carry_half(d, carry);
             uint32_t af[4];
             ldsm4(af, a0 + (uint32_t)((k * SK + j) * 256));
 #pragma unroll
@@ -427,6 +450,7 @@ __device__ __forceinline__ void products16x8(float (&d)[Dig<P>::L][4], uint32_t 
                 if (i + j < L) mma16816(d[i + j], af, bf[i / 2][2 * (i & 1)], bf[i / 2][2 * (i & 1) + 1]);
         }
     }
+    if (CARRY) carry_end(d, carry);
 }
 
 /* Where a CTA (or a group of its warps) is. */
@@ -495,7 +519,7 @@ constexpr int EBITS = 11; /* bits of an exponent */
 template <typename P, int NB, int NT, bool CARRY>
 __device__ __forceinline__ void tc_tile2d(const TcGeom &g, const Exchange<P> &xc, bool last, int tile_i, unsigned char *smem,
                                           uint32_t sm_op, uint32_t sm_a, uint32_t sm_ex, uint32_t bar_op, bool wait_op,
-                                          bool &ok)
+                                          int carry, bool &ok)
 {
     constexpr int S = Dig<P>::S, L = Dig<P>::L, CELL = S * NB * 128;
     using Fix = typename FixT<P>::T;
@@ -549,7 +573,7 @@ __device__ __forceinline__ void tc_tile2d(const TcGeom &g, const Exchange<P> &xc
     for (int u = warp; u < nr * np * NB; u += NT / 32) {
         const int b = u % NB, v = u / NB, rg = nr == 1 ? 0 : v / np, cp = v - rg * np;
         float d[L][4];
-        products16x8<P, NB, CARRY>(d, sbase + sm_op, sbase + sm_a, nk8, ks, nc, rg, cp, b);
+        products16x8<P, NB, CARRY>(d, sbase + sm_op, sbase + sm_a, nk8, ks, nc, rg, cp, b, carry);
         Acc *at = ex + (rg * 8 + 2 * (lane & 3)) * pitch + (b * nc + 2 * cp) * W + (lane >> 2);
 #pragma unroll
         for (int i = 0; i < 4; ++i)
@@ -642,7 +666,7 @@ __device__ __forceinline__ void tc_tile2d(const TcGeom &g, const Exchange<P> &xc
 template <typename P, int NB, int NT, bool SPLIT, bool CARRY>
 __device__ __forceinline__ void tc_tile(const TcGeom &g, const P *src, P *dst, const P *bz,
                                         bool first, bool last, int tile_i, int part, unsigned char *smem,
-                                        uint32_t sm_op, uint32_t sm_a, uint32_t bar_op, bool wait_op, TcPhase &ph)
+                                        uint32_t sm_op, uint32_t sm_a, uint32_t bar_op, bool wait_op, int carry, TcPhase &ph)
 {
     constexpr int S = Dig<P>::S, SK = Dig<P>::SK, L = Dig<P>::L;
     using Fix = typename FixT<P>::T;
@@ -801,7 +825,7 @@ __device__ __forceinline__ void tc_tile(const TcGeom &g, const P *src, P *dst, c
         for (int u = warp; u < nr * np * NB; u += NT / 32) {
             const int b = u % NB, v = u / NB, rg = nr == 1 ? 0 : v / np, cp = v - rg * np;
             float d[L][4];
-            products16x8<P, NB, CARRY>(d, sbase + sm_op, sbase + sm_a, nk8, ks, nc, rg, cp, b);
+            products16x8<P, NB, CARRY>(d, sbase + sm_op, sbase + sm_a, nk8, ks, nc, rg, cp, b, carry);
             Acc *at = ex + (rg * 8 + 2 * (lane & 3)) * pitch + (b * nc + 2 * cp) * W + (lane >> 2);
 #pragma unroll
             for (int i = 0; i < 4; ++i)
@@ -846,12 +870,13 @@ __device__ __forceinline__ void tc_tile(const TcGeom &g, const P *src, P *dst, c
                 for (int v = 0; v < 4; ++v) d[l][v] = 0.0f;
 #pragma unroll 1
             for (int k = 0; k < ks; ++k) {
-                if (CARRY && k > 0) carry_sums(d);
+                if (CARRY && k > 0) carry_step(d, carry);
                 uint32_t bf[SK / 2][4]; /* digits 2j, 2j + 1 */
 #pragma unroll
                 for (int j = 0; j < SK / 2; ++j) ldsm4(bf[j], b0 + (uint32_t)(k * SK * 256 + j * 512));
 #pragma unroll
                 for (int i = 0; i < S; ++i) {
+                    if (CARRY && i == S / 2) carry_half(d, carry);
                     uint32_t af[4];
                     ldsm4(af, a0 + (uint32_t)(2 * k * CELL + i * NB * 128));
 #pragma unroll
@@ -859,6 +884,7 @@ __device__ __forceinline__ void tc_tile(const TcGeom &g, const P *src, P *dst, c
                         if (i + j < L) mma16816(d[i + j], af, bf[j / 2][2 * (j & 1)], bf[j / 2][2 * (j & 1) + 1]);
                 }
             }
+            if (CARRY) carry_end(d, carry);
 #pragma unroll
             for (int v = 0; v < 4; ++v) acc[v] = join(d, v);
         };
@@ -969,7 +995,8 @@ __global__ void __launch_bounds__(256, 2) k_pass_tc(TcGeom g, PassArgs a)
     P *dst = a.last ? reinterpret_cast<P *>(cd.q) + (long)(a.s + 1) * a.sstride : reinterpret_cast<P *>(cd.tmp);
     const P *bz = reinterpret_cast<const P *>(a.s < cd.seg_end ? cd.b0 : cd.b1);
     TcPhase ph = {0, true};
-    tc_tile<P, NB, 256, false, CARRY>(g, src, dst, bz, a.first, a.last, tile_i, part, smem, SM_OP, SM_OP + g.op_part, bar_op, true, ph);
+    const int carry = CARRY ? cd.ops->tc_carry >> 2 * a.axis & 3 : 0;
+    tc_tile<P, NB, 256, false, CARRY>(g, src, dst, bz, a.first, a.last, tile_i, part, smem, SM_OP, SM_OP + g.op_part, bar_op, true, carry, ph);
     if (!ph.ok && threadIdx.x == 0) atomicExch(&g_scft_pass_fault, 1);
 }
 
@@ -1015,6 +1042,7 @@ __global__ void __launch_bounds__(512, 1) k_chain_tc(const __grid_constant__ TcL
         return;
     }
     TcPhase ph = {0, true};
+    const int carry = CARRY ? cd.ops->tc_carry : 0;
     const int group = threadIdx.x / (512 / GROUPS);
     const uint32_t tile_at = lp.tile_at + (uint32_t)group * lp.tile_bytes;
 #pragma unroll 1
@@ -1033,10 +1061,10 @@ __global__ void __launch_bounds__(512, 1) k_chain_tc(const __grid_constant__ TcL
                 for (int t = t0; (long)t * g.tile < g.lines; t += GROUPS * lp.slots[ax]) {
                     if (g.nb == 4)
                         tc_tile<P, 4, 512 / GROUPS, true, CARRY>(g, src, dst, bz, first, last, t, part, smem, lp.op_at[ax], tile_at,
-                                                 sbase + SM_BAR + 8 * ax, s == run.s && t == t0, ph);
+                                                 sbase + SM_BAR + 8 * ax, s == run.s && t == t0, carry >> 2 * ax & 3, ph);
                     else
                         tc_tile<P, 2, 512 / GROUPS, true, CARRY>(g, src, dst, bz, first, last, t, part, smem, lp.op_at[ax], tile_at,
-                                                 sbase + SM_BAR + 8 * ax, s == run.s && t == t0, ph);
+                                                 sbase + SM_BAR + 8 * ax, s == run.s && t == t0, carry >> 2 * ax & 3, ph);
                 }
             /* this axis' slice is complete before the next one reads it */
             asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
@@ -1089,6 +1117,7 @@ __global__ void __launch_bounds__(512, 1) k_chain2d_tc(const __grid_constant__ T
     bool mine[2], ok = true;
     uint32_t bytes[2];
     int tiles = 0; /* tiles done */
+    const int carry = CARRY ? cd.ops->tc_carry : 0;
 #pragma unroll
     for (int ax = 0; ax < 2; ++ax) {
         const TcGeom &g = lp.g[ax];
@@ -1161,9 +1190,9 @@ __global__ void __launch_bounds__(512, 1) k_chain2d_tc(const __grid_constant__ T
                                     reinterpret_cast<const P *>(s + 1 < cd.seg_end ? cd.b0 : cd.b1),
                                     reinterpret_cast<P *>(cd.q) + (long)(s + 1) * a.sstride};
             if (g.nb == 4)
-                tc_tile2d<P, 4, 512, CARRY>(g, xc, ax == 1, rank, smem, lp.op_at[ax], lp.tile_at, lp.ex_at, bars + 8 * ax, t == 0, ok);
+                tc_tile2d<P, 4, 512, CARRY>(g, xc, ax == 1, rank, smem, lp.op_at[ax], lp.tile_at, lp.ex_at, bars + 8 * ax, t == 0, carry >> 2 * ax & 3, ok);
             else
-                tc_tile2d<P, 2, 512, CARRY>(g, xc, ax == 1, rank, smem, lp.op_at[ax], lp.tile_at, lp.ex_at, bars + 8 * ax, t == 0, ok);
+                tc_tile2d<P, 2, 512, CARRY>(g, xc, ax == 1, rank, smem, lp.op_at[ax], lp.tile_at, lp.ex_at, bars + 8 * ax, t == 0, carry >> 2 * ax & 3, ok);
         }
     }
     if (!ok && threadIdx.x == 0) atomicExch(&g_scft_pass_fault, 1);
@@ -1193,12 +1222,12 @@ int scft_pass_tc_fits(int prec, const TcGeom &g, int smem_limit)
     return scft_pass_tc_smem(prec, g) <= (size_t)smem_limit;
 }
 
-/* carry: an operator of the context needs the carries of carry_sums (FP32 never does). */
+/* carry: some operator of the context needs the carries of carry_sums. */
 cudaError_t scft_launch_pass_tc(int prec, int carry, const TcGeom &g, const PassArgs &a, cudaStream_t st)
 {
     if (prec == SCFT_PREC_FP64) return carry ? launch_tc<double, true>(g, a, st) : launch_tc<double, false>(g, a, st);
     if (prec == SCFT_PREC_FP32X2) return carry ? launch_tc<dfloat, true>(g, a, st) : launch_tc<dfloat, false>(g, a, st);
-    return launch_tc<float, false>(g, a, st);
+    return carry ? launch_tc<float, true>(g, a, st) : launch_tc<float, false>(g, a, st);
 }
 
 /* Shared-memory layout of the cluster loop, from the axes' tiles and parts;
@@ -1283,7 +1312,7 @@ cudaError_t scft_launch_chain_tc(int prec, int carry, const TcLoop &lp, const St
         return carry ? launch_chain<double, true>(lp, a, nchains, st, clusters) : launch_chain<double, false>(lp, a, nchains, st, clusters);
     if (prec == SCFT_PREC_FP32X2)
         return carry ? launch_chain<dfloat, true>(lp, a, nchains, st, clusters) : launch_chain<dfloat, false>(lp, a, nchains, st, clusters);
-    return launch_chain<float, false>(lp, a, nchains, st, clusters);
+    return carry ? launch_chain<float, true>(lp, a, nchains, st, clusters) : launch_chain<float, false>(lp, a, nchains, st, clusters);
 }
 
 template <typename P, bool CARRY>
@@ -1305,9 +1334,17 @@ static cudaError_t configure_tc(int smem_bytes)
 /* Raise the dynamic shared-memory limit of a form's kernels once, outside any stream capture. */
 cudaError_t scft_pass_tc_configure(int prec, int smem_bytes)
 {
-    if (prec == SCFT_PREC_FP32) return configure_tc<float, false>(smem_bytes);
-    cudaError_t e = prec == SCFT_PREC_FP64 ? configure_tc<double, false>(smem_bytes) : configure_tc<dfloat, false>(smem_bytes);
-    if (e == cudaSuccess) e = prec == SCFT_PREC_FP64 ? configure_tc<double, true>(smem_bytes) : configure_tc<dfloat, true>(smem_bytes);
+    cudaError_t e;
+    if (prec == SCFT_PREC_FP64) {
+        e = configure_tc<double, false>(smem_bytes);
+        if (e == cudaSuccess) e = configure_tc<double, true>(smem_bytes);
+    } else if (prec == SCFT_PREC_FP32X2) {
+        e = configure_tc<dfloat, false>(smem_bytes);
+        if (e == cudaSuccess) e = configure_tc<dfloat, true>(smem_bytes);
+    } else {
+        e = configure_tc<float, false>(smem_bytes);
+        if (e == cudaSuccess) e = configure_tc<float, true>(smem_bytes);
+    }
     return e;
 }
 
